@@ -389,11 +389,12 @@ struct PairData {
     DevBuf<uint4> batch_rec;         // contact pairs in colour order: body a, body b, pair | rows << 29, 0
     DevBuf<uint4> split_rec;         // the same for the pairs with split-active rows
     DevBuf<float4> vtab, stab;       // solver contact tables in batch-slot order (k_solver.cu)
-    // Chunked PGS (k_solver.cu): per body its chunk and the foreign chunks whose groups touch it;
-    // per (colour, chunk) the group counts / cursors and bin offsets; the chunk adjacency
-    // bit matrix and the per-chunk progress counters.
-    DevBuf<uint32_t> chunk_of, chunk_touch, chunk_hist, chunk_off, chunk_adj;
-    DevBuf<unsigned int> chunk_ctr;
+    // Chunked PGS (k_solver.cu): per body its chunk, the colours of its groups and split groups
+    // (4 words) and its versioned velocities and push velocities (2 float4 each); per (colour,
+    // chunk) the group counts / cursors and bin offsets.
+    DevBuf<uint32_t> chunk_of, chunk_hist, chunk_off;
+    DevBuf<unsigned long long> body_used;
+    DevBuf<float4> flow_vel;
     DevBuf<uint32_t> flags;          // selection flags
     DevBuf<uint32_t> sel_a, sel_b;   // cache compaction lists
     DevBuf<unsigned char> cub_tmp;
@@ -414,6 +415,7 @@ struct PairData {
         body_prio.reserve(nbodies);
         body_mask.reserve(2 * nbodies);
         body_dup.reserve(2 * nbodies);
+        body_used.reserve(4 * nbodies);
         colour_remap.reserve(132);
         colour_count.reserve(132);
         colour_offset.reserve(132);

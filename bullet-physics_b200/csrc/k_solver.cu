@@ -10,10 +10,10 @@
 // is touched twice, so the result is bit-identical to the reference's
 // sequential solve over the same rows taken in (colour, pair) order.
 //
-// Worlds without joints use the chunked PGS (k_solve_chunks): the bodies are cut into
-// Morton-ordered chunks, one per block of a cooperative launch, each block solves its own
-// chunk's groups colour by colour, and between two phases it waits only for the blocks whose
-// groups share a dynamic body with its own. A group's contacts are spread over lanes (one
+// Worlds without joints use the chunked PGS (k_solve_flow): the bodies are cut into
+// Morton-ordered chunks, one per block of a cooperative launch, and each warp solves its share of
+// the chunk's groups colour by colour, waiting only for the versions of its groups' own velocities
+// (a version rides in the fourth word of a velocity). A group's contacts are spread over lanes (one
 // contact per lane, the velocities handed from lane to lane in contact order), and the split
 // sweep s rides in the phases of velocity sweep s + 1. Worlds with joints use the team kernel
 // (k_solve): a persistent cooperative launch split into two teams of blocks with their own
@@ -75,6 +75,7 @@ struct ColourArgs {
     unsigned long long* prio;
     unsigned long long* mask;
     unsigned long long* dup;      // 2 words per body: colours seeded twice at the body
+    unsigned long long* used;     // 4 words per body, zeroed here for the histogram pass (null: not wanted)
     const float4* entries;        // this step's manifold entries (their meta carries last step's colour)
     uint32_t seed;                // 1: start from last step's colours
     unsigned int* bar;  // [0] barrier counter, [5] colour max, [6] [7] uncoloured-list lengths
@@ -197,6 +198,9 @@ __global__ void k_colour(ColourArgs a, JpList wl) {
         } else {
             wl.items[0][k] = k;  // every group starts uncoloured
         }
+        if (a.used) {
+            for (uint32_t x = 0; x < 4; ++x) a.used[4 * u + x] = a.used[4 * v + x] = 0ull;
+        }
     }
     if (tid == 0) {
         a.bar[5] = 0;
@@ -292,18 +296,19 @@ __global__ void k_colour(ColourArgs a, JpList wl) {
 // Colour histograms of all groups and of the groups with split-active rows,
 // plus the row and split-row totals.
 // With chunk histograms (vhist non-null) the pass also counts each group into its (colour,
-// chunk) bins and records its touch sets (chunk_count, with the chunked PGS's code below).
+// chunk) bins and marks its colour at its dynamic bodies (chunk_count, with the chunked PGS's
+// code below).
 __device__ __forceinline__ void chunk_count(const uint64_t* __restrict__ pairs, uint32_t p, uint32_t c, uint32_t rows,
                                             bool split, const float4* __restrict__ iw,
                                             const uint32_t* __restrict__ chunk_of, uint32_t P, uint32_t* vhist,
-                                            uint32_t* shist, uint32_t* touch, uint32_t* all_flag);
+                                            uint32_t* shist, unsigned long long* used);
 
 __global__ void k_colour_hist(const uint32_t* __restrict__ count, const uint32_t* __restrict__ contact_pairs,
                               const uint32_t* __restrict__ colour, const uint32_t* __restrict__ row_count,
                               const float4* __restrict__ rows, uint32_t* hist, uint32_t* split_hist, uint32_t* split_flag,
                               uint32_t* sub_hist, const uint64_t* __restrict__ pairs, const float4* __restrict__ iw,
                               const uint32_t* __restrict__ chunk_of, uint32_t P, uint32_t* vhist, uint32_t* shist,
-                              uint32_t* touch, uint32_t* all_flag) {
+                              unsigned long long* used) {
     // Block-local histograms; [MAX_COLOURS] rows, [MAX_COLOURS + 1] split-active rows;
     // shc: groups per (colour, row count - 1).
     __shared__ uint32_t sh[MAX_COLOURS + 2], ssh[MAX_COLOURS], shc[MAX_COLOURS * 4];
@@ -331,7 +336,7 @@ __global__ void k_colour_hist(const uint32_t* __restrict__ count, const uint32_t
             nsplit_rows += nsr;
             atomicAdd(&ssh[c], 1u);
         }
-        if (vhist) chunk_count(pairs, p, c, n, nsr != 0u, iw, chunk_of, P, vhist, shist, touch, all_flag);
+        if (vhist) chunk_count(pairs, p, c, n, nsr != 0u, iw, chunk_of, P, vhist, shist, used);
     }
     nrows = __reduce_add_sync(0xffffffffu, nrows);
     nsplit_rows = __reduce_add_sync(0xffffffffu, nsplit_rows);
@@ -446,60 +451,61 @@ __device__ __forceinline__ uint32_t claim_slot(uint32_t* cursor, uint32_t c) {
 // ---------------------------------------------------------------- chunks (chunked PGS)
 // The chunked PGS deals each colour batch to the blocks of the launch by chunk: a chunk is a
 // run of bodies in Morton order (the broad phase's tree leaves), and a group belongs to the
-// chunk of its first dynamic body. Block b solves chunk b's groups of every colour; before
-// a phase it waits only for the blocks whose groups share a dynamic body with its own (its
-// neighbours), not for the whole grid. Every block whose groups touch a body appears in the
-// body's touch set (its own chunk plus the foreign chunks recorded by the histogram pass), so
-// making every two chunks of each touch set neighbours covers every shared body.
-constexpr uint32_t CHUNK_TOUCH = 8;          // foreign chunks recorded per body
-constexpr uint32_t CHUNK_EMPTY = 0xffffffffu;
+// chunk of its first dynamic body. Block b solves chunk b's groups of every colour.
+//
+// Ordering: within a sweep a dynamic body is updated by its groups in colour order, so its
+// velocity goes through a chain of versions known before the solve starts: the group with rank r
+// among the body's d groups finds version s d + r in sweep s and leaves version s d + r + 1.
+// The colours of a body's groups are a bit mask (two 64-bit words), so d is its population count
+// and r the count of the bits below the group's colour; both ride in the group's slot record.
 constexpr uint32_t CHUNK_MAX = 1024;         // blocks of a chunked launch
-constexpr uint32_t CHUNK_CTR_STRIDE = 8;     // progress counters 32 bytes apart
-constexpr uint32_t CHUNK_TB = 512;           // threads of a chunk block (one block per SM)
+constexpr uint32_t CHUNK_TB = 384;           // threads of a chunk block (one block per SM)
 
 __device__ __forceinline__ uint32_t group_owner(uint32_t ia, uint32_t ib, const float4* __restrict__ iw,
-                                                const uint32_t* __restrict__ chunk_of) {
-    return chunk_of[inv_mass_of(iw, ia) > 0.0f ? ia : ib];
+                                                const uint32_t* __restrict__ chunk_of, uint32_t P) {
+    return min(chunk_of[inv_mass_of(iw, ia) > 0.0f ? ia : ib], P - 1u);
 }
 
-// Bodies in Morton order cut into P equal runs (bodies outside the tree keep chunk 0); with no
-// tree, runs of body indices.
-__global__ void k_chunk_of(uint32_t n, uint32_t P, const uint32_t* __restrict__ leaf, uint32_t m, uint32_t* chunk_of) {
+// Bodies in Morton order cut into P equal runs; with no tree, runs of body indices. (Dynamic
+// bodies are all in the tree when there is one; other bodies own no group.) Also clears the version
+// tags of the bodies' velocity words (vel, 2 float4 a body, velocities then push velocities).
+__global__ void k_chunk_of(uint32_t n, uint32_t P, const uint32_t* __restrict__ leaf, uint32_t m, uint32_t* chunk_of,
+                           float4* vel) {
     const uint32_t lim = leaf ? m : n;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < lim; i += gridDim.x * blockDim.x) {
-        const uint32_t c = uint32_t(uint64_t(i) * P / lim);
-        chunk_of[leaf ? leaf[i] : i] = c;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < 4u * n; i += gridDim.x * blockDim.x) {
+        vel[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (i < lim) chunk_of[leaf ? leaf[i] : i] = uint32_t(uint64_t(i) * P / lim);
     }
 }
 
-// Records chunk B in the touch set of body x when B is not x's own chunk (slot values only
-// ever go from empty to a chunk id, so a stale read of a filled slot is still correct).
-__device__ __forceinline__ void chunk_touch(uint32_t* touch, uint32_t x, uint32_t B, uint32_t* all_flag) {
-    uint32_t* t = touch + size_t(x) * CHUNK_TOUCH;
-    for (uint32_t s = 0; s < CHUNK_TOUCH; ++s) {
-        uint32_t v = t[s];
-        if (v == B) return;
-        if (v == CHUNK_EMPTY) {
-            v = atomicCAS(&t[s], CHUNK_EMPTY, B);
-            if (v == CHUNK_EMPTY || v == B) return;
-        }
-    }
-    atomicOr(all_flag, 1u);  // more foreign chunks than slots: every block becomes every block's neighbour
-}
-
-// Groups per (colour, chunk, row count) and split groups per (colour, chunk), plus the
-// touch sets of the groups' dynamic bodies (k_colour_hist's pass, for each group).
+// Groups per (colour, chunk, row count) and split groups per (colour, chunk), and the colours of
+// the groups (words 0, 1) and split groups (words 2, 3) at their dynamic bodies (k_colour_hist's
+// pass, for each group).
 __device__ __forceinline__ void chunk_count(const uint64_t* __restrict__ pairs, uint32_t p, uint32_t c, uint32_t rows,
                                             bool split, const float4* __restrict__ iw,
                                             const uint32_t* __restrict__ chunk_of, uint32_t P, uint32_t* vhist,
-                                            uint32_t* shist, uint32_t* touch, uint32_t* all_flag) {
+                                            uint32_t* shist, unsigned long long* used) {
     const uint64_t key = pairs[p];
     const uint32_t ia = key_lo(key), ib = key_hi(key);
-    const uint32_t B = group_owner(ia, ib, iw, chunk_of);
+    const uint32_t B = group_owner(ia, ib, iw, chunk_of, P);
     atomicAdd(&vhist[(size_t(c) * P + B) * 4 + (rows - 1)], 1u);
     if (split) atomicAdd(&shist[size_t(c) * P + B], 1u);
-    if (inv_mass_of(iw, ia) > 0.0f && chunk_of[ia] != B) chunk_touch(touch, ia, B, all_flag);
-    if (inv_mass_of(iw, ib) > 0.0f && chunk_of[ib] != B) chunk_touch(touch, ib, B, all_flag);
+    const unsigned long long bit = 1ull << (c & 63u);
+    for (uint32_t side = 0; side < 2; ++side) {
+        const uint32_t x = side ? ib : ia;
+        if (!(inv_mass_of(iw, x) > 0.0f)) continue;
+        atomicOr(&used[4 * size_t(x) + (c >> 6)], bit);
+        if (split) atomicOr(&used[4 * size_t(x) + 2 + (c >> 6)], bit);
+    }
+}
+
+// A group's rank among its body's groups | the number of them << 8 (0: the body is not dynamic);
+// m: the two mask words.
+__device__ __forceinline__ uint32_t colour_rank(const unsigned long long* __restrict__ m, uint32_t c) {
+    const unsigned long long lo = m[0], hi = m[1];
+    const unsigned long long below = (1ull << (c & 63u)) - 1ull;
+    const uint32_t r = c < 64u ? __popcll(lo & below) : __popcll(lo) + __popcll(hi & below);
+    return r | ((__popcll(lo) + __popcll(hi)) << 8);
 }
 
 // One block per raw colour: the colour's batch is laid out chunk by chunk (inside a chunk the
@@ -552,38 +558,17 @@ __global__ void __launch_bounds__(TB) k_chunk_scan(uint32_t P, const uint32_t* _
     }
 }
 
-// Neighbour bits: every two distinct chunks of a body's touch set (its own chunk included).
-__global__ void k_chunk_adjacency(uint32_t n, const uint32_t* __restrict__ chunk_of, const uint32_t* __restrict__ touch,
-                                  uint32_t W, uint32_t* adj) {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t* t = touch + size_t(i) * CHUNK_TOUCH;
-        if (t[0] == CHUNK_EMPTY) continue;  // touched by its own chunk only
-        uint32_t v[CHUNK_TOUCH + 1];
-        uint32_t m = 0;
-        v[m++] = chunk_of[i];
-#pragma unroll
-        for (uint32_t s = 0; s < CHUNK_TOUCH; ++s)
-            if (t[s] != CHUNK_EMPTY) v[m++] = t[s];
-        for (uint32_t a = 0; a < m; ++a)
-            for (uint32_t b = 0; b < m; ++b) {
-                if (v[a] == v[b]) continue;
-                uint32_t* w = &adj[size_t(v[a]) * W + (v[b] >> 5)];
-                const uint32_t bit = 1u << (v[b] & 31u);
-                if (!(*w & bit)) atomicOr(w, bit);
-            }
-    }
-}
-
 // Slot record of a group: its two bodies and its pair index with the row count
 // in the top three bits. With chunk cursors (vcur / scur, by raw colour) the slot is taken
-// in the group's (colour, chunk, row count) part.
+// in the group's (colour, chunk, row count) part, and the record's last word holds the
+// group's rank and the group count of each body (colour_rank, body b's in the upper half).
 __global__ void k_colour_scatter(const uint32_t* __restrict__ count, const uint32_t* __restrict__ contact_pairs,
                                  const uint64_t* __restrict__ pairs, const uint32_t* __restrict__ row_count,
                                  const uint32_t* __restrict__ colour, const uint32_t* __restrict__ split_flag,
                                  uint32_t* sub_cursor, uint32_t* split_cursor, uint4* batch_rec, uint4* split_rec,
                                  float4* entries, const uint32_t* __restrict__ remap,
                                  const uint32_t* __restrict__ chunk_of, const float4* __restrict__ iw, uint32_t P,
-                                 uint32_t* vcur, uint32_t* scur) {
+                                 uint32_t* vcur, uint32_t* scur, const unsigned long long* __restrict__ used) {
     uint32_t K = *count;
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < K; k += gridDim.x * blockDim.x) {
         if (colour[k] >= MAX_COLOURS) continue;  // colouring gave up (its status bit is set)
@@ -596,9 +581,15 @@ __global__ void k_colour_scatter(const uint32_t* __restrict__ count, const uint3
         float* mw = &entries[size_t(p) * ENTRY_F4 + 2].w;
         *mw = __uint_as_float((__float_as_uint(*mw) & ~(0xffu << META_COLOUR_SHIFT)) | ((c + 1u) << META_COLOUR_SHIFT));
         if (vcur) {
-            const uint32_t B = group_owner(rec.x, rec.y, iw, chunk_of);
+            const uint32_t B = group_owner(rec.x, rec.y, iw, chunk_of, P);
+            const unsigned long long *ua = used + 4 * size_t(rec.x), *ub = used + 4 * size_t(rec.y);
+            const bool da = inv_mass_of(iw, rec.x) > 0.0f, db = inv_mass_of(iw, rec.y) > 0.0f;
+            rec.w = (da ? colour_rank(ua, raw) : 0u) | ((db ? colour_rank(ub, raw) : 0u) << 16);
             batch_rec[claim_slot(vcur, (raw * P + B) * 4 + (row_count[p] - 1))] = rec;
-            if (split_flag[k]) split_rec[claim_slot(scur, raw * P + B)] = rec;
+            if (split_flag[k]) {
+                rec.w = (da ? colour_rank(ua + 2, raw) : 0u) | ((db ? colour_rank(ub + 2, raw) : 0u) << 16);
+                split_rec[claim_slot(scur, raw * P + B)] = rec;
+            }
         } else {
             batch_rec[claim_slot(sub_cursor, c * 4 + (row_count[p] - 1))] = rec;
             if (split_flag[k]) split_rec[claim_slot(split_cursor, c)] = rec;
@@ -632,10 +623,16 @@ struct SolveArgs {
     float damping;            // joint rows (info.rs damping)
 };
 
+// Only dynamic bodies move. Selects, not branches: a branch inside the contact's dependent chain
+// costs more than the arithmetic it skips.
+__device__ __forceinline__ V3 pick(bool c, V3 x, V3 y) { return V3{c ? x.x : y.x, c ? x.y : y.y, c ? x.z : y.z}; }
+
 __device__ __forceinline__ void apply(V3& la, V3& wa, V3& lb, V3& wb, bool appa, bool appb, float ima, float imb, V3 d,
                                       V3 ca, V3 cb, float j) {
-    if (appa) { la -= d * (j * ima); wa -= ca * j; }
-    if (appb) { lb += d * (j * imb); wb += cb * j; }
+    la = pick(appa, la - d * (j * ima), la);
+    wa = pick(appa, wa - ca * j, wa);
+    lb = pick(appb, lb + d * (j * imb), lb);
+    wb = pick(appb, wb + cb * j, wb);
 }
 
 enum Kind { WARM = 0, ITER = 1, SPLIT = 2 };
@@ -703,83 +700,93 @@ __device__ __forceinline__ void warm_group(const SolveArgs& a, uint32_t t, uint3
     }
 }
 
-// The velocity-table entries of one contact.
-struct VPlanes {
-    float4 r0, r1, r2, q3, q5, q6, q7, q8, q9, q10, r3;
+// A contact's table entries and the terms of solve_contact that depend on nothing else: the second
+// tangent and the velocity couplings (sequential_impulse.rs:352-520).
+struct ContactTerms {
+    V3 n, ra, rb, t1, t2, ana, anb, a1a, a1b, a2a, a2b, kn, kt1, kt2;
+    float friction, bias_a, bias_b, mn, m1, m2, cfm, restitution;
+
+    // Keeps the terms' computation where it stands (the compiler would sink it to their use).
+    __device__ __forceinline__ void pin() {
+        auto v = [](V3& x) { asm volatile("" : "+f"(x.x), "+f"(x.y), "+f"(x.z)); };
+        v(n); v(ra); v(rb); v(t1); v(t2); v(ana); v(anb); v(a1a); v(a1b); v(a2a); v(a2b); v(kn); v(kt1); v(kt2);
+        asm volatile("" : "+f"(friction), "+f"(bias_a), "+f"(bias_b), "+f"(mn), "+f"(m1), "+f"(m2), "+f"(cfm),
+                     "+f"(restitution));
+    }
 };
 
-__device__ __forceinline__ VPlanes load_vplanes(const float4* e) {
-    VPlanes v;
-    v.r0 = e[VT_N * PLANE_STRIDE];
-    v.r1 = e[VT_RA * PLANE_STRIDE];
-    v.r2 = e[VT_RB * PLANE_STRIDE];
-    v.q3 = e[VT_T1 * PLANE_STRIDE];
-    v.q5 = e[VT_ANA * PLANE_STRIDE];
-    v.q6 = e[VT_ANB * PLANE_STRIDE];
-    v.q7 = e[VT_A1A * PLANE_STRIDE];
-    v.q8 = e[VT_A1B * PLANE_STRIDE];
-    v.q9 = e[VT_A2A * PLANE_STRIDE];
-    v.q10 = e[VT_A2B * PLANE_STRIDE];
-    v.r3 = e[VT_IMP * PLANE_STRIDE];
-    return v;
-}
-
-// One solve_contact (sequential_impulse.rs:804-930) of contact k of slot t (pair p) from its
-// table entries (plane pl at src[pl * st]: the table itself or a shared-memory copy); the new
-// impulses go back to the table entry e (and, on the last sweep, to the pair's row).
-__device__ __forceinline__ void iter_contact(const SolveArgs& a, const float4* src, uint32_t st, float ima, float imb,
-                                             bool appa, bool appb, V3& la, V3& wa, V3& lb, V3& wb, float4* e,
-                                             uint32_t sweep, uint32_t k, uint32_t t, bool last, uint32_t p) {
+__device__ __forceinline__ ContactTerms contact_terms(const float4* src, uint32_t st, float ima, float imb) {
     const float ims = ima + imb;
     const float4 r0 = src[VT_N * st], r1 = src[VT_RA * st], r2 = src[VT_RB * st], q3 = src[VT_T1 * st],
                  q5 = src[VT_ANA * st], q6 = src[VT_ANB * st], q7 = src[VT_A1A * st], q8 = src[VT_A1B * st],
-                 q9 = src[VT_A2A * st], q10 = src[VT_A2B * st], r3 = src[VT_IMP * st];
-    const V3 n = from4(r0), ra = from4(r1), rb = from4(r2), t1 = from4(q3);
-    const V3 t2 = cross(n, t1);  // tangent_basis (sequential_impulse.rs:620-629), as warm_terms made it
-    const V3 ana = from4(q5), anb = from4(q6), a1a = from4(q7), a1b = from4(q8), a2a = from4(q9), a2b = from4(q10);
+                 q9 = src[VT_A2A * st], q10 = src[VT_A2B * st];
+    ContactTerms c;
+    c.n = from4(r0); c.ra = from4(r1); c.rb = from4(r2); c.t1 = from4(q3);
+    c.t2 = cross(c.n, c.t1);  // tangent_basis (sequential_impulse.rs:620-629), as warm_terms made it
+    c.ana = from4(q5); c.anb = from4(q6); c.a1a = from4(q7); c.a1b = from4(q8); c.a2a = from4(q9); c.a2b = from4(q10);
     // The velocity couplings of sequential_impulse.rs:352-520, in warm_terms's operand order.
-    const V3 kn = n * ims + cross(anb, rb) + cross(ana, ra);
-    const V3 kt1 = t1 * ims + cross(a1b, rb) + cross(a1a, ra);
-    const V3 kt2 = t2 * ims + cross(a2b, rb) + cross(a2a, ra);
-    const float4 r4 = make_float4(q5.w, q6.w, q7.w, q8.w);
-    V3 va = la + cross(wa, ra);
-    V3 vb = lb + cross(wb, rb);
+    c.kn = c.n * ims + cross(c.anb, c.rb) + cross(c.ana, c.ra);
+    c.kt1 = c.t1 * ims + cross(c.a1b, c.rb) + cross(c.a1a, c.ra);
+    c.kt2 = c.t2 * ims + cross(c.a2b, c.rb) + cross(c.a2a, c.ra);
+    c.friction = r0.w; c.bias_a = r1.w; c.bias_b = r2.w;
+    c.mn = q5.w; c.m1 = q6.w; c.m2 = q7.w; c.cfm = q8.w; c.restitution = q9.w;
+    return c;
+}
+
+// One solve_contact (sequential_impulse.rs:804-930): r3 holds the contact's accumulated impulses,
+// and the new ones come back with the values the adjoint's records need.
+struct ContactResult {
+    float4 r3;
+    float vn, u1, u2, maxf;
+};
+
+__device__ __forceinline__ ContactResult solve_contact(const SolveArgs& a, const ContactTerms& c, float4 r3, float ima,
+                                                       float imb, bool appa, bool appb, V3& la, V3& wa, V3& lb, V3& wb) {
+    V3 va = la + cross(wa, c.ra);
+    V3 vb = lb + cross(wb, c.rb);
     V3 rel = vb - va;
-    float vn = dot(rel, n);
-    float bias = 0.0f;
-    if (vn < -a.restitution_threshold) bias = -q9.w * vn;
-    if (r1.w != 0.0f) bias += r1.w;
-    if (r2.w != 0.0f) bias += r2.w;
-    float lambda = r4.w != 0.0f ? r4.x * (bias - vn) - r4.w * r3.x : r4.x * (bias - vn);
+    const float vn = dot(rel, c.n);
+    float bias = vn < -a.restitution_threshold ? -c.restitution * vn : 0.0f;
+    bias = c.bias_a != 0.0f ? bias + c.bias_a : bias;
+    bias = c.bias_b != 0.0f ? bias + c.bias_b : bias;
+    const float lam0 = c.mn * (bias - vn);
+    const float lambda = c.cfm != 0.0f ? lam0 - c.cfm * r3.x : lam0;
     float old = r3.x;
     float nimp = fmaxf(old + lambda, 0.0f);
     float jn = nimp - old;
-    apply(la, wa, lb, wb, appa, appb, ima, imb, n, ana, anb, jn);
-    rel += kn * jn;
-    float maxf = r0.w * nimp;
-    float vt = dot(rel, t1);
-    float lam = -r4.y * (vt - 0.0f * a.inv_dt);
+    apply(la, wa, lb, wb, appa, appb, ima, imb, c.n, c.ana, c.anb, jn);
+    rel += c.kn * jn;
+    float maxf = c.friction * nimp;
+    float vt = dot(rel, c.t1);
+    float lam = -c.m1 * (vt - 0.0f * a.inv_dt);
     float o1 = r3.y;
     const float u1 = o1 + lam;
     float n1 = fminf(fmaxf(u1, -maxf), maxf);
     float j1 = n1 - o1;
-    apply(la, wa, lb, wb, appa, appb, ima, imb, t1, a1a, a1b, j1);
-    rel += kt1 * j1;
-    vt = dot(rel, t2);
-    lam = -r4.z * (vt - 0.0f * a.inv_dt);
+    apply(la, wa, lb, wb, appa, appb, ima, imb, c.t1, c.a1a, c.a1b, j1);
+    rel += c.kt1 * j1;
+    vt = dot(rel, c.t2);
+    lam = -c.m2 * (vt - 0.0f * a.inv_dt);
     float o2 = r3.z;
     const float u2 = o2 + lam;
     float n2 = fminf(fmaxf(u2, -maxf), maxf);
     float j2 = n2 - o2;
-    apply(la, wa, lb, wb, appa, appb, ima, imb, t2, a2a, a2b, j2);
-    const float4 nr3 = make_float4(nimp, n1, n2, r3.w);
+    apply(la, wa, lb, wb, appa, appb, ima, imb, c.t2, c.a2a, c.a2b, j2);
+    return ContactResult{make_float4(nimp, n1, n2, r3.w), vn, u1, u2, maxf};
+}
+
+// Contact k of slot t (pair p): its new impulses go back to the table entry e and, on the last sweep,
+// to the pair's row.
+__device__ __forceinline__ void store_contact(const SolveArgs& a, const ContactResult& x, float4* e, uint32_t sweep,
+                                              uint32_t k, uint32_t t, bool last, uint32_t p) {
     if (a.srec) {  // the forward values the adjoint's frozen linearisation needs
-        const uint32_t s1 = u1 > maxf ? 1u : (u1 < -maxf ? 2u : 0u);
-        const uint32_t s2 = u2 > maxf ? 1u : (u2 < -maxf ? 2u : 0u);
-        a.srec[sweep_index(sweep, k, t, a.iterations)] = make_float4(vn, nimp, __uint_as_float(s1 | (s2 << 2)), 0.0f);
+        const uint32_t s1 = x.u1 > x.maxf ? 1u : (x.u1 < -x.maxf ? 2u : 0u);
+        const uint32_t s2 = x.u2 > x.maxf ? 1u : (x.u2 < -x.maxf ? 2u : 0u);
+        a.srec[sweep_index(sweep, k, t, a.iterations)] =
+            make_float4(x.vn, x.r3.x, __uint_as_float(s1 | (s2 << 2)), 0.0f);
     }
-    e[VT_IMP * PLANE_STRIDE] = nr3;
-    if (last) a.rows[(size_t(p) * 4 + k) * ROW_F4 + 3] = nr3;
+    e[VT_IMP * PLANE_STRIDE] = x.r3;
+    if (last) a.rows[(size_t(p) * 4 + k) * ROW_F4 + 3] = x.r3;
 }
 
 // One solve_contact sweep (sequential_impulse.rs:804-930) over group slot t;
@@ -792,7 +799,9 @@ __device__ __forceinline__ void iter_group(const SolveArgs& a, uint32_t t, uint3
     appb = imb > 0.0f;
     for (uint32_t k = 0; k < cnt; ++k) {
         float4* e = a.vtab + tix<VT_PLANES>(0, k, t);
-        iter_contact(a, e, PLANE_STRIDE, ima, imb, appa, appb, la, wa, lb, wb, e, sweep, k, t, last, p);
+        const float4 r3 = e[VT_IMP * PLANE_STRIDE];
+        const ContactTerms c = contact_terms(e, PLANE_STRIDE, ima, imb);
+        store_contact(a, solve_contact(a, c, r3, ima, imb, appa, appb, la, wa, lb, wb), e, sweep, k, t, last, p);
     }
 }
 
@@ -911,77 +920,6 @@ __device__ __forceinline__ void shfl_v3(V3& v, int src) {
     v.x = __shfl_sync(0xffffffffu, v.x, src);
     v.y = __shfl_sync(0xffffffffu, v.y, src);
     v.z = __shfl_sync(0xffffffffu, v.z, src);
-}
-
-// One group spread over a segment of lanes: lane k holds contact k of slot t (k < cnt; a
-// segment of 4 lanes holding a 3-contact group keeps its last lane idle). Every lane loads
-// its own contact's table entries (or, on the warm start, computes its contact's terms
-// from the rows) at once, in lane_prepare, which reads nothing another block writes during
-// the solve; lane_exec then loads the two bodies' velocities and solves the contacts in
-// order k = 0, 1, ..., the lane of contact k updating the velocities and handing them to
-// the segment by shuffles, so each contact sees exactly the velocities of the sequential
-// solve. All 32 lanes of the warp call lane_exec together (lanes without a group have
-// cnt = 0); seg0 is the lane of the segment's contact 0.
-template <bool WARM>
-struct LaneState {  // sweeps >= 1: the contact's table entries are in shared memory
-    uint4 rec;
-    float ima, imb;
-};
-template <>
-struct LaneState<true> {
-    uint4 rec;
-    float ima, imb;
-    WarmTerms W;  // the warm start
-};
-
-// Warm start: the slot record and the contact's terms (from the rows and the bodies' inverse
-// inertia), written to the velocity table.
-__device__ __forceinline__ void lane_prepare_warm(const SolveArgs& a, uint32_t t, uint32_t cnt, uint32_t k,
-                                                  LaneState<true>& S) {
-    S.rec = cnt ? __ldg(&a.batch_rec[t]) : make_uint4(0u, 0u, 0u, 0u);
-    S.ima = S.imb = 0.0f;
-    if (k >= cnt) return;
-    const M3 iwa = load_iw(a.iw, S.rec.x, S.ima);
-    const M3 iwb = load_iw(a.iw, S.rec.y, S.imb);
-    S.W = warm_terms(a, S.rec.z & 0x1fffffffu, k, iwa, iwb, S.ima, S.imb, a.vtab + tix<VT_PLANES>(0, k, t));
-}
-
-template <bool WARM>
-__device__ __forceinline__ void lane_exec(const SolveArgs& a, uint32_t t, uint32_t cnt, uint32_t k, uint32_t seg0,
-                                          uint32_t sweep, uint32_t last, const LaneState<WARM>& S, const float4* sp) {
-    const uint32_t jmax = __reduce_max_sync(0xffffffffu, cnt);
-    if (jmax == 0) return;
-    const uint32_t ia = S.rec.x, ib = S.rec.y, p = S.rec.z & 0x1fffffffu;
-    const uint32_t lane = threadIdx.x & 31u;
-    V3 la{0.0f, 0.0f, 0.0f}, wa = la, lb = la, wb = la;
-    if (cnt) {
-        la = from4(__ldcg(&a.linvel[ia]));
-        wa = from4(__ldcg(&a.angvel[ia]));
-        lb = from4(__ldcg(&a.linvel[ib]));
-        wb = from4(__ldcg(&a.angvel[ib]));
-    }
-    const bool mine = k < cnt;
-    // Every lane of a segment holds the group's inverse masses except an idle fourth lane,
-    // which only forwards velocities; the store below is lane 0's.
-    const bool appa = S.ima > 0.0f, appb = S.imb > 0.0f;
-    float4* e = a.vtab + tix<VT_PLANES>(0, mine ? k : 0u, t);
-    for (uint32_t j = 0; j < jmax; ++j) {
-        if (mine && k == j) {
-            if constexpr (WARM) warm_apply(S.W, la, wa, lb, wb, appa, appb, S.ima, S.imb);
-            else iter_contact(a, sp, blockDim.x, S.ima, S.imb, appa, appb, la, wa, lb, wb, e, sweep, k, t, sweep == last, p);
-        }
-        if (jmax > 1) {  // else every segment is one lane
-            const int src = int(j < cnt ? seg0 + j : lane);
-            shfl_v3(la, src);
-            shfl_v3(wa, src);
-            shfl_v3(lb, src);
-            shfl_v3(wb, src);
-        }
-    }
-    if (cnt && k == 0) {
-        if (appa) { __stcg(&a.linvel[ia], to4(la, 0.0f)); __stcg(&a.angvel[ia], to4(wa, 0.0f)); }
-        if (appb) { __stcg(&a.linvel[ib], to4(lb, 0.0f)); __stcg(&a.angvel[ib], to4(wb, 0.0f)); }
-    }
 }
 
 // Phases 0 .. nphases-1 of a team: phase q is colour q % ncol of sweep q / ncol.
@@ -1129,191 +1067,330 @@ __global__ void __launch_bounds__(256, 2) k_solve(SolveArgs a) {
 }
 
 // ---------------------------------------------------------------- chunked PGS
-struct ChunkArgs {
-    uint32_t P;                        // blocks of the launch = chunks
-    uint32_t W;                        // words per adjacency row
-    const uint32_t* voff;              // [d (P + 1) + b]: chunk b's part of colour batch d
-    const uint32_t* soff;              // the same for the split batches
-    const uint32_t* vsec;              // [(d P + b) 4 + i]: groups of 4 - i rows in chunk b's part of batch d
-    const uint32_t* adj;               // [b W + w]: neighbour bits of chunk b
-    const uint32_t* all_flag;          // nonzero: every chunk is every chunk's neighbour
-    unsigned int* ctr;                 // [b CHUNK_CTR_STRIDE]: phases chunk b has finished
+// k_flow_table writes every contact's velocity table entries; k_solve_flow then runs the warm
+// start, the velocity sweeps and the split sweeps in one cooperative launch without any barrier
+// between warps.
+struct FlowArgs {
+    uint32_t P;             // blocks of the launch = chunks
+    const uint32_t* voff;   // [d (P + 1) + b]: chunk b's part of colour batch d
+    const uint32_t* soff;   // the same for the split batches
+    const uint32_t* vsec;   // [(d P + b) 4 + i]: groups of 4 - i rows in chunk b's part of batch d
+    float4* vel;            // 2 per body: linear velocity | version, angular velocity | version
+    float4* push;           // 2 per body: the push velocities
 };
 
-// Publishes that this block finished every phase before q. The block's global writes are
-// ordered before the release store by the bar.sync.
-__device__ __forceinline__ void chunk_arrive(const ChunkArgs& ch, uint32_t q) {
-    __syncthreads();
-    if (threadIdx.x == 0)
-        asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(ch.ctr + blockIdx.x * CHUNK_CTR_STRIDE), "r"(q)
-                     : "memory");
-}
-
-// Waits until each neighbour has finished every phase before q: one warp polls the
-// neighbours' counters (acquire loads), and the closing bar.sync makes their writes visible
-// to the block. The wait is bounded like team_barrier's.
-__device__ __forceinline__ void chunk_poll(const ChunkArgs& ch, const uint16_t* nb, uint32_t nnb, uint32_t q,
-                                           uint32_t* status) {
-    if (threadIdx.x < 32u) {
-        uint32_t spins = 0;
-        unsigned long long t0 = 0;
-        bool gave_up = false;
-        for (uint32_t k = threadIdx.x; k < nnb && !gave_up; k += 32u) {
-            const unsigned int* c = ch.ctr + uint32_t(nb[k]) * CHUNK_CTR_STRIDE;
-            for (;;) {
-                unsigned int v;
-                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(c) : "memory");
-                if (v >= q) break;
-                if ((++spins & 63u) == 0u) {
-                    const unsigned long long now = globaltimer_ns();
-                    if (t0 == 0) t0 = now;
-                    if ((*(volatile uint32_t*)status & ST_BARRIER_TIMEOUT) || now - t0 > BARRIER_TIMEOUT_NS ||
-                        spins > BARRIER_SPIN_LIMIT) {
-                        atomicOr(status, ST_BARRIER_TIMEOUT);
-                        gave_up = true;
-                        break;
-                    }
-                }
-            }
-        }
-    }
-    __syncthreads();
-}
+constexpr uint32_t FLOW_PLANES = VT_PLANES - 1;  // every plane but the impulses is staged in shared memory
+constexpr size_t FLOW_SMEM = size_t(2) * FLOW_PLANES * CHUNK_TB * sizeof(float4);
 
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
     const unsigned int d = static_cast<unsigned int>(__cvta_generic_to_shared(smem));
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(gmem) : "memory");
 }
 
-// One phase of a chunked block: velocity items are lanes (groups of 4 and 3 rows take 4 lanes,
-// of 2 rows 2, of 1 row one: parts L4, L3, L2, L), padded to a whole warp; split items (one
-// group per thread) follow from LV. Between publishing its progress and polling its
-// neighbours the block starts round 0's loads (item threadIdx.x), which read nothing another
-// block writes during the solve: its slot record and its contact's table entries (copied
-// into shared memory, s_pl[plane][thread]) or its warm-start terms, or its split group's
-// table entries (into L2). The loads come after the publishing bar.sync, which orders this
-// thread's earlier table writes before them. The item-to-thread deal depends only on the
-// bin's counts, so a contact's table entries are read by the thread that wrote them.
-template <bool WARM>
-__device__ __forceinline__ void chunk_phase(const SolveArgs& a, const ChunkArgs& ch, const uint16_t* nb, uint32_t nnb,
-                                            uint32_t q, uint32_t sw, uint32_t iters, uint32_t v0, uint32_t nv,
-                                            uint32_t n4, uint32_t n3, uint32_t n2, uint32_t s0, uint32_t ns,
-                                            float4* s_pl) {
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t L4 = 4u * n4, L3 = L4 + 4u * n3, L2 = L3 + 2u * n2, L = L2 + (nv - n4 - n3 - n2);
-    const uint32_t LV = (L + 31u) & ~31u;
-    auto lane_item = [&](uint32_t i, uint32_t& g, uint32_t& k, uint32_t& cnt, uint32_t& seg0) {
-        g = 0; k = 0; cnt = 0; seg0 = lane;
-        if (i < L4) { g = i >> 2; k = i & 3u; cnt = 4; seg0 = lane & ~3u; }
-        else if (i < L3) { g = n4 + ((i - L4) >> 2); k = i & 3u; cnt = 3; seg0 = lane & ~3u; }
-        else if (i < L2) { g = n4 + n3 + ((i - L3) >> 1); k = i & 1u; cnt = 2; seg0 = lane & ~1u; }
-        else if (i < L) { g = n4 + n3 + n2 + (i - L2); cnt = 1; }
-    };
-    const uint32_t first = threadIdx.x & ~31u;
-    // Round r's table entries of this thread's contact go to s_pl by cp.async.
-    auto stage = [&](uint32_t g, uint32_t k, uint32_t cnt) {
-        if (k < cnt) {
-            const float4* e = a.vtab + tix<VT_PLANES>(0, k, v0 + g);
-            for (uint32_t pl = 0; pl < VT_PLANES; ++pl)
-                cp_async16(&s_pl[pl * blockDim.x + threadIdx.x], e + pl * PLANE_STRIDE);
-        }
-    };
-    if (q) chunk_arrive(ch, q);
-    uint4 rec0 = make_uint4(0u, 0u, 0u, 0u);
-    LaneState<WARM> S0;
-    if (WARM && first < LV) {
-        uint32_t g, k, cnt, seg0;
-        lane_item(threadIdx.x, g, k, cnt, seg0);
-        if constexpr (WARM) lane_prepare_warm(a, v0 + g, cnt, k, S0);
-    } else if (!WARM && first < LV) {
-        uint32_t g, k, cnt, seg0;
-        lane_item(threadIdx.x, g, k, cnt, seg0);
-        stage(g, k, cnt);
-        if (cnt) rec0 = __ldg(&a.batch_rec[v0 + g]);
-    } else if (threadIdx.x >= LV && threadIdx.x - LV < ns && sw >= 2) {
-        prefetch_slot_l2<false>(a, s0 + threadIdx.x - LV, __ldg(&a.split_rec[s0 + threadIdx.x - LV]).z >> 29);
+// A versioned velocity word: one 128-bit access carries the vector and its version, so a reader
+// that finds the version it waits for has the vector that goes with it (no fence, no second
+// round trip).
+__device__ __forceinline__ float4 flow_load(const float4* p) {
+    unsigned long long lo, hi;
+    asm volatile("{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}"
+                 : "=l"(lo), "=l"(hi)
+                 : "l"(p));
+    return make_float4(__uint_as_float(uint32_t(lo)), __uint_as_float(uint32_t(lo >> 32)), __uint_as_float(uint32_t(hi)),
+                       __uint_as_float(uint32_t(hi >> 32)));
+}
+
+__device__ __forceinline__ void flow_store(float4* p, V3 v, uint32_t version) {
+    const unsigned long long lo = (uint64_t(__float_as_uint(v.y)) << 32) | __float_as_uint(v.x);
+    const unsigned long long hi = (uint64_t(version) << 32) | __float_as_uint(v.z);
+    asm volatile("{\n\t.reg .b128 t;\n\tmov.b128 t, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], t;\n\t}" ::"l"(p), "l"(lo),
+                 "l"(hi)
+                 : "memory");
+}
+
+// The two velocity vectors of one body of a group and their versions. deg: the body's groups a
+// sweep (0: not dynamic; its velocities are constant), total: its versions over the whole
+// solve. Version 0 is the body's own array (lin, ang), and the last version goes back there.
+struct FlowBody {
+    uint32_t i, want, total;
+
+    __device__ __forceinline__ void init(uint32_t body, uint32_t rank_deg, uint32_t sweep, uint32_t sweeps) {
+        const uint32_t deg = (rank_deg >> 8) & 0xffu;
+        i = body;
+        want = sweep * deg + (rank_deg & 0xffu);
+        total = deg * sweeps;
     }
-    if (q) chunk_poll(ch, nb, nnb, q, a.status);
-    for (uint32_t base = first; base < LV + ns; base += blockDim.x) {
-        const uint32_t i = base + lane;
-        if (base < LV) {  // warp-uniform: the whole warp runs velocity lanes
-            uint32_t g, k, cnt, seg0;
-            lane_item(i, g, k, cnt, seg0);
-            LaneState<WARM> S;
-            const float4* sp = s_pl + threadIdx.x;
-            if constexpr (WARM) {
-                if (base != first) lane_prepare_warm(a, v0 + g, cnt, k, S);
-                else S = S0;
-            } else {
-                if (base != first) {
-                    stage(g, k, cnt);
-                    S.rec = cnt ? __ldg(&a.batch_rec[v0 + g]) : make_uint4(0u, 0u, 0u, 0u);
-                } else {
-                    S.rec = rec0;
-                }
-                asm volatile("cp.async.wait_all;" ::: "memory");
-                S.ima = k < cnt ? sp[VT_T1 * blockDim.x].w : 0.0f;
-                S.imb = k < cnt ? sp[VT_A2B * blockDim.x].w : 0.0f;
+    // Reads the vectors; false: not yet at the version wanted.
+    __device__ __forceinline__ bool read(const float4* lin, const float4* ang, const float4* ver, V3& l, V3& w) const {
+        const bool own = want == 0u;
+        const float4* v = ver + 2 * size_t(i);
+        const float4 x = flow_load(own ? lin + i : v), y = flow_load(own ? ang + i : v + 1);
+        l = from4(x);
+        w = from4(y);
+        return own || (__float_as_uint(x.w) == want && __float_as_uint(y.w) == want);
+    }
+    __device__ __forceinline__ void write(float4* lin, float4* ang, float4* ver, V3 l, V3 w) const {
+        if (total == 0u) return;
+        const bool end = want + 1u == total;
+        float4* v = ver + 2 * size_t(i);
+        flow_store(end ? lin + i : v, l, end ? 0u : want + 1u);
+        flow_store(end ? ang + i : v + 1, w, end ? 0u : want + 1u);
+    }
+};
+
+// Waits until every lane of the warp that takes part has both its bodies' versions. The wait is
+// bounded like team_barrier's; false: it gave up (the status word says so).
+__device__ __forceinline__ bool flow_wait(bool take, const FlowBody& A, const FlowBody& B, const float4* lin,
+                                          const float4* ang, const float4* ver, V3& la, V3& wa, V3& lb, V3& wb,
+                                          uint32_t* status) {
+    bool ra = !take, rb = !take;
+    uint32_t spins = 0;
+    unsigned long long t0 = 0;
+    for (;;) {
+        if (!ra) ra = A.read(lin, ang, ver, la, wa);
+        if (!rb) rb = B.read(lin, ang, ver, lb, wb);
+        if (__all_sync(0xffffffffu, ra && rb)) return true;
+        if ((++spins & 63u) == 0u) {
+            const unsigned long long now = globaltimer_ns();
+            if (t0 == 0) t0 = now;
+            const bool stop = (*(volatile uint32_t*)status & ST_BARRIER_TIMEOUT) || now - t0 > BARRIER_TIMEOUT_NS ||
+                              spins > BARRIER_SPIN_LIMIT;
+            if (__any_sync(0xffffffffu, stop)) {
+                if ((threadIdx.x & 31u) == 0u) atomicOr(status, ST_BARRIER_TIMEOUT);
+                return false;
             }
-            lane_exec<WARM>(a, v0 + g, cnt, k, seg0, sw, iters, S, sp);
-        } else if (i - LV < ns) {
-            run_item<false>(a, sw - 1u, iters - 1u, s0 + i - LV, __ldg(&a.split_rec[s0 + i - LV]));
         }
     }
 }
 
-// solve() (sequential_impulse.rs:692-705) for worlds without joints, one chunk per block:
-// phase (s, c) runs velocity sweep s (s = 0: warm start) over the block's groups of colour c
-// and split sweep s - 1 over its split groups of colour c (split sweeps touch only the push
-// velocities, so they share the phase). Each block runs its phases in the team kernel's order
-// and waits only on its neighbours, so every body sees the same sequence of updates as under
-// grid barriers: the result is the sequential solve in (colour, pair) order. A block skips
-// the phases it has no groups in. The warm start (phases 0 .. ncol - 1, WARM) and the sweeps
-// (the rest) are two launches of their own code (each keeps its registers); the counters run
-// on across the two, so the second launch starts with every neighbour past the warm start.
-template <bool WARM>
-__global__ void __launch_bounds__(CHUNK_TB, 512 / CHUNK_TB) k_solve_chunks(SolveArgs a, ChunkArgs ch) {
+// Every contact's table entries from its row and its bodies' inverse inertia: one warp per 32 slots
+// and contact index, so the table's planes are written in whole lines.
+__global__ void __launch_bounds__(256) k_flow_table(SolveArgs a) {
+    __shared__ uint32_t s_off[MAX_COLOURS], s_end[MAX_COLOURS];
+    const uint32_t ncol = a.scalars[4];
+    for (uint32_t c = threadIdx.x; c < ncol; c += blockDim.x) {
+        s_off[c] = a.offset[c];
+        s_end[c] = a.end[c];
+    }
+    __syncthreads();
+    if (ncol == 0) return;
+    const uint32_t lane = threadIdx.x & 31u, nblk = (s_end[ncol - 1] + 31u) / 32u * 4u;
+    for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < nblk; w += (gridDim.x * blockDim.x) >> 5) {
+        const uint32_t t = (w >> 2) * 32u + lane, k = w & 3u;
+        uint32_t lo = 0, hi = ncol - 1;  // the batch this block of 32 slots belongs to
+        while (lo < hi) {
+            const uint32_t mid = (lo + hi + 1) >> 1;
+            if (s_off[mid] <= t) lo = mid;
+            else hi = mid - 1;
+        }
+        if (t >= s_end[lo]) continue;  // padding at the batch's end
+        const uint4 rec = __ldg(&a.batch_rec[t]);
+        if (k >= rec.z >> 29) continue;
+        float ima, imb;
+        const M3 iwa = load_iw(a.iw, rec.x, ima);
+        const M3 iwb = load_iw(a.iw, rec.y, imb);
+        warm_terms(a, rec.z & 0x1fffffffu, k, iwa, iwb, ima, imb, a.vtab + tix<VT_PLANES>(0, k, t));
+    }
+}
+
+// The items of a warp: 32 lanes of a phase (sweep, colour) of its chunk. A phase's lanes are its
+// velocity lanes (a group of 4 or 3 rows takes 4 lanes, of 2 rows 2, of 1 row one), padded to a
+// whole warp, then one lane per split group; split sweep s runs in the phases of velocity sweep
+// s + 1 (it touches only the push velocities). Each colour starts its deal at another warp, so that
+// the small colours do not all fall to the first.
+struct FlowItem {
+    uint32_t sweep, c, base;
+};
+
+// solve() (sequential_impulse.rs:692-705) for worlds without joints, one chunk per block. A warp
+// walks its items in (sweep, colour) order and waits, item by item, only for the velocities the
+// item's own bodies have in that order; nothing else holds it up. What a body's update waits
+// for always lies in an earlier phase, every block is resident (cooperative launch) and each warp
+// takes its items in phase order, so the wait always ends. Each body sees its groups in (sweep,
+// colour) order, as under a barrier after every phase: the result is the sequential solve in
+// (colour, pair) order.
+//
+// Lane k of a group's segment holds contact k: the table entries come by cp.async one item ahead
+// (two stages of shared memory, private to the thread), the terms that need no velocity are computed
+// before the wait, and the contacts are solved in order k = 0, 1, ..., the velocities handed from lane
+// to lane by shuffles; the last contact's lane stores the new versions.
+//
+// What bounds it: the chain of dependent contacts. A phase costs a version's way through L2 (about
+// 1,200 cycles from the store to the reader's poll) plus the item itself (about 390 cycles a contact
+// for a lone warp, 700 when three warps share a scheduler); a warp that holds several items of a
+// large colour does them one after the other. Measured against the block-level neighbour waits it
+// replaces (release store, counter poll, then the velocity loads), warm start included, one step's
+// launches: 131,072-body pile with 15 colours and 20 iterations 2,489 -> 1,575 us, 5,681-body pile 934
+// -> 380 us, 16,384 mixed bodies with 15 colours and 10 iterations 604 -> 245 us. 384 threads: at 512 the
+// 128 registers spill (1,628 us on the pile, 528 on the small one), at 320 too few groups are in
+// flight (1,785 us). One group a lane instead of one contact a lane halves the instructions but holds
+// a warp up for the slowest of 32 groups (1,887 us at 160 threads, the most its staging allows).
+__global__ void __launch_bounds__(CHUNK_TB, 1) k_solve_flow(SolveArgs a, FlowArgs f) {
+    extern __shared__ float4 s_pl[];  // [stage][plane][thread]
+    // Per colour: the chunk's part of the batches, and the ends of its velocity lanes on 4 and on 2
+    // lanes a group, of all of them, and the phase's lanes with the split groups.
+    __shared__ uint32_t s_v0[MAX_COLOURS], s_s0[MAX_COLOURS];
+    __shared__ uint4 s_end[MAX_COLOURS];
     const uint32_t ncol = a.scalars[4];
     const uint32_t iters = a.iterations;
-    const uint32_t b = blockIdx.x;
-    extern __shared__ float4 s_pl[];  // [VT_PLANES][blockDim.x]: round 0's table entries
-    __shared__ uint32_t s_v[MAX_COLOURS][2], s_s[MAX_COLOURS][2], s_sec[MAX_COLOURS][3];
-    __shared__ uint16_t s_nb[CHUNK_MAX];
-    __shared__ unsigned int s_nnb;
-    if (threadIdx.x == 0) s_nnb = 0;
+    const uint32_t b = blockIdx.x, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     for (uint32_t c = threadIdx.x; c < ncol; c += blockDim.x) {
-        s_v[c][0] = ch.voff[size_t(c) * (ch.P + 1) + b];
-        s_v[c][1] = ch.voff[size_t(c) * (ch.P + 1) + b + 1];
-        s_s[c][0] = ch.soff[size_t(c) * (ch.P + 1) + b];
-        s_s[c][1] = ch.soff[size_t(c) * (ch.P + 1) + b + 1];
-        for (uint32_t i = 0; i < 3; ++i) s_sec[c][i] = ch.vsec[(size_t(c) * ch.P + b) * 4 + i];
+        const uint32_t v0 = f.voff[size_t(c) * (f.P + 1) + b], nv = f.voff[size_t(c) * (f.P + 1) + b + 1] - v0;
+        const uint32_t s0 = f.soff[size_t(c) * (f.P + 1) + b], ns = f.soff[size_t(c) * (f.P + 1) + b + 1] - s0;
+        const uint32_t* sec = f.vsec + (size_t(c) * f.P + b) * 4;
+        const uint32_t n4 = sec[0] + sec[1], n2 = sec[2];
+        const uint32_t L4 = 4u * n4, L2 = L4 + 2u * n2, L1 = L2 + (nv - n4 - n2);
+        s_v0[c] = v0;
+        s_s0[c] = s0;
+        s_end[c] = make_uint4(L4, L2, L1, ((L1 + 31u) & ~31u) + ns);
     }
-    __syncthreads();  // s_nnb
-    const bool all = *ch.all_flag != 0u;
-    for (uint32_t w = threadIdx.x; w < ch.W; w += blockDim.x) {
-        uint32_t bits = all ? 0xffffffffu : ch.adj[size_t(b) * ch.W + w];
-        while (bits) {
-            const uint32_t j = w * 32u + uint32_t(__ffs(int(bits)) - 1);
-            bits &= bits - 1u;
-            if (j < ch.P && j != b) s_nb[atomicAdd(&s_nnb, 1u)] = uint16_t(j);
-        }
-    }
-    __syncthreads();  // the neighbour list
-    const uint32_t nnb = s_nnb;
-    const uint32_t nphases = WARM ? ncol : (iters + 1) * ncol;
-    for (uint32_t q = WARM ? 0u : ncol; q < nphases; ++q) {
-        const uint32_t c = q % ncol, sw = q / ncol;
-        const uint32_t v0 = s_v[c][0], nv = s_v[c][1] - v0;
-        const uint32_t s0 = s_s[c][0], ns = sw >= 1 ? s_s[c][1] - s0 : 0u;
-        if (nv + ns == 0) continue;
-        const uint32_t n4 = s_sec[c][0], n3 = s_sec[c][1], n2 = s_sec[c][2];
-        chunk_phase<WARM>(a, ch, s_nb, nnb, q, sw, iters, v0, nv, n4, n3, n2, s0, ns, s_pl);
-    }
-    // Every later phase of this block is empty: publish the end.
     __syncthreads();
-    if (threadIdx.x == 0)
-        asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(ch.ctr + b * CHUNK_CTR_STRIDE), "r"(nphases)
-                     : "memory");
+    const uint32_t nwarps = blockDim.x >> 5;
+    auto start = [&](uint32_t c) { return ((warp + 5u * c) % nwarps) * 32u; };
+    // The colours with an item for this warp, a bit each (from sweep 1 on; in sweep 0 some may
+    // hold split groups only).
+    unsigned long long mine0 = 0, mine1 = 0;
+    for (uint32_t c0 = 0; c0 < ncol; c0 += 32u) {
+        const uint32_t c = c0 + lane;
+        const unsigned long long w = __ballot_sync(0xffffffffu, c < ncol && start(c) < s_end[c].w);
+        if (c0 < 64u) mine0 |= w << c0;
+        else mine1 |= w << (c0 - 64u);
+    }
+    if ((mine0 | mine1) == 0ull) return;
+    // The next item at or after `it`; false: none.
+    auto settle = [&](FlowItem& it) {
+        while (it.base >= (it.sweep ? s_end[it.c].w : (s_end[it.c].z + 31u) & ~31u)) {
+            const uint32_t c = it.c + 1u;
+            unsigned long long lo = c < 64u ? mine0 & (~0ull << c) : 0ull;
+            unsigned long long hi = c < 64u ? mine1 : (c < 128u ? mine1 & (~0ull << (c - 64u)) : 0ull);
+            if ((lo | hi) == 0ull) {
+                if (++it.sweep > iters) return false;
+                lo = mine0;
+                hi = mine1;
+            }
+            it.c = lo ? uint32_t(__ffsll((long long)lo) - 1) : 63u + uint32_t(__ffsll((long long)hi));
+            it.base = start(it.c);
+        }
+        return true;
+    };
+    // What an item's lane needs: its slot, contact, record and the contact's impulses (which this
+    // lane wrote a sweep before); its other table entries head for a stage.
+    struct Lane {
+        uint4 rec;
+        uint32_t t, k;
+        float4 r3;
+    };
+    auto fetch = [&](const FlowItem& it, uint32_t stage) {
+        Lane L;
+        L.rec = make_uint4(0u, 0u, 0u, 0u);
+        L.t = 0;
+        L.k = 0;
+        L.r3 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        const uint4 end = s_end[it.c];
+        const uint32_t LV = (end.z + 31u) & ~31u, i = it.base + lane;
+        if (it.base < LV) {
+            if (i < end.z) {
+                uint32_t g = end.x / 4u + (end.y - end.x) / 2u + (i - end.y);
+                if (i < end.x) { g = i >> 2; L.k = i & 3u; }
+                else if (i < end.y) { g = (end.x / 4u) + ((i - end.x) >> 1); L.k = i & 1u; }
+                L.t = s_v0[it.c] + g;
+                L.rec = __ldg(&a.batch_rec[L.t]);
+                // (The fourth lane of a 3-row group copies entries nothing reads: no wait for the record.)
+                const float4* e = a.vtab + tix<VT_PLANES>(0, L.k, L.t);
+                L.r3 = e[VT_IMP * PLANE_STRIDE];
+#pragma unroll
+                for (uint32_t pl = 0; pl < FLOW_PLANES; ++pl)
+                    cp_async16(&s_pl[(stage * FLOW_PLANES + pl) * CHUNK_TB + threadIdx.x], e + pl * PLANE_STRIDE);
+            }
+        } else if (i < end.w) {
+            L.t = s_s0[it.c] + (i - LV);
+            L.rec = __ldg(&a.split_rec[L.t]);
+            if (it.sweep >= 2) prefetch_slot_l2<false>(a, L.t, L.rec.z >> 29);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        return L;
+    };
+    FlowItem cur{0u, 0u, start(0)};
+    if (!settle(cur)) return;
+    Lane L = fetch(cur, 0);
+    uint32_t stage = 0;
+    for (;;) {
+        FlowItem nxt = cur;
+        nxt.base += blockDim.x;
+        const bool more = settle(nxt);
+        const bool same = nxt.c == cur.c && nxt.base == cur.base;  // the warp's only item of a sweep
+        Lane N = L;
+        if (more && !same) {
+            N = fetch(nxt, stage ^ 1u);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        const uint32_t cnt = L.rec.z >> 29, p = L.rec.z & 0x1fffffffu, ia = L.rec.x, ib = L.rec.y;
+        V3 la{0.0f, 0.0f, 0.0f}, wa = la, lb = la, wb = la;
+        FlowBody A, B;
+        if (cur.base < ((s_end[cur.c].z + 31u) & ~31u)) {
+            const uint32_t k = L.k, t = L.t;
+            const bool mine = k < cnt;
+            const uint32_t jmax = __reduce_max_sync(0xffffffffu, cnt);
+            const uint32_t seg0 = lane - k;
+            A.init(ia, L.rec.w & 0xffffu, cur.sweep, iters + 1u);
+            B.init(ib, L.rec.w >> 16, cur.sweep, iters + 1u);
+            const float4* sp = s_pl + stage * (FLOW_PLANES * CHUNK_TB) + threadIdx.x;
+            ContactTerms C{};
+            float ima = 0.0f, imb = 0.0f;
+            if (mine) {
+                ima = sp[VT_T1 * CHUNK_TB].w;
+                imb = sp[VT_A2B * CHUNK_TB].w;
+                C = contact_terms(sp, CHUNK_TB, ima, imb);
+            }
+            C.pin();  // before the wait, not after it
+            const bool appa = ima > 0.0f, appb = imb > 0.0f;
+            ContactResult X{};
+            if (!flow_wait(mine && k == 0u, A, B, a.linvel, a.angvel, f.vel, la, wa, lb, wb, a.status)) break;
+            for (uint32_t j = 0; j < jmax; ++j) {
+                if (mine && k == j) {
+                    if (cur.sweep == 0u) {
+                        apply(la, wa, lb, wb, appa, appb, ima, imb, C.n, C.ana, C.anb, L.r3.x);
+                        apply(la, wa, lb, wb, appa, appb, ima, imb, C.t1, C.a1a, C.a1b, L.r3.y);
+                        apply(la, wa, lb, wb, appa, appb, ima, imb, C.t2, C.a2a, C.a2b, L.r3.z);
+                    } else {
+                        X = solve_contact(a, C, L.r3, ima, imb, appa, appb, la, wa, lb, wb);
+                    }
+                    if (k + 1u == cnt) {
+                        A.write(a.linvel, a.angvel, f.vel, la, wa);
+                        B.write(a.linvel, a.angvel, f.vel, lb, wb);
+                    }
+                }
+                if (j + 1u < jmax) {
+                    const int src = int(j < cnt ? seg0 + j : lane);
+                    shfl_v3(la, src);
+                    shfl_v3(wa, src);
+                    shfl_v3(lb, src);
+                    shfl_v3(wb, src);
+                }
+            }
+            if (mine && cur.sweep) {
+                store_contact(a, X, a.vtab + tix<VT_PLANES>(0, k, t), cur.sweep, k, t, cur.sweep == iters, p);
+                if (same) N.r3 = X.r3;
+            }
+        } else {
+            const uint32_t sw = cur.sweep - 1u;
+            A.init(ia, L.rec.w & 0xffffu, sw, iters);
+            B.init(ib, L.rec.w >> 16, sw, iters);
+            if (!flow_wait(cnt != 0u, A, B, a.push_lin, a.push_ang, f.push, la, wa, lb, wb, a.status)) break;
+            if (cnt) {
+                bool appa, appb;
+                split_group(a, L.t, p, cnt, ia, ib, sw == 0u, sw + 1u == iters, la, wa, lb, wb, appa, appb);
+                A.write(a.push_lin, a.push_ang, f.push, la, wa);
+                B.write(a.push_lin, a.push_ang, f.push, lb, wb);
+            }
+        }
+        if (!more) break;
+        cur = nxt;
+        L = N;
+        if (!same) stage ^= 1u;
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
 // ---------------------------------------------------------------- per-world PGS (batched worlds)
@@ -1781,19 +1858,12 @@ static int pgs_mode() {
 static int g_last_solver_kind = 0;
 int last_solver_kind() { return g_last_solver_kind; }
 
-constexpr size_t CHUNK_SMEM = size_t(VT_PLANES) * CHUNK_TB * sizeof(float4);
-
 static int chunk_grid() {
     static int grid = 0;
     if (!grid) {
-        int g[2];
-        const void* fns[2] = {(const void*)k_solve_chunks<true>, (const void*)k_solve_chunks<false>};
-        for (int i = 0; i < 2; ++i) {
-            check_cuda(cudaFuncSetAttribute(fns[i], cudaFuncAttributeMaxDynamicSharedMemorySize, int(CHUNK_SMEM)),
-                       "smem attribute");
-            g[i] = coop_grid(fns[i], CHUNK_TB, CHUNK_SMEM);
-        }
-        grid = std::min(g[0], g[1]);  // both launches cut the bodies into the same chunks
+        check_cuda(cudaFuncSetAttribute((const void*)k_solve_flow, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        int(FLOW_SMEM)), "smem attribute");
+        grid = coop_grid((const void*)k_solve_flow, CHUNK_TB, FLOW_SMEM);
     }
     if (grid > int(CHUNK_MAX)) throw CudaError{cudaErrorInvalidValue, "chunked PGS: more blocks than chunk slots"};
     return grid;
@@ -1835,7 +1905,7 @@ void run_solver(const WorldView& w, const uint64_t* pairs, uint32_t npairs, Pair
     // Colouring (cooperative launch).
     check_cuda(cudaMemsetAsync(pd.barrier.p, 0, 16 * sizeof(unsigned int), s), "memset barrier");
     ColourArgs ca{pd.scalars.p + 2, pd.contact_pairs.p, pairs, w.b.iw, pd.colour.p, pd.body_prio.p, pd.body_mask.p,
-                  pd.body_dup.p, pd.entries.p, seed_colours ? 1u : 0u, pd.barrier.p, status_dev};
+                  pd.body_dup.p, chunked ? pd.body_used.p : nullptr, pd.entries.p, seed_colours ? 1u : 0u, pd.barrier.p, status_dev};
     // Two blocks per SM: enough threads for a pile's groups, and the rounds' grid barriers
     // are cheaper than with every block the SM could hold.
     static int colour_grid = 0;
@@ -1855,32 +1925,25 @@ void run_solver(const WorldView& w, const uint64_t* pairs, uint32_t npairs, Pair
     uint32_t g = std::min<uint32_t>((npairs + TB - 1) / TB, 148u * 8u);
     // Chunks: each body's chunk; the (colour, chunk) counts and the touch sets come with the
     // colour histograms.
-    uint32_t P = 0, W = 0;
-    uint32_t *vhist = nullptr, *shist = nullptr, *all_flag = nullptr;
+    uint32_t P = 0;
+    uint32_t *vhist = nullptr, *shist = nullptr;
     if (chunked) {
         P = uint32_t(chunk_grid());
-        W = (P + 31u) / 32u;
         const uint32_t n = w.nbodies;
+        const bool tree = morton_leaf && tree_m;
         pd.chunk_of.reserve(std::max<uint32_t>(n, 1));
-        pd.chunk_touch.reserve(size_t(std::max<uint32_t>(n, 1)) * CHUNK_TOUCH);
         pd.chunk_hist.reserve(size_t(MAX_COLOURS) * P * 5);
         pd.chunk_off.reserve(2 * size_t(MAX_COLOURS) * (P + 1) + size_t(MAX_COLOURS) * P * 4);
-        pd.chunk_adj.reserve(size_t(P) * W + 1);
-        pd.chunk_ctr.reserve(size_t(P) * CHUNK_CTR_STRIDE);
+        pd.flow_vel.reserve(4 * size_t(std::max<uint32_t>(n, 1)));
         vhist = pd.chunk_hist.p;
         shist = pd.chunk_hist.p + size_t(MAX_COLOURS) * P * 4;
-        all_flag = pd.chunk_adj.p + size_t(P) * W;
         check_cuda(cudaMemsetAsync(pd.chunk_hist.p, 0, size_t(MAX_COLOURS) * P * 5 * sizeof(uint32_t), s), "memset");
-        check_cuda(cudaMemsetAsync(pd.chunk_touch.p, 0xff, size_t(n) * CHUNK_TOUCH * sizeof(uint32_t), s), "memset");
-        check_cuda(cudaMemsetAsync(pd.chunk_adj.p, 0, (size_t(P) * W + 1) * sizeof(uint32_t), s), "memset");
-        check_cuda(cudaMemsetAsync(pd.chunk_of.p, 0, size_t(n) * sizeof(uint32_t), s), "memset");
-        const uint32_t lim = (morton_leaf && tree_m) ? tree_m : n;
-        k_chunk_of<<<std::min<uint32_t>((lim + TB - 1) / TB, 148u * 8u), TB, 0, s>>>(
-            n, P, (morton_leaf && tree_m) ? morton_leaf : nullptr, tree_m, pd.chunk_of.p);
+        k_chunk_of<<<std::min<uint32_t>((4 * n + TB - 1) / TB, 148u * 8u), TB, 0, s>>>(
+            n, P, tree ? morton_leaf : nullptr, tree_m, pd.chunk_of.p, pd.flow_vel.p);
     }
     k_colour_hist<<<g, TB, 0, s>>>(pd.scalars.p + 2, pd.contact_pairs.p, pd.colour.p, pd.row_count.p, pd.rows.p,
                                    pd.colour_count.p, pd.split_count.p, pd.flags.p, sub_hist, pairs, w.b.iw,
-                                   pd.chunk_of.p, P, vhist, shist, pd.chunk_touch.p, all_flag);
+                                   pd.chunk_of.p, P, vhist, shist, pd.body_used.p);
     k_colour_scan<<<1, 32, 0, s>>>(pd.colour_count.p, pd.colour_offset.p, pd.colour_cursor.p, pd.split_count.p,
                                    pd.split_offset.p, pd.split_cursor.p, pd.barrier.p, pd.scalars.p, pd.colour_remap.p,
                                    sub_hist, sub_cursor, chunked ? 1u : 0u);
@@ -1895,30 +1958,23 @@ void run_solver(const WorldView& w, const uint64_t* pairs, uint32_t npairs, Pair
     k_colour_scatter<<<g, TB, 0, s>>>(pd.scalars.p + 2, pd.contact_pairs.p, pairs, pd.row_count.p, pd.colour.p,
                                       pd.flags.p, sub_cursor, pd.split_cursor.p, pd.batch_rec.p,
                                       pd.split_rec.p, pd.entries.p, pd.colour_remap.p, pd.chunk_of.p, w.b.iw, P,
-                                      vhist, shist);
-    if (chunked)
-        k_chunk_adjacency<<<std::min<uint32_t>((w.nbodies + TB - 1) / TB, 148u * 8u), TB, 0, s>>>(
-            w.nbodies, pd.chunk_of.p, pd.chunk_touch.p, W, pd.chunk_adj.p);
+                                      vhist, shist, pd.body_used.p);
     mark(5);
     // Slot capacity: every group plus the 32-alignment padding of each batch.
     const size_t slots = (size_t(npairs) + 32u * (MAX_COLOURS + 1) + 31u) & ~size_t(31);
     pd.vtab.reserve(size_t(VT_PLANES) * 4 * slots);
     pd.stab.reserve(size_t(ST_PLANES) * 4 * slots);
     if (chunked) {
-        check_cuda(cudaMemsetAsync(pd.chunk_ctr.p, 0, size_t(P) * CHUNK_CTR_STRIDE * sizeof(unsigned int), s),
-                   "memset");
         SolveArgs sa{pd.rows.p, pd.batch_rec.p, pd.colour_offset.p, pd.colour_cursor.p, pd.split_rec.p,
                      pd.split_offset.p, pd.split_cursor.p, pd.scalars.p, w.b.linvel, w.b.angvel, w.b.push_lin,
                      w.b.push_ang, w.b.iw, pd.vtab.p, pd.stab.p, pd.rec.sweeps,
                      pd.barrier.p, status_dev, sp.inv_dt, sp.info.restitution_velocity_threshold,
                      sp.info.num_iterations, JointsDev{}, sp.info.damping};
-        ChunkArgs ch{P, W, voff, soff, vsec, pd.chunk_adj.p, all_flag, pd.chunk_ctr.p};
-        void* args[] = {&sa, &ch};
-        check_cuda(cudaLaunchCooperativeKernel((const void*)k_solve_chunks<true>, dim3(P), dim3(CHUNK_TB), args,
-                                               CHUNK_SMEM, s), "chunked warm-start launch");
-        if (sp.info.num_iterations)
-            check_cuda(cudaLaunchCooperativeKernel((const void*)k_solve_chunks<false>, dim3(P), dim3(CHUNK_TB), args,
-                                                   CHUNK_SMEM, s), "chunked solve launch");
+        FlowArgs fa{P, voff, soff, vsec, pd.flow_vel.p, pd.flow_vel.p + 2 * size_t(w.nbodies)};
+        k_flow_table<<<std::min<uint32_t>((npairs + TB / 4 - 1) / (TB / 4), 148u * 8u), TB, 0, s>>>(sa);
+        void* args[] = {&sa, &fa};
+        check_cuda(cudaLaunchCooperativeKernel((const void*)k_solve_flow, dim3(P), dim3(CHUNK_TB), args, FLOW_SMEM, s),
+                   "chunked solve launch");
         g_last_solver_kind = 2;
     } else {
         launch_solve(w, pd, sp, status_dev, s, with_joints ? joints : nullptr);
