@@ -202,6 +202,7 @@ struct World {
     DevBuf<float2> ccd_par_d;
     DevBuf<float> ccd_clamp_d;
     uint32_t nccd = 0;
+    CcdScratch ccd_scratch;
     DevBuf<uint64_t> suppressed_d;  // sorted keys of the pairs a joint keeps from colliding
     uint32_t nsuppressed = 0;
 
@@ -960,7 +961,7 @@ struct World {
         launch_ccd_sweep(b, shapes_d.p, hull_d.p, ccd_ids_d.p, ccd_par_d.p, nccd, n, batch ? world_off_d.p : nullptr,
                          world_of, sp.suppressed, sp.nsuppressed, dt, ccd_clamp_d.p, status,
                          batch ? nullptr : bp.node_rec.p, bp.leaf_body.p, batch ? 0 : bp.tree_m, bp.unbounded.p,
-                         batch ? 0u : bp.nunb, stream);
+                         batch ? 0u : bp.nunb, ccd_scratch, stream);
         // 6c + 7 + 8: deactivation, pose integration with the split push, force clear.
         launch_integrate_positions(b, n, dt, info.split_impulse_turn_erp, stream);
         launch_ccd_apply(b, ccd_ids_d.p, ccd_clamp_d.p, nccd, dt, stream);

@@ -214,3 +214,49 @@ def test_ccd_in_batched_worlds_sweeps_only_its_own_world(gpu):
     assert abs(st[1, 1] - 0.9) <= 0.05 and clamps[1] < 1.0
     assert st[3, 1] < -0.5 and clamps[3] == 1.0
     assert w.stats()["device_status"] == 0
+
+
+@pytest.mark.parametrize("n", [250, 1500, 3000])
+def test_ccd_casts_do_not_depend_on_how_many_run(gpu, n):
+    """Few casts take a warp each, more share one: spheres that only the plates stop, all in one
+    world against 125 at a time, must be clamped at the same fractions bit for bit."""
+    rng = np.random.default_rng(11)
+    pos = np.stack([rng.uniform(-8, 8, n), rng.uniform(1.0, 4.0, n), rng.uniform(-8, 8, n)], axis=1)
+    vel = np.stack([rng.uniform(-60, 60, n), rng.uniform(-300, -60, n), np.zeros(n)], axis=1)
+
+    def clamps(lo, hi):
+        w = gpu.World(gravity=(0.0, 0.0, 0.0))
+        kinds = [w.add_shape(orc.BOX, [0.7, 0.04, 0.7]), w.add_shape(orc.CAPSULE, [0.2, 0.5]),
+                 w.hull([[x, y, z] for x in (-0.5, 0.5) for y in (-0.1, 0.2) for z in (-0.4, 0.6)]), w.add_shape(orc.SPHERE, [0.5])]
+        for px in range(-4, 5):
+            for pz in range(-4, 5):
+                w.add_body(kinds[(px + 2 * pz) % 4], (px * 1.8, 0.25 * ((px * pz) % 3), pz * 1.8), mass=0.0)
+        sph = w.add_shape(orc.SPHERE, [0.1])
+        first = w.num_bodies
+        for k in range(lo, hi):
+            w.add_body(sph, pos[k], linvel=vel[k], mass=1.0, group=2, mask=1)
+        w.set_ccd(first, np.full(hi - lo, 0.05), np.full(hi - lo, 0.1))
+        w.step(DT)
+        assert w.stats()["device_status"] == 0
+        return w.ccd_clamps()[first:]
+
+    together = clamps(0, n)
+    apart = np.concatenate([clamps(lo, min(lo + 125, n)) for lo in range(0, n, 125)])
+    assert np.count_nonzero(together < 1.0) > n // 4
+    np.testing.assert_array_equal(together, apart)
+
+
+def test_ccd_with_more_candidates_than_the_casting_kernel_takes(gpu):
+    """Twelve plates under one fast sphere (more than 8 candidates: cast where they are found), and
+    two under another."""
+    t = Twin(gpu)
+    plate = t.shape(orc.BOX, [1.0, 0.02, 1.0])
+    for k in range(12):
+        t.body(plate, (0.0, -0.4 * k, 0.0), mass=0.0)
+    for k in range(2):
+        t.body(plate, (9.0, -0.4 * k, 0.0), quat=(0.0, 0.0, math.sin(0.2), math.cos(0.2)), mass=0.0)
+    sph = t.shape(orc.SPHERE, [0.15])
+    for x in (0.1, 9.1):
+        t.ccd(t.body(sph, (x, 1.5, 0.0), linvel=(0.0, -400.0, 0.0), mass=1.0), 0.05, 0.15)
+    t.step()
+    assert (t.g.ccd_clamps() < 1.0).sum() == 2
