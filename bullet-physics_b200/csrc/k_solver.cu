@@ -460,6 +460,7 @@ __device__ __forceinline__ uint32_t claim_slot(uint32_t* cursor, uint32_t c) {
 // and r the count of the bits below the group's colour; both ride in the group's slot record.
 constexpr uint32_t CHUNK_MAX = 1024;         // blocks of a chunked launch
 constexpr uint32_t CHUNK_TB = 384;           // threads of a chunk block (one block per SM)
+constexpr uint32_t SMALL_TB = 128;           // threads of a block when one chunk has many (a warp a scheduler)
 
 __device__ __forceinline__ uint32_t group_owner(uint32_t ia, uint32_t ib, const float4* __restrict__ iw,
                                                 const uint32_t* __restrict__ chunk_of, uint32_t P) {
@@ -1071,7 +1072,8 @@ __global__ void __launch_bounds__(256, 2) k_solve(SolveArgs a) {
 // start, the velocity sweeps and the split sweeps in one cooperative launch without any barrier
 // between warps.
 struct FlowArgs {
-    uint32_t P;             // blocks of the launch = chunks
+    uint32_t P;             // chunks
+    uint32_t bpc;           // blocks a chunk: the launch has P bpc blocks
     const uint32_t* voff;   // [d (P + 1) + b]: chunk b's part of colour batch d
     const uint32_t* soff;   // the same for the split batches
     const uint32_t* vsec;   // [(d P + b) 4 + i]: groups of 4 - i rows in chunk b's part of batch d
@@ -1080,7 +1082,7 @@ struct FlowArgs {
 };
 
 constexpr uint32_t FLOW_PLANES = VT_PLANES - 1;  // every plane but the impulses is staged in shared memory
-constexpr size_t FLOW_SMEM = size_t(2) * FLOW_PLANES * CHUNK_TB * sizeof(float4);
+constexpr size_t flow_smem(uint32_t tb) { return size_t(2) * FLOW_PLANES * tb * sizeof(float4); }
 
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
     const unsigned int d = static_cast<unsigned int>(__cvta_generic_to_shared(smem));
@@ -1224,7 +1226,8 @@ struct FlowItem {
 // 128 registers spill (1,628 us on the pile, 528 on the small one), at 320 too few groups are in
 // flight (1,785 us). One group a lane instead of one contact a lane halves the instructions but holds
 // a warp up for the slowest of 32 groups (1,887 us at 160 threads, the most its staging allows).
-__global__ void __launch_bounds__(CHUNK_TB, 1) k_solve_flow(SolveArgs a, FlowArgs f) {
+template <uint32_t TB>
+__global__ void __launch_bounds__(TB, 1) k_solve_flow(SolveArgs a, FlowArgs f) {
     extern __shared__ float4 s_pl[];  // [stage][plane][thread]
     // Per colour: the chunk's part of the batches, and the ends of its velocity lanes on 4 and on 2
     // lanes a group, of all of them, and the phase's lanes with the split groups.
@@ -1232,8 +1235,9 @@ __global__ void __launch_bounds__(CHUNK_TB, 1) k_solve_flow(SolveArgs a, FlowArg
     __shared__ uint4 s_end[MAX_COLOURS];
     const uint32_t ncol = a.scalars[4];
     const uint32_t iters = a.iterations;
-    const uint32_t b = blockIdx.x, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    for (uint32_t c = threadIdx.x; c < ncol; c += blockDim.x) {
+    const uint32_t b = blockIdx.x / f.bpc, lane = threadIdx.x & 31u;  // the chunk
+    const uint32_t nwarps = f.bpc * (TB / 32u), warp = (blockIdx.x % f.bpc) * (TB / 32u) + (threadIdx.x >> 5);
+    for (uint32_t c = threadIdx.x; c < ncol; c += TB) {
         const uint32_t v0 = f.voff[size_t(c) * (f.P + 1) + b], nv = f.voff[size_t(c) * (f.P + 1) + b + 1] - v0;
         const uint32_t s0 = f.soff[size_t(c) * (f.P + 1) + b], ns = f.soff[size_t(c) * (f.P + 1) + b + 1] - s0;
         const uint32_t* sec = f.vsec + (size_t(c) * f.P + b) * 4;
@@ -1244,7 +1248,6 @@ __global__ void __launch_bounds__(CHUNK_TB, 1) k_solve_flow(SolveArgs a, FlowArg
         s_end[c] = make_uint4(L4, L2, L1, ((L1 + 31u) & ~31u) + ns);
     }
     __syncthreads();
-    const uint32_t nwarps = blockDim.x >> 5;
     auto start = [&](uint32_t c) { return ((warp + 5u * c) % nwarps) * 32u; };
     // The colours with an item for this warp, a bit each (from sweep 1 on; in sweep 0 some may
     // hold split groups only).
@@ -1299,7 +1302,7 @@ __global__ void __launch_bounds__(CHUNK_TB, 1) k_solve_flow(SolveArgs a, FlowArg
                 L.r3 = e[VT_IMP * PLANE_STRIDE];
 #pragma unroll
                 for (uint32_t pl = 0; pl < FLOW_PLANES; ++pl)
-                    cp_async16(&s_pl[(stage * FLOW_PLANES + pl) * CHUNK_TB + threadIdx.x], e + pl * PLANE_STRIDE);
+                    cp_async16(&s_pl[(stage * FLOW_PLANES + pl) * TB + threadIdx.x], e + pl * PLANE_STRIDE);
             }
         } else if (i < end.w) {
             L.t = s_s0[it.c] + (i - LV);
@@ -1315,7 +1318,7 @@ __global__ void __launch_bounds__(CHUNK_TB, 1) k_solve_flow(SolveArgs a, FlowArg
     uint32_t stage = 0;
     for (;;) {
         FlowItem nxt = cur;
-        nxt.base += blockDim.x;
+        nxt.base += nwarps * 32u;
         const bool more = settle(nxt);
         const bool same = nxt.c == cur.c && nxt.base == cur.base;  // the warp's only item of a sweep
         Lane N = L;
@@ -1335,13 +1338,13 @@ __global__ void __launch_bounds__(CHUNK_TB, 1) k_solve_flow(SolveArgs a, FlowArg
             const uint32_t seg0 = lane - k;
             A.init(ia, L.rec.w & 0xffffu, cur.sweep, iters + 1u);
             B.init(ib, L.rec.w >> 16, cur.sweep, iters + 1u);
-            const float4* sp = s_pl + stage * (FLOW_PLANES * CHUNK_TB) + threadIdx.x;
+            const float4* sp = s_pl + stage * (FLOW_PLANES * TB) + threadIdx.x;
             ContactTerms C{};
             float ima = 0.0f, imb = 0.0f;
             if (mine) {
-                ima = sp[VT_T1 * CHUNK_TB].w;
-                imb = sp[VT_A2B * CHUNK_TB].w;
-                C = contact_terms(sp, CHUNK_TB, ima, imb);
+                ima = sp[VT_T1 * TB].w;
+                imb = sp[VT_A2B * TB].w;
+                C = contact_terms(sp, TB, ima, imb);
             }
             C.pin();  // before the wait, not after it
             const bool appa = ima > 0.0f, appb = imb > 0.0f;
@@ -1463,26 +1466,17 @@ __device__ __forceinline__ void run_group_shared(const SolveArgs& a, uint32_t t,
     if (appb) { lin[lb_i] = to4(lb, 0.0f); ang[lb_i] = to4(wb, 0.0f); }
 }
 
-// The whole PGS of world w by `nt` threads (lane = 0 .. nt - 1), `sm` its 4 * nb float4 of
-// shared memory, `C` its context. Every thread of the CTA (block mode) or of the warp (warp
-// mode) calls it; every early return is taken by all of them together, so every sync is
-// reached by all of them.
+// The range of world w's groups and their colours (A.colour), by `nt` threads (lane = 0 .. nt - 1):
+// `mask` its 4 * nb words of shared memory, `C` its context. Every thread of the CTA (block mode) or
+// of the warp (warp mode) calls it, and every sync is reached by all of them.
 template <bool WARP>
-__device__ void solve_world(const WorldSolveArgs& A, uint32_t w, uint32_t lane, uint32_t nt, float4* sm, WorldCtx& C) {
+__device__ __forceinline__ void colour_world(const WorldSolveArgs& A, uint32_t b0, uint32_t nb, uint32_t lane, uint32_t nt,
+                                             unsigned long long* mask, WorldCtx& C) {
     const SolveArgs& a = A.a;
-    const uint32_t b0 = A.world_off[w], nb = A.world_off[w + 1] - b0;
-    float4* lin = sm;
-    float4* ang = sm + nb;
-    float4* plin = sm + 2 * nb;
-    float4* pang = sm + 3 * nb;
-    // Colouring scratch over the push-velocity region (24 of its 32 bytes per body).
-    unsigned long long* mask = reinterpret_cast<unsigned long long*>(plin);
     unsigned long long* best0 = mask + nb;
     unsigned long long* best1 = best0 + nb;
     unsigned long long* dup = best1 + nb;  // seeded colours claimed twice at a body
     for (uint32_t i = lane; i < nb; i += nt) {
-        lin[i] = __ldcg(&A.linvel[b0 + i]);
-        ang[i] = __ldcg(&A.angvel[b0 + i]);
         mask[i] = 0ull;
         best0[i] = 0ull;
         best1[i] = 0ull;
@@ -1502,15 +1496,8 @@ __device__ void solve_world(const WorldSolveArgs& A, uint32_t w, uint32_t lane, 
     }
     ws_sync<WARP>();
     const uint32_t g0 = C.g0, g1 = C.g1;
-    if (g0 == g1 && !a.j.ncol) {  // no rows in this world: its velocities stay as they are
-        if (lane == 0) {  // an empty record (the adjoint's reverse pass reads every world's)
-            A.wcol[size_t(w) * WS_STRIDE] = g0;
-            A.wcol[size_t(w) * WS_STRIDE + 1] = 0;
-        }
-        return;
-    }
     auto dyn = [&](uint32_t i) { return inv_mass_of(a.iw, i) > 0.0f; };
-    // 1. Jones-Plassmann rounds: an uncoloured group wins when its priority is the largest
+    // Jones-Plassmann rounds: an uncoloured group wins when its priority is the largest
     //    among the uncoloured groups at each of its dynamic bodies; a winner takes the lowest
     //    colour free at both bodies (winners of one round share no dynamic body).
     auto seed_of = [&](uint32_t g) -> uint32_t {  // last step's colour + 1 (0: none)
@@ -1588,6 +1575,34 @@ __device__ void solve_world(const WorldSolveArgs& A, uint32_t w, uint32_t lane, 
         for (uint32_t i = lane; i < nb; i += nt) other[i] = 0ull;
         if (won) atomicSub(&C.left, won);
         ws_sync<WARP>();
+    }
+}
+
+// The whole PGS of world w by `nt` threads (lane = 0 .. nt - 1), `sm` its 4 * nb float4 of
+// shared memory, `C` its context. Every thread of the CTA (block mode) or of the warp (warp
+// mode) calls it; every early return is taken by all of them together, so every sync is
+// reached by all of them.
+template <bool WARP>
+__device__ void solve_world(const WorldSolveArgs& A, uint32_t w, uint32_t lane, uint32_t nt, float4* sm, WorldCtx& C) {
+    const SolveArgs& a = A.a;
+    const uint32_t b0 = A.world_off[w], nb = A.world_off[w + 1] - b0;
+    float4* lin = sm;
+    float4* ang = sm + nb;
+    float4* plin = sm + 2 * nb;
+    float4* pang = sm + 3 * nb;
+    for (uint32_t i = lane; i < nb; i += nt) {
+        lin[i] = __ldcg(&A.linvel[b0 + i]);
+        ang[i] = __ldcg(&A.angvel[b0 + i]);
+    }
+    // 1. Colours, with the push-velocity region as scratch.
+    colour_world<WARP>(A, b0, nb, lane, nt, reinterpret_cast<unsigned long long*>(plin), C);
+    const uint32_t g0 = C.g0, g1 = C.g1;
+    if (g0 == g1 && !a.j.ncol) {  // no rows in this world: its velocities stay as they are
+        if (lane == 0) {  // an empty record (the adjoint's reverse pass reads every world's)
+            A.wcol[size_t(w) * WS_STRIDE] = g0;
+            A.wcol[size_t(w) * WS_STRIDE + 1] = 0;
+        }
+        return;
     }
     // 2. Colour batches: histogram, offsets, scatter of the slot records.
     for (uint32_t g = g0 + lane; g < g1; g += nt) {
@@ -1687,6 +1702,136 @@ __device__ void solve_world(const WorldSolveArgs& A, uint32_t w, uint32_t lane, 
         __stcg(&A.angvel[b0 + i], ang[i]);
         __stcg(&A.push_lin[b0 + i], plin[i]);
         __stcg(&A.push_ang[b0 + i], pang[i]);
+    }
+}
+
+// What k_world_prep leaves for k_solve_flow: the batches of one chunk.
+struct WorldPrepOut {
+    uint32_t *offset, *end;       // colour batch starts and ends (slots)
+    uint4* split_rec;
+    uint32_t *voff, *soff, *vsec; // FlowArgs
+    uint32_t* split_flag;         // scratch, one a group
+    float4* vel;                  // FlowArgs::vel and, 2 nb further on, push
+};
+
+// A plain world's colours and batches by one block, for k_solve_flow to solve with many: one launch
+// instead of the global colouring's eleven, which for a world this small cost more than the solve.
+// The colours are solve_world's; a batch holds its groups of 4 rows first, then 3, 2, 1.
+__global__ void __launch_bounds__(512) k_world_prep(WorldSolveArgs A, WorldPrepOut O) {
+    extern __shared__ float4 ws_dyn[];
+    __shared__ WorldCtx C;
+    __shared__ uint32_t hist[WS_MAX_COLOURS * 4], scur[WS_MAX_COLOURS];
+    const SolveArgs& a = A.a;
+    const uint32_t lane = threadIdx.x, nt = blockDim.x, nb = A.world_off[1];
+    unsigned long long* mask = reinterpret_cast<unsigned long long*>(ws_dyn);
+    for (uint32_t i = lane; i < 4 * nb; i += nt) O.vel[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (uint32_t i = lane; i < WS_MAX_COLOURS * 4; i += nt) hist[i] = 0;
+    colour_world<false>(A, 0u, nb, lane, nt, mask, C);
+    const uint32_t K = C.g1;
+    // The colours of a body's groups and split groups (the masks above may hold dropped seeds too).
+    unsigned long long *used = mask + nb, *split_used = used + nb;
+    for (uint32_t i = lane; i < 2 * nb; i += nt) used[i] = 0ull;
+    __syncthreads();
+    auto dyn = [&](uint32_t i) { return inv_mass_of(a.iw, i) > 0.0f; };
+    uint32_t rows = 0, split_groups = 0, split_rows = 0;
+    for (uint32_t g = lane; g < K; g += nt) {
+        const uint32_t c = A.colour[g];
+        if (c >= WS_MAX_COLOURS) continue;  // left uncoloured (round limit; the status word says so)
+        const uint32_t p = A.contact_pairs[g], cnt = A.row_count[p];
+        const uint64_t key = A.pairs[p];
+        uint32_t nsplit = 0;
+        for (uint32_t k = 0; k < cnt; ++k) nsplit += a.rows[(size_t(p) * 4 + k) * ROW_F4 + 5].z != 0.0f ? 1u : 0u;
+        O.split_flag[g] = nsplit;
+        atomicAdd(&hist[c * 4 + (4u - cnt)], 1u);
+        atomicMax(&C.ncol, c + 1u);
+        rows += cnt;
+        if (nsplit) {
+            ++split_groups;
+            split_rows += nsplit;
+            atomicAdd(&C.split_hist[c], 1u);
+        }
+        const unsigned long long bit = 1ull << c;
+        for (uint32_t side = 0; side < 2; ++side) {
+            const uint32_t x = side ? key_hi(key) : key_lo(key);
+            if (!dyn(x)) continue;
+            atomicOr(&used[x], bit);
+            if (nsplit) atomicOr(&split_used[x], bit);
+        }
+    }
+    if (rows) atomicAdd(&C.rows, rows);
+    if (split_groups) {
+        atomicAdd(&C.split_groups, split_groups);
+        atomicAdd(&C.split_rows, split_rows);
+    }
+    __syncthreads();
+    const uint32_t ncol = C.ncol;
+    if (lane < 32u) {  // batch offsets: two colours a lane
+        uint32_t n[2], s[2], nsum = 0, ssum = 0;
+        for (uint32_t k = 0; k < 2; ++k) {
+            const uint32_t c = 2u * lane + k;
+            n[k] = hist[4 * c] + hist[4 * c + 1] + hist[4 * c + 2] + hist[4 * c + 3];
+            s[k] = C.split_hist[c];
+            nsum += n[k];
+            ssum += s[k];
+        }
+        uint32_t v = nsum, w = ssum;
+        for (uint32_t o = 1; o < 32; o <<= 1) {
+            const uint32_t x = __shfl_up_sync(0xffffffffu, v, o), y = __shfl_up_sync(0xffffffffu, w, o);
+            if (lane >= o) { v += x; w += y; }
+        }
+        v -= nsum;
+        w -= ssum;
+        for (uint32_t k = 0; k < 2; ++k) {
+            const uint32_t c = 2u * lane + k;
+            if (c < ncol) {
+                O.offset[c] = O.voff[2 * c] = A.wcol[2 + c] = v;
+                O.end[c] = O.voff[2 * c + 1] = v + n[k];
+                O.soff[2 * c] = w;
+                O.soff[2 * c + 1] = w + s[k];
+                A.colour_count[c] = n[k];
+                A.split_count[c] = s[k];
+            }
+            for (uint32_t r = 0; r < 4; ++r) {
+                const uint32_t cnt = hist[4 * c + r];
+                if (c < ncol) O.vsec[4 * c + r] = cnt;
+                hist[4 * c + r] = v;  // the scatter's cursor
+                v += cnt;
+            }
+            scur[c] = w;
+            w += s[k];
+            if (c + 1u == ncol) {
+                O.offset[ncol] = A.wcol[2 + ncol] = v;
+                A.scalars[3] = C.rows;
+                A.scalars[4] = ncol;
+                A.scalars[5] = C.split_groups;
+                A.scalars[10] = C.split_rows;
+            }
+        }
+        if (lane == 0) {
+            A.wcol[0] = 0u;
+            A.wcol[1] = ncol;
+        }
+    }
+    __syncthreads();
+    for (uint32_t g = lane; g < K; g += nt) {
+        const uint32_t c = A.colour[g];
+        if (c >= WS_MAX_COLOURS) continue;
+        const uint32_t p = A.contact_pairs[g], cnt = A.row_count[p];
+        const uint64_t key = A.pairs[p];
+        const uint32_t ia = key_lo(key), ib = key_hi(key);
+        const unsigned long long below = (1ull << c) - 1ull;
+        auto rank = [&](const unsigned long long* m, uint32_t i) {
+            return dyn(i) ? uint32_t(__popcll(m[i] & below)) | (uint32_t(__popcll(m[i])) << 8) : 0u;
+        };
+        uint4 rec = make_uint4(ia, ib, p | (cnt << 29), rank(used, ia) | (rank(used, ib) << 16));
+        A.recs[atomicAdd(&hist[c * 4 + (4u - cnt)], 1u)] = rec;
+        if (O.split_flag[g]) {
+            rec.w = rank(split_used, ia) | (rank(split_used, ib) << 16);
+            O.split_rec[atomicAdd(&scur[c], 1u)] = rec;
+        }
+        // The colour rides in the manifold's meta bits to seed next step's colouring.
+        float* mw = &A.entries[size_t(p) * ENTRY_F4 + 2].w;
+        *mw = __uint_as_float((__float_as_uint(*mw) & ~(0xffu << META_COLOUR_SHIFT)) | ((c + 1u) << META_COLOUR_SHIFT));
     }
 }
 
@@ -1855,15 +2000,24 @@ static int pgs_mode() {
     return mode;
 }
 
+// Plain worlds of up to 1,024 bodies: one block colours and batches, many solve, four warps each.
+// A phase then costs a trip through L2 (1.8 us) but a warp holds only a few groups, where one block's
+// threads solve theirs in turn, each contact after a table load. Measured on box stacks, colouring
+// and solve: 1,000 bodies 504 us by one block, 209 / 200 / 196 us with 64 / 32 / 16 bodies a block;
+// 512 bodies 262 and 137, 216 bodies 111 and 109, 125 bodies 88 and 105, 8 bodies 48 and 58. Hence
+// the line at 256 bodies, below which one block solves the world alone.
+constexpr uint32_t SMALL_BODIES_PER_BLOCK = 16;
+constexpr uint32_t SMALL_FLOW_MIN_BODIES = 256;
+
 static int g_last_solver_kind = 0;
 int last_solver_kind() { return g_last_solver_kind; }
 
 static int chunk_grid() {
     static int grid = 0;
     if (!grid) {
-        check_cuda(cudaFuncSetAttribute((const void*)k_solve_flow, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        int(FLOW_SMEM)), "smem attribute");
-        grid = coop_grid((const void*)k_solve_flow, CHUNK_TB, FLOW_SMEM);
+        check_cuda(cudaFuncSetAttribute((const void*)k_solve_flow<CHUNK_TB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        int(flow_smem(CHUNK_TB))), "smem attribute");
+        grid = coop_grid((const void*)k_solve_flow<CHUNK_TB>, CHUNK_TB, flow_smem(CHUNK_TB));
     }
     if (grid > int(CHUNK_MAX)) throw CudaError{cudaErrorInvalidValue, "chunked PGS: more blocks than chunk slots"};
     return grid;
@@ -1970,11 +2124,11 @@ void run_solver(const WorldView& w, const uint64_t* pairs, uint32_t npairs, Pair
                      w.b.push_ang, w.b.iw, pd.vtab.p, pd.stab.p, pd.rec.sweeps,
                      pd.barrier.p, status_dev, sp.inv_dt, sp.info.restitution_velocity_threshold,
                      sp.info.num_iterations, JointsDev{}, sp.info.damping};
-        FlowArgs fa{P, voff, soff, vsec, pd.flow_vel.p, pd.flow_vel.p + 2 * size_t(w.nbodies)};
+        FlowArgs fa{P, 1u, voff, soff, vsec, pd.flow_vel.p, pd.flow_vel.p + 2 * size_t(w.nbodies)};
         k_flow_table<<<std::min<uint32_t>((npairs + TB / 4 - 1) / (TB / 4), 148u * 8u), TB, 0, s>>>(sa);
         void* args[] = {&sa, &fa};
-        check_cuda(cudaLaunchCooperativeKernel((const void*)k_solve_flow, dim3(P), dim3(CHUNK_TB), args, FLOW_SMEM, s),
-                   "chunked solve launch");
+        check_cuda(cudaLaunchCooperativeKernel((const void*)k_solve_flow<CHUNK_TB>, dim3(P), dim3(CHUNK_TB), args,
+                                               flow_smem(CHUNK_TB), s), "chunked solve launch");
         g_last_solver_kind = 2;
     } else {
         launch_solve(w, pd, sp, status_dev, s, with_joints ? joints : nullptr);
@@ -2025,8 +2179,9 @@ bool build_world_plan(const std::vector<uint32_t>& world_off, uint32_t block, ui
     if (nw) check_cuda(cudaMemcpyAsync(plan.list.p, order.data(), nw * sizeof(uint32_t), cudaMemcpyHostToDevice, s), "h2d");
     check_cuda(cudaStreamSynchronize(s), "sync");  // the host vectors go out of scope
     // Without this opt-in, dynamic shared memory is limited to 48 KB minus the kernel's static part.
+    // The limit is the function's, for every world of the process: always the largest plan's.
     check_cuda(cudaFuncSetAttribute(block > 256 ? (const void*)k_world_solve<512> : (const void*)k_world_solve<256>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)), "smem attribute");
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_cap)), "smem attribute");
     plan.ncta = uint32_t(cta.size());
     plan.block = block;
     plan.tau = tau;
@@ -2063,6 +2218,9 @@ void run_world_solver(const WorldView& w, const uint64_t* pairs, uint32_t npairs
                                               pd.scalars.p + 2, int(npairs), s), "select");
     }
     mark(5);
+    // A plain world's contacts go to many blocks; with joints, and a world of a few bodies, to one
+    // block with its velocities in shared memory.
+    const bool prep = !with_joints && nworlds == 1 && plan.block > 256 && w.nbodies >= SMALL_FLOW_MIN_BODIES;
     const size_t slots = (size_t(npairs) + 32u * (MAX_COLOURS + 1) + 31u) & ~size_t(31);
     pd.vtab.reserve(size_t(VT_PLANES) * 4 * slots);
     pd.stab.reserve(size_t(ST_PLANES) * 4 * slots);
@@ -2091,7 +2249,22 @@ void run_world_solver(const WorldView& w, const uint64_t* pairs, uint32_t npairs
     A.plan = plan.dev();
     A.entries = pd.entries.p;
     A.seed = seed_colours ? 1u : 0u;
-    if (plan.block > 256) k_world_solve<512><<<plan.ncta, plan.block, plan.smem, s>>>(A);
+    if (prep) {
+        const uint32_t n = w.nbodies;
+        pd.chunk_off.reserve(size_t(WS_MAX_COLOURS) * 8);
+        pd.flow_vel.reserve(4 * size_t(n));
+        uint32_t *voff = pd.chunk_off.p, *soff = voff + 2 * WS_MAX_COLOURS, *vsec = soff + 2 * WS_MAX_COLOURS;
+        const WorldPrepOut O{pd.colour_offset.p, pd.colour_cursor.p, pd.split_rec.p, voff, soff, vsec, pd.flags.p,
+                             pd.flow_vel.p};
+        k_world_prep<<<1, 512, size_t(n) * 32, s>>>(A, O);
+        const uint32_t blocks = std::min<uint32_t>((n + SMALL_BODIES_PER_BLOCK - 1) / SMALL_BODIES_PER_BLOCK,
+                                                   uint32_t(device_sms()));
+        k_flow_table<<<std::min<uint32_t>((npairs + TB / 4 - 1) / (TB / 4), 148u * 8u), TB, 0, s>>>(A.a);
+        FlowArgs fa{1u, blocks, voff, soff, vsec, pd.flow_vel.p, pd.flow_vel.p + 2 * size_t(n)};
+        void* args[] = {&A.a, &fa};
+        check_cuda(cudaLaunchCooperativeKernel((const void*)k_solve_flow<SMALL_TB>, dim3(blocks), dim3(SMALL_TB), args,
+                                               flow_smem(SMALL_TB), s), "solve launch");
+    } else if (plan.block > 256) k_world_solve<512><<<plan.ncta, plan.block, plan.smem, s>>>(A);
     else k_world_solve<256><<<plan.ncta, plan.block, plan.smem, s>>>(A);
     check_cuda(cudaGetLastError(), "world solve launch");
     mark(6);

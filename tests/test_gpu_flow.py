@@ -56,3 +56,42 @@ def test_chunked_kernel_equals_team_kernel(tmp_path, kind, iters, steps):
         assert r.returncode == 0, r.stderr[-1500:]
         states.append(np.load(out))
     np.testing.assert_array_equal(*states)
+
+
+@pytest.mark.parametrize("n", [255, 256, 1024, 1025])
+def test_plain_worlds_on_both_sides_of_the_lines(gpu_oracle, n):
+    """One block (up to 255 bodies), one block to prepare and many to solve (256 to 1,024), chunks
+    (more): each step equals the oracle's from the same state."""
+    bgpu, orc, scenes = gpu_oracle
+    s = scenes.large_pile(nx=6, nz=6, ny=-(-(n - 1) // 36), seed=n, spacing=1.0)
+    for f in ("shape_of", "pos", "quat", "linvel", "angvel", "mass", "friction", "restitution"):
+        setattr(s, f, getattr(s, f)[:n])
+    g, o = s.build_gpu(bgpu), s.build_oracle(orc)
+    for _ in range(12):
+        g.step(s.dt)
+        o.set_solve_order(g.solve_order())
+        o.step(s.dt)
+        a, b = g.state(), o.state()
+        assert np.abs(a[:, :13] - b[:, :13]).max() <= 1e-5 * max(1.0, np.abs(b[:, :13]).max())
+    assert g.num_bodies == n and g.stats()["num_contacts"] > n and g.stats()["device_status"] == 0
+
+
+@pytest.fixture(scope="module")
+def gpu_oracle():
+    sys.path[:0] = [os.path.join(ROOT, "bullet-physics_b200"), os.path.join(ROOT, "tests")]
+    import bgpu
+    import oracle_api
+    import scenes
+    return bgpu, oracle_api, scenes
+
+
+def test_worlds_of_different_sizes_step_side_by_side(gpu_oracle):
+    """The shared-memory limit of the per-world kernel is the process's: a later, smaller world must
+    not lower it for an earlier one."""
+    bgpu, _, scenes = gpu_oracle
+    big = scenes.batched_worlds(4, seed=1, min_bodies=200, max_bodies=220).build_gpu(bgpu)
+    big.set_tuning(256, 0x7fffffff)
+    small = scenes.batched_worlds(4, seed=1, min_bodies=8, max_bodies=9).build_gpu(bgpu)
+    for w in (big, small, big):
+        w.step(1.0 / 60.0, 30)
+        assert w.stats()["device_status"] == 0
