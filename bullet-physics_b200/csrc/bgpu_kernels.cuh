@@ -67,6 +67,62 @@ struct DevBuf {
     }
 };
 
+// One launch of an ordered scan over tiles (k_scan.cuh).
+struct TileScan {
+    unsigned long long* words;  // one per tile
+    uint32_t* ticket;           // tiles are dealt in this order
+    uint32_t base, epoch;       // the ticket when the launch begins; the launch's mark in the words
+    uint32_t* status;
+};
+struct TileScanBuf {
+    DevBuf<unsigned long long> words;
+    DevBuf<uint32_t> ticket;
+    uint32_t tickets = 0, epoch = 0;
+    // The state of a launch of `tiles` blocks, each of which takes one ticket. No word needs
+    // clearing between launches: an earlier launch's words carry an earlier epoch.
+    TileScan begin(uint32_t tiles, uint32_t* status, cudaStream_t s) {
+        if (!ticket.p) {
+            ticket.reserve(1);
+            check_cuda(cudaMemsetAsync(ticket.p, 0, sizeof(uint32_t), s), "memset");
+        }
+        if (tiles > words.cap || epoch + 1u >= (1u << 30)) {
+            words.reserve(tiles);
+            check_cuda(cudaMemsetAsync(words.p, 0, words.cap * sizeof(unsigned long long), s), "memset");
+            epoch = 0;
+        }
+        const TileScan t{words.p, ticket.p, tickets, ++epoch, status};
+        tickets += tiles;
+        return t;
+    }
+};
+
+// Small counters that a step's first kernel clears for the kernels after it.
+struct StepReset {
+    static constexpr int MAX = 10;
+    uint32_t* w[MAX] = {};
+    uint32_t n[MAX] = {};
+    int count = 0;
+    uint32_t* owned = nullptr;           // the old manifolds' owned marks, as many as
+    const uint32_t* owned_n = nullptr;   // this device count says
+    void add(uint32_t* p, size_t words) {
+        w[count] = p;
+        n[count++] = uint32_t(words);
+    }
+};
+// What a step's last kernel hands to the host (pinned, written by the device).
+struct HostStats {
+    uint32_t scalars[16];
+    uint32_t status;
+    uint32_t cache_count;
+};
+struct StepEnd {
+    HostStats* host;
+    const uint32_t *scalars, *status, *cache_count;
+    const uint32_t* simulate;  // per world; copied to
+    uint32_t* prev_simulate;   // the next step's previous flags
+    uint32_t worlds;
+};
+
 // ---------------------------------------------------------------- device helpers shared by the solver and its adjoint
 constexpr unsigned int BARRIER_SPIN_LIMIT = 1u << 26;
 constexpr unsigned long long BARRIER_TIMEOUT_NS = 2000000000ull;  // 2 s: phases take microseconds
@@ -158,11 +214,13 @@ __device__ __forceinline__ size_t tix(uint32_t plane, uint32_t k, uint32_t t) {
 constexpr uint32_t PLANE_STRIDE = 4 * 32;
 
 // ---------------------------------------------------------------- body kernels (k_body.cu)
+// The first kernel of a step (it also clears the step's counters) and, CCD clamps apart, the last.
 void launch_integrate_velocities(const BodyDev& b, const Shape* shapes, const float4* hull, uint32_t n, float dt,
-                                 cudaStream_t s);
+                                 const StepReset& reset, cudaStream_t s);
 void launch_initial_aabbs(const BodyDev& b, const Shape* shapes, const float4* hull, uint32_t first, uint32_t n,
                           cudaStream_t s);
-void launch_integrate_positions(const BodyDev& b, uint32_t n, float dt, float turn_erp, cudaStream_t s);
+void launch_integrate_positions(const BodyDev& b, uint32_t n, float dt, float turn_erp, const StepEnd& end,
+                                cudaStream_t s);
 // Casts found by the CCD sweep, for the kernel that runs them.
 struct CcdScratch {
     DevBuf<uint4> items;
@@ -330,6 +388,8 @@ struct Islands {
 struct StepParams {
     float dt, inv_dt;
     SolverParams info;
+    const uint32_t *simulate = nullptr, *prev_simulate = nullptr;  // per world (none outside a step)
+    uint32_t worlds = 0;
     const uint64_t* suppressed = nullptr;  // sorted keys of pairs whose collisions a joint disables
     uint32_t nsuppressed = 0;
 };
@@ -379,6 +439,7 @@ struct PairData {
     DevBuf<uint32_t> scalars;      // [0] analytic count [1] convex count [2] contact pairs [3] contacts
                                    // [4] colours [5] split pairs [6] detect total [7] manifolds
                                    // [8] [9] cache compaction counts [10] split contacts [11] largest split batch
+                                   // [12] every world prunes its vanished manifolds
                                    // [ROUTE_COUNT0 + r] pairs on narrow-phase route r [CAPTURE_COUNT]
     // Solver batches
     DevBuf<uint32_t> contact_pairs;  // pair ids with rows (ascending)
@@ -401,10 +462,33 @@ struct PairData {
     DevBuf<unsigned long long> body_used;
     DevBuf<float4> flow_vel;
     DevBuf<uint32_t> flags;          // selection flags
+    TileScanBuf list_scan, cache_scan;
     DevBuf<uint32_t> sel_a, sel_b;   // cache compaction lists
-    DevBuf<unsigned char> cub_tmp;
     DevBuf<unsigned int> barrier;    // grid barrier words + round counters
     RecordDev rec;                   // set by an adjoint tape while it records a step
+    // The counters a step clears at its start.
+    void reserve_counters() {
+        scalars.reserve(32);
+        colour_count.reserve(132);
+        split_count.reserve(132);
+        colour_sub.reserve(2 * 4 * MAX_COLOURS);
+        barrier.reserve(16);
+    }
+    void add_counters(StepReset& r) {
+        r.add(scalars.p, 32);
+        r.add(colour_count.p, 132);
+        r.add(split_count.p, 132);
+        r.add(colour_sub.p, 4 * MAX_COLOURS);
+        r.add(barrier.p, 16);
+    }
+    // The same for a solve outside a step.
+    void clear_counters(cudaStream_t s) {
+        StepReset r;
+        reserve_counters();
+        add_counters(r);
+        for (int k = 0; k < r.count; ++k)
+            check_cuda(cudaMemsetAsync(r.w[k], 0, r.n[k] * sizeof(uint32_t), s), "memset counters");
+    }
     void reserve(size_t npairs, size_t nbodies, size_t old_manifolds) {
         status.reserve(npairs);
         entries.reserve(npairs * ENTRY_F4);
@@ -414,7 +498,8 @@ struct PairData {
         rows.reserve(npairs * 4 * ROW_F4);
         route_list.reserve(size_t(CAPTURE_LIST + 1) * npairs);
         old_owned.reserve(old_manifolds + 1);
-        scalars.reserve(CAPTURE_COUNT + 1);
+        static_assert(CAPTURE_COUNT < 32, "counters");
+        reserve_counters();
         contact_pairs.reserve(npairs);
         colour.reserve(npairs);
         body_prio.reserve(nbodies);
@@ -422,10 +507,8 @@ struct PairData {
         body_dup.reserve(2 * nbodies);
         body_used.reserve(4 * nbodies);
         colour_remap.reserve(132);
-        colour_count.reserve(132);
         colour_offset.reserve(132);
         colour_cursor.reserve(132);
-        split_count.reserve(132);
         split_offset.reserve(132);
         split_cursor.reserve(132);
         batch_rec.reserve(npairs + 32 * 130);  // batches start on multiples of 32
@@ -433,7 +516,6 @@ struct PairData {
         flags.reserve(npairs + old_manifolds + 1);
         sel_a.reserve(npairs);
         sel_b.reserve(old_manifolds + 1);
-        barrier.reserve(16);
     }
     PairDataDev dev() {
         return PairDataDev{status.p, entries.p, detect.p, detect_n.p, row_count.p, rows.p, route_list.p, old_owned.p,
@@ -459,6 +541,7 @@ struct WorldView {
     const float4* hull;
     uint32_t nbodies;
     bool has_mesh = false;  // some shape is a triangle mesh (the mesh narrow-phase launch runs)
+    bool has_convex = true; // some shape is a capsule or hull (the GJK/EPA launch runs)
 };
 
 // Pair pass: classify + refresh, narrow phase, capture. Fills PairData for `npairs`.
@@ -527,7 +610,7 @@ void run_wait_selftest(unsigned long long limit_ns, unsigned int* ctr, uint32_t*
 // simulate / prev_simulate hold one flag per world, indexed through world_of (null: one world).
 void run_cache_update(const uint64_t* pairs, uint32_t npairs, const Manifolds& old_cache, PairData& pd,
                       Manifolds& next, const uint32_t* world_of, const uint32_t* simulate_flag,
-                      const uint32_t* prev_simulate, cudaStream_t s);
+                      const uint32_t* prev_simulate, uint32_t* status_dev, cudaStream_t s);
 
 // ---------------------------------------------------------------- adjoint (k_adjoint.cu)
 // One recorded step as the reverse solve reads it (device pointers).

@@ -46,9 +46,14 @@ __device__ __forceinline__ V3 gyroscopic_implicit(V3 inv, Q q, V3 w, float step)
 }
 
 // step.rs:306-363 + body.rs:1113-1126, 1175-1181, shapes/mod.rs:350, util.rs:52-55.
+// Also clears the step's counters (a dozen memsets otherwise, each a launch).
 __global__ void k_integrate_velocities(BodyDev b, const Shape* __restrict__ shapes, const float4* __restrict__ hull,
-                                       uint32_t n, float dt, float aabb_margin) {
+                                       uint32_t n, float dt, float aabb_margin, StepReset reset) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    for (int k = 0; k < reset.count; ++k)
+        for (uint32_t t = i; t < reset.n[k]; t += gridDim.x * blockDim.x) reset.w[k][t] = 0u;
+    if (reset.owned)
+        for (uint32_t t = i, m = *reset.owned_n; t < m; t += gridDim.x * blockDim.x) reset.owned[t] = 0u;
     if (i >= n) return;
     uint4 info = b.info[i];
     float4 p4 = b.pos[i];
@@ -134,8 +139,14 @@ __device__ __forceinline__ void interpolate_pose(V3& p, Q& q, V3 lv, V3 av, floa
 
 // step.rs:1059-1061 (update_deactivation, body.rs:639-657) fused with
 // step.rs:1171-1215 (integrate_position + split-impulse push) and step.rs:1272 (clear forces).
-__global__ void k_integrate_positions(BodyDev b, uint32_t n, float dt, float turn_erp) {
+// Also keeps the worlds' simulate flags for the next step and writes the step's counters to the
+// host's pinned memory (a copy each otherwise).
+__global__ void k_integrate_positions(BodyDev b, uint32_t n, float dt, float turn_erp, StepEnd end) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    for (uint32_t w = i; w < end.worlds; w += gridDim.x * blockDim.x) end.prev_simulate[w] = end.simulate[w];
+    if (i < 16u) end.host->scalars[i] = end.scalars[i];
+    else if (i == 16u) end.host->status = *end.status;
+    else if (i == 17u) end.host->cache_count = *end.cache_count;
     if (i >= n) return;
     uint4 info = b.info[i];
     bool stat = (info.y & BF_STATIC) != 0;
@@ -203,9 +214,8 @@ void launch_compute_iw(const BodyDev& b, uint32_t n, cudaStream_t s) {
 }
 
 void launch_integrate_velocities(const BodyDev& b, const Shape* shapes, const float4* hull, uint32_t n, float dt,
-                                 cudaStream_t s) {
-    if (n == 0) return;
-    k_integrate_velocities<<<(n + 255) / 256, 256, 0, s>>>(b, shapes, hull, n, dt, 0.02f);
+                                 const StepReset& reset, cudaStream_t s) {
+    k_integrate_velocities<<<n ? (n + 255) / 256 : 1u, 256, 0, s>>>(b, shapes, hull, n, dt, 0.02f, reset);
 }
 
 void launch_initial_aabbs(const BodyDev& b, const Shape* shapes, const float4* hull, uint32_t first, uint32_t n,
@@ -214,9 +224,9 @@ void launch_initial_aabbs(const BodyDev& b, const Shape* shapes, const float4* h
     k_initial_aabbs<<<(n + 255) / 256, 256, 0, s>>>(b, shapes, hull, first, n, 0.02f);
 }
 
-void launch_integrate_positions(const BodyDev& b, uint32_t n, float dt, float turn_erp, cudaStream_t s) {
-    if (n == 0) return;
-    k_integrate_positions<<<(n + 255) / 256, 256, 0, s>>>(b, n, dt, turn_erp);
+void launch_integrate_positions(const BodyDev& b, uint32_t n, float dt, float turn_erp, const StepEnd& end,
+                                cudaStream_t s) {
+    k_integrate_positions<<<n ? (n + 255) / 256 : 1u, 256, 0, s>>>(b, n, dt, turn_erp, end);
 }
 
 namespace {

@@ -22,7 +22,6 @@ struct Simplex {
 
 __device__ __forceinline__ void keep1(Simplex& s, V3 a) { s.p[0] = a; s.n = 1; }
 __device__ __forceinline__ void keep2(Simplex& s, V3 a, V3 b) { s.p[0] = a; s.p[1] = b; s.n = 2; }
-__device__ __forceinline__ void keep3(Simplex& s, V3 a, V3 b, V3 c) { s.p[0] = a; s.p[1] = b; s.p[2] = c; s.n = 3; }
 
 // gjk.rs:889-906
 __device__ __forceinline__ V3 closest_segment(V3 a, V3 b, Simplex& keep) {
@@ -715,7 +714,6 @@ __global__ void __launch_bounds__(CCD_CAST_THREADS) k_ccd_cast(BodyDev b, const 
     const uint32_t g = total <= CCD_WARP_CASTS ? 32u : (total <= 2u * CCD_WARP_CASTS ? 16u : 8u);
     const uint32_t td = g == 32u ? 4u : (g == 16u ? 3u : 2u), bd = td + 1u;
     const uint32_t segs = 32u / g, sl = lane % g;
-    const uint32_t mask = (g == 32u ? 0xffffffffu : ((1u << g) - 1u) << (lane - sl));
     // The segment's cast (the same values on all its lanes) and the lane's walk.
     enum { TERNARY, CLOSEST, BISECT, IDLE };
     int phase = IDLE;

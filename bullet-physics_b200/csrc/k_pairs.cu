@@ -485,7 +485,10 @@ __global__ void k_classify(BodyDev b, const Shape* __restrict__ shapes, const ui
     }
     uint32_t route = route_of(shapes[ia.x].type, shapes[ib.x].type);
     pd.status[p] = PS_DETECT | (route << 8);
-    if (route == NP_NONE) return;
+    if (route == NP_NONE) {  // plane-plane pairs detect nothing: their manifold (if any) is dropped
+        store_meta_only(ne, 0u);
+        return;
+    }
     // One list per route (route r in [(r - 1) P, r P), P = npairs), so that the narrow
     // phase's warps run one shape routine each instead of every route their lanes hold.
     const uint32_t slot = claim_route_slot(&pd.scalars[ROUTE_COUNT0], route);
@@ -1021,13 +1024,6 @@ __global__ void __launch_bounds__(CAPTURE_TB) k_capture(BodyDev b, const Shape* 
     }
 }
 
-// Plane-plane pairs (route NP_NONE) detect nothing: their manifold (if any) is dropped.
-__global__ void k_drop_undetectable(uint32_t npairs, PairDataDev pd) {
-    uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= npairs) return;
-    if (pd.status[p] == (PS_DETECT | (NP_NONE << 8))) store_meta_only(pd.entries + size_t(p) * ENTRY_F4, 0u);
-}
-
 constexpr uint32_t COLLIDE_QUERIES_TB = 64;
 
 __global__ __launch_bounds__(COLLIDE_QUERIES_TB) void k_collide_queries(const Shape* __restrict__ shapes, const float4* __restrict__ hull, uint32_t n,
@@ -1095,17 +1091,15 @@ void run_pair_pass(const WorldView& w, const uint64_t* pairs, uint32_t npairs, c
     (void)simulate_flag;
     if (npairs == 0) return;
     PairDataDev d = pd.dev();
-    check_cuda(cudaMemsetAsync(pd.scalars.p, 0, 8 * sizeof(uint32_t), s), "memset scalars");
-    check_cuda(cudaMemsetAsync(pd.scalars.p + ROUTE_COUNT0, 0, (CAPTURE_COUNT + 1 - ROUTE_COUNT0) * sizeof(uint32_t), s),
-               "memset scalars");
     const int TB = 128;
     k_classify<<<(npairs + TB - 1) / TB, TB, 0, s>>>(w.b, w.shapes, pairs, npairs, old_cache.keys.p,
                                                      old_cache.entries.p, old_cache.count_dev, sp, d);
-    k_drop_undetectable<<<(npairs + 255) / 256, 256, 0, s>>>(npairs, d);
     uint32_t grid = std::min<uint32_t>((npairs + TB - 1) / TB, 148u * 16u);
     k_narrow_analytic<<<grid, NARROW_ANALYTIC_TB, 0, s>>>(w.b, w.shapes, w.hull, pairs, npairs, d);
-    uint32_t cgrid = std::min<uint32_t>((npairs + 63) / 64, 148u * 8u);
-    k_narrow_convex<<<cgrid, 64, 0, s>>>(w.b, w.shapes, w.hull, pairs, npairs, d, status_dev);
+    if (w.has_convex) {
+        uint32_t cgrid = std::min<uint32_t>((npairs + 63) / 64, 148u * 8u);
+        k_narrow_convex<<<cgrid, 64, 0, s>>>(w.b, w.shapes, w.hull, pairs, npairs, d, status_dev);
+    }
     if (w.has_mesh) {
         const uint32_t mgrid = std::min<uint32_t>((npairs + MESH_WARPS - 1) / MESH_WARPS, 148u * 8u);
         k_narrow_mesh<<<mgrid, 32 * MESH_WARPS, 0, s>>>(w.b, w.shapes, w.hull, pairs, npairs, d, status_dev);

@@ -34,7 +34,7 @@
 #include <cstring>
 #include <cooperative_groups.h>
 #include <cub/cub.cuh>
-#include "bgpu_kernels.cuh"
+#include "k_scan.cuh"
 
 namespace bgpu {
 
@@ -61,9 +61,45 @@ __device__ __forceinline__ M3 load_iw(const float4* __restrict__ iw, uint32_t i,
     return M3{V3{a.x, a.y, a.z}, V3{a.w, b.x, b.y}, V3{b.z, b.w, c.x}};
 }
 
-__global__ void k_flag_contact_pairs(uint32_t npairs, const uint32_t* __restrict__ row_count, uint32_t* flags) {
-    uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p < npairs) flags[p] = row_count[p] > 0 ? 1u : 0u;
+// The pairs with rows, ascending, and their number; scalars[12]: every world prunes (step.rs:1006-1010).
+template <uint32_t ROUNDS>
+__global__ void __launch_bounds__(TILE_TB) k_contact_list(uint32_t npairs, const uint32_t* __restrict__ row_count,
+                                                          uint32_t* contact_pairs, uint32_t* scalars,
+                                                          const uint32_t* __restrict__ simulate,
+                                                          const uint32_t* __restrict__ prev_simulate, uint32_t worlds,
+                                                          TileScan ts) {
+    const uint32_t tile = tile_take(ts), base = tile * (TILE_TB * ROUNDS);
+    bool flag[ROUNDS];
+    uint32_t rank[ROUNDS];
+#pragma unroll
+    for (uint32_t r = 0; r < ROUNDS; ++r) {
+        const uint32_t p = base + r * TILE_TB + threadIdx.x;
+        flag[r] = p < npairs && row_count[p] > 0;
+    }
+    const uint32_t total = tile_ranks(flag, rank);
+    const uint32_t at = tile_prefix(ts, tile, 0u, total);
+#pragma unroll
+    for (uint32_t r = 0; r < ROUNDS; ++r)
+        if (flag[r]) contact_pairs[at + rank[r]] = base + r * TILE_TB + threadIdx.x;
+    if (base + TILE_TB * ROUNDS >= npairs && threadIdx.x == 0) scalars[2] = at + total;
+    if (tile == 0u && worlds) {
+        bool all = true;
+#pragma unroll 4
+        for (uint32_t w = threadIdx.x; w < worlds; w += TILE_TB)
+            all &= (simulate[w] != 0u) & (prev_simulate[w] != 0u);  // (no short cut: the loads overlap)
+        if (__syncthreads_and(all ? 1 : 0) && threadIdx.x == 0) scalars[12] = 1u;
+    }
+}
+
+// Tiles of 4,096 pairs from 256k pairs on: the look-back's rounds count there (918k pairs: 13.7 us
+// with tiles of 1,024), with fewer pairs the blocks.
+void launch_contact_list(uint32_t npairs, PairData& pd, const StepParams& sp, uint32_t* status, cudaStream_t s) {
+    auto go = [&](auto kernel, uint32_t tiles) {
+        kernel<<<tiles, TILE_TB, 0, s>>>(npairs, pd.row_count.p, pd.contact_pairs.p, pd.scalars.p, sp.simulate,
+                                         sp.prev_simulate, sp.worlds, pd.list_scan.begin(tiles, status, s));
+    };
+    if (npairs > (1u << 18)) go(k_contact_list<16>, tile_count<16>(npairs));
+    else go(k_contact_list<4>, tile_count<4>(npairs));
 }
 
 struct ColourArgs {
@@ -80,6 +116,8 @@ struct ColourArgs {
     uint32_t seed;                // 1: start from last step's colours
     unsigned int* bar;  // [0] barrier counter, [5] colour max, [6] [7] uncoloured-list lengths
     uint32_t* status;
+    uint32_t* zero;     // nzero words to clear for the kernels after this one
+    uint32_t nzero;
 };
 
 __device__ __forceinline__ unsigned long long* colour_word(unsigned long long* m, uint32_t x, uint32_t c) {
@@ -186,6 +224,7 @@ __global__ void k_colour(ColourArgs a, JpList wl) {
     unsigned int nbar = 0;
     __shared__ unsigned int s_cmax;
     if (threadIdx.x == 0) s_cmax = 0u;
+    for (uint32_t k = tid; k < a.nzero; k += stride) a.zero[k] = 0u;
     for (uint32_t k = tid; k < K; k += stride) {
         a.colour[k] = NO_COLOUR;
         uint64_t key = a.pairs[a.contact_pairs[k]];
@@ -1860,32 +1899,114 @@ __global__ void __launch_bounds__(MAXT) k_world_solve(WorldSolveArgs A) {
 }
 
 // ---------------------------------------------------------------- cache update
-// step.rs:982-1005: the solved normal impulse goes back to its manifold point.
-__global__ void k_writeback(uint32_t npairs, const uint32_t* __restrict__ row_count, const float4* __restrict__ rows,
-                            float4* entries, uint32_t* valid_flags) {
-    uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= npairs) return;
-    float4* e = entries + size_t(p) * ENTRY_F4;
-    uint32_t n = row_count[p];
-    for (uint32_t k = 0; k < n; ++k) {
-        float imp = rows[(size_t(p) * 4 + k) * ROW_F4 + 3].x;
-        float4 y = e[5 + 3 * k];
-        y.w = imp;
-        e[5 + 3 * k] = y;
-    }
-    valid_flags[p] = (__float_as_uint(e[2].w) & META_VALID) ? 1u : 0u;
-}
+// step.rs:982-1010. Tiles [0, ta): the solved normal impulse goes back to its manifold point, and the
+// surviving manifolds of the current pairs go, in pair order, to the new cache. Tiles [ta, ..): the
+// old manifolds that no pair took over and whose world does not prune (prune = simulate &&
+// prev_simulate). When every world prunes there are none of these, the new cache's positions are
+// the current manifolds' ranks, and their entries are copied here and now; otherwise the two lists go to
+// k_merge.
+// What bounds it: the 256-byte manifolds' traffic and, on small worlds, its own latency. One launch
+// for what took nine (write-back, two flag passes and two selections): 1,000-box stack 8.5 us for 20,
+// 131,072-body pile 100 us for 123 (write-back 43, merge 50, the rest the selections).
+struct CacheArgs {
+    uint32_t npairs, nold, ta;
+    const uint32_t* row_count;
+    const float4* rows;
+    float4* entries;
+    const uint64_t* pairs;
+    const uint32_t* owned;
+    const uint64_t* old_keys;
+    const uint32_t *world_of, *simulate, *prev_simulate;
+    uint32_t *sel_a, *sel_b, *scalars;  // scalars[8], [9]: the lists' lengths; [12]: every world prunes
+    uint64_t* out_keys;
+    float4* out_entries;
+    uint32_t* out_count;
+    uint32_t* rec_merge_pos;
+};
 
-// step.rs:1006-1010: with prune = simulate && prev_simulate (of the manifold's world), manifolds
-// whose pair vanished die; otherwise the unowned old manifolds survive.
-__global__ void k_flag_unowned(uint32_t nold, const uint32_t* __restrict__ owned, const uint64_t* __restrict__ old_keys,
-                               const uint32_t* __restrict__ world_of, const uint32_t* __restrict__ simulate,
-                               const uint32_t* __restrict__ prev_simulate, uint32_t* flags) {
-    uint32_t o = blockIdx.x * blockDim.x + threadIdx.x;
-    if (o >= nold) return;
-    uint32_t w = world_of ? world_of[key_lo(old_keys[o])] : 0u;
-    bool prune = (simulate[w] != 0) && (prev_simulate[w] != 0);
-    flags[o] = (!prune && !owned[o]) ? 1u : 0u;
+template <uint32_t ROUNDS>
+__global__ void __launch_bounds__(TILE_TB) k_cache_lists(CacheArgs a, TileScan ts) {
+    constexpr uint32_t ITEMS = TILE_TB * ROUNDS;
+    __shared__ uint32_t s_pair[ITEMS];  // the tile's surviving pairs | rows << 29
+    const uint32_t tile = tile_take(ts);
+    const bool prune_all = a.scalars[12] != 0u;
+    bool flag[ROUNDS];
+    uint32_t rank[ROUNDS];
+    if (tile >= a.ta) {
+        if (prune_all) return;
+        const uint32_t base = (tile - a.ta) * ITEMS;
+#pragma unroll
+        for (uint32_t r = 0; r < ROUNDS; ++r) {
+            const uint32_t o = base + r * TILE_TB + threadIdx.x;
+            flag[r] = false;
+            if (o < a.nold) {
+                const uint32_t w = a.world_of ? a.world_of[key_lo(a.old_keys[o])] : 0u;
+                flag[r] = !(a.simulate[w] != 0u && a.prev_simulate[w] != 0u) && !a.owned[o];
+            }
+        }
+        const uint32_t total = tile_ranks(flag, rank);
+        const uint32_t at = tile_prefix(ts, tile, a.ta, total);
+#pragma unroll
+        for (uint32_t r = 0; r < ROUNDS; ++r)
+            if (flag[r]) a.sel_b[at + rank[r]] = base + r * TILE_TB + threadIdx.x;
+        if (base + ITEMS >= a.nold && threadIdx.x == 0) a.scalars[9] = at + total;
+        return;
+    }
+    const uint32_t base = tile * ITEMS;
+    uint32_t rows[ROUNDS];
+#pragma unroll
+    for (uint32_t r = 0; r < ROUNDS; ++r) {
+        const uint32_t p = base + r * TILE_TB + threadIdx.x;
+        flag[r] = p < a.npairs && (__float_as_uint(a.entries[size_t(p) * ENTRY_F4 + 2].w) & META_VALID) != 0u;
+        rows[r] = p < a.npairs ? a.row_count[p] : 0u;
+    }
+    const uint32_t total = tile_ranks(flag, rank);
+#pragma unroll
+    for (uint32_t r = 0; r < ROUNDS; ++r)
+        if (flag[r]) s_pair[rank[r]] = (base + r * TILE_TB + threadIdx.x) | (rows[r] << 29);
+    const uint32_t at = tile_prefix(ts, tile, 0u, total);  // (its last step is a block barrier: s_pair is ready)
+    if (base + ITEMS >= a.npairs && threadIdx.x == 0) {
+        a.scalars[8] = at + total;
+        if (prune_all) *a.out_count = at + total;
+    }
+    // 16 threads a manifold, one float4 each: point k's impulse is word w of entry 5 + 3 k.
+    const uint32_t q = threadIdx.x & 15u, k = (q - 5u) / 3u;
+    const bool holds = q >= 5u && (q - 5u) % 3u == 0u;
+    if (prune_all) {
+        constexpr uint32_t BATCH = 4;  // manifolds in flight a thread
+        for (uint32_t t0 = threadIdx.x >> 4; t0 < total; t0 += BATCH * (TILE_TB / 16u)) {
+            float4 e[BATCH];
+            float imp[BATCH];
+#pragma unroll
+            for (uint32_t u = 0; u < BATCH; ++u) {
+                const uint32_t t = t0 + u * (TILE_TB / 16u);
+                if (t >= total) continue;
+                const uint32_t x = s_pair[t], p = x & 0x1fffffffu;
+                e[u] = __ldcs(&a.entries[size_t(p) * ENTRY_F4 + q]);
+                imp[u] = e[u].w;
+                if (holds && k < x >> 29) imp[u] = a.rows[(size_t(p) * 4 + k) * ROW_F4 + 3].x;
+            }
+#pragma unroll
+            for (uint32_t u = 0; u < BATCH; ++u) {
+                const uint32_t t = t0 + u * (TILE_TB / 16u);
+                if (t >= total) continue;
+                e[u].w = imp[u];
+                a.out_entries[size_t(at + t) * ENTRY_F4 + q] = e[u];
+                if (q == 0u) {
+                    const uint32_t p = s_pair[t] & 0x1fffffffu;
+                    a.out_keys[at + t] = a.pairs[p];
+                    if (a.rec_merge_pos) a.rec_merge_pos[p] = at + t;
+                }
+            }
+        }
+        return;
+    }
+    for (uint32_t t = threadIdx.x >> 4; t < total; t += TILE_TB / 16u) {
+        const uint32_t p = s_pair[t] & 0x1fffffffu;
+        if (holds && k < s_pair[t] >> 29)
+            a.entries[size_t(p) * ENTRY_F4 + q].w = a.rows[(size_t(p) * 4 + k) * ROW_F4 + 3].x;
+        if (q == 0u) a.sel_a[at + t] = p;
+    }
 }
 
 __device__ __forceinline__ uint32_t lower_bound_pairs(const uint64_t* __restrict__ pairs, const uint32_t* __restrict__ sel,
@@ -1915,7 +2036,9 @@ __global__ void k_merge(const uint64_t* __restrict__ pairs, const float4* __rest
                         const uint32_t* __restrict__ sel_a, const uint32_t* __restrict__ na_ptr,
                         const uint64_t* __restrict__ old_keys, const float4* __restrict__ old_entries,
                         const uint32_t* __restrict__ sel_b, const uint32_t* __restrict__ nb_ptr, uint64_t* out_keys,
-                        float4* out_entries, uint32_t* out_count, uint32_t* rec_merge_pos) {
+                        float4* out_entries, uint32_t* out_count, uint32_t* rec_merge_pos,
+                        const uint32_t* __restrict__ done) {
+    if (*done) return;  // every world pruned: k_cache_lists has filled the cache
     uint32_t na = *na_ptr, nb = *nb_ptr;
     uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t == 0) *out_count = na + nb;
@@ -2033,8 +2156,6 @@ void run_solver(const WorldView& w, const uint64_t* pairs, uint32_t npairs, Pair
     const bool with_joints = joints && joints->n && joints->ncol;
     g_last_solver_kind = 0;
     if (npairs == 0) {
-        check_cuda(cudaMemsetAsync(pd.scalars.p + 2, 0, 4 * sizeof(uint32_t), s), "memset");
-        check_cuda(cudaMemsetAsync(pd.scalars.p + 10, 0, 2 * sizeof(uint32_t), s), "memset");
         mark(5);
         if (with_joints) {
             launch_solve(w, pd, sp, status_dev, s, joints);
@@ -2048,18 +2169,25 @@ void run_solver(const WorldView& w, const uint64_t* pairs, uint32_t npairs, Pair
     const int TB = 256;
     if (npairs >= (1u << 29)) throw CudaError{cudaErrorInvalidValue, "more than 2^29 pairs for the solver's slot records"};
     // Contact pairs (ascending pair order).
-    k_flag_contact_pairs<<<(npairs + TB - 1) / TB, TB, 0, s>>>(npairs, pd.row_count.p, pd.flags.p);
-    size_t bytes = 0;
-    cub::CountingInputIterator<uint32_t> it(0);
-    check_cuda(cub::DeviceSelect::Flagged(nullptr, bytes, it, pd.flags.p, pd.contact_pairs.p, pd.scalars.p + 2,
-                                          int(npairs), s), "select size");
-    pd.cub_tmp.reserve(bytes);
-    check_cuda(cub::DeviceSelect::Flagged(pd.cub_tmp.p, bytes, it, pd.flags.p, pd.contact_pairs.p, pd.scalars.p + 2,
-                                          int(npairs), s), "select");
+    launch_contact_list(npairs, pd, sp, status_dev, s);
+    // Chunks: each body's chunk; the (colour, chunk) counts and the bodies' colour masks come with
+    // the colour histograms.
+    uint32_t P = 0;
+    uint32_t *vhist = nullptr, *shist = nullptr;
+    if (chunked) {
+        P = uint32_t(chunk_grid());
+        const uint32_t n = w.nbodies;
+        pd.chunk_of.reserve(std::max<uint32_t>(n, 1));
+        pd.chunk_hist.reserve(size_t(MAX_COLOURS) * P * 5);
+        pd.chunk_off.reserve(2 * size_t(MAX_COLOURS) * (P + 1) + size_t(MAX_COLOURS) * P * 4);
+        pd.flow_vel.reserve(4 * size_t(std::max<uint32_t>(n, 1)));
+        vhist = pd.chunk_hist.p;
+        shist = pd.chunk_hist.p + size_t(MAX_COLOURS) * P * 4;
+    }
     // Colouring (cooperative launch).
-    check_cuda(cudaMemsetAsync(pd.barrier.p, 0, 16 * sizeof(unsigned int), s), "memset barrier");
     ColourArgs ca{pd.scalars.p + 2, pd.contact_pairs.p, pairs, w.b.iw, pd.colour.p, pd.body_prio.p, pd.body_mask.p,
-                  pd.body_dup.p, chunked ? pd.body_used.p : nullptr, pd.entries.p, seed_colours ? 1u : 0u, pd.barrier.p, status_dev};
+                  pd.body_dup.p, chunked ? pd.body_used.p : nullptr, pd.entries.p, seed_colours ? 1u : 0u, pd.barrier.p,
+                  status_dev, vhist, P * MAX_COLOURS * 5u};
     // Two blocks per SM: enough threads for a pile's groups, and the rounds' grid barriers
     // are cheaper than with every block the SM could hold.
     static int colour_grid = 0;
@@ -2070,28 +2198,12 @@ void run_solver(const WorldView& w, const uint64_t* pairs, uint32_t npairs, Pair
     check_cuda(cudaLaunchCooperativeKernel((const void*)k_colour, dim3(colour_grid), dim3(TB), cargs, 0, s),
                "colour launch");
     // Batches.
-    check_cuda(cudaMemsetAsync(pd.colour_count.p, 0, (MAX_COLOURS + 3) * sizeof(uint32_t), s), "memset");
-    check_cuda(cudaMemsetAsync(pd.split_count.p, 0, (MAX_COLOURS + 3) * sizeof(uint32_t), s), "memset");
-    pd.colour_sub.reserve(2 * 4 * MAX_COLOURS);
     uint32_t* sub_hist = pd.colour_sub.p;
     uint32_t* sub_cursor = pd.colour_sub.p + 4 * MAX_COLOURS;
-    check_cuda(cudaMemsetAsync(sub_hist, 0, 4 * MAX_COLOURS * sizeof(uint32_t), s), "memset");
     uint32_t g = std::min<uint32_t>((npairs + TB - 1) / TB, 148u * 8u);
-    // Chunks: each body's chunk; the (colour, chunk) counts and the touch sets come with the
-    // colour histograms.
-    uint32_t P = 0;
-    uint32_t *vhist = nullptr, *shist = nullptr;
     if (chunked) {
-        P = uint32_t(chunk_grid());
         const uint32_t n = w.nbodies;
         const bool tree = morton_leaf && tree_m;
-        pd.chunk_of.reserve(std::max<uint32_t>(n, 1));
-        pd.chunk_hist.reserve(size_t(MAX_COLOURS) * P * 5);
-        pd.chunk_off.reserve(2 * size_t(MAX_COLOURS) * (P + 1) + size_t(MAX_COLOURS) * P * 4);
-        pd.flow_vel.reserve(4 * size_t(std::max<uint32_t>(n, 1)));
-        vhist = pd.chunk_hist.p;
-        shist = pd.chunk_hist.p + size_t(MAX_COLOURS) * P * 4;
-        check_cuda(cudaMemsetAsync(pd.chunk_hist.p, 0, size_t(MAX_COLOURS) * P * 5 * sizeof(uint32_t), s), "memset");
         k_chunk_of<<<std::min<uint32_t>((4 * n + TB - 1) / TB, 148u * 8u), TB, 0, s>>>(
             n, P, tree ? morton_leaf : nullptr, tree_m, pd.chunk_of.p, pd.flow_vel.p);
     }
@@ -2195,10 +2307,6 @@ void run_world_solver(const WorldView& w, const uint64_t* pairs, uint32_t npairs
                       const uint32_t* world_off, uint32_t nworlds, const WorldPlan& plan, uint32_t* wcol,
                       const JointsDev* joints, bool seed_colours) {
     const bool with_joints = joints && joints->n && joints->ncol;
-    check_cuda(cudaMemsetAsync(pd.scalars.p + 2, 0, 4 * sizeof(uint32_t), s), "memset");
-    check_cuda(cudaMemsetAsync(pd.scalars.p + 10, 0, 2 * sizeof(uint32_t), s), "memset");
-    check_cuda(cudaMemsetAsync(pd.colour_count.p, 0, (MAX_COLOURS + 3) * sizeof(uint32_t), s), "memset");
-    check_cuda(cudaMemsetAsync(pd.split_count.p, 0, (MAX_COLOURS + 3) * sizeof(uint32_t), s), "memset");
     if (nworlds == 0 || (npairs == 0 && !with_joints)) {
         mark(5);
         mark(6);
@@ -2206,17 +2314,7 @@ void run_world_solver(const WorldView& w, const uint64_t* pairs, uint32_t npairs
     }
     const int TB = 256;
     if (npairs >= (1u << 29)) throw CudaError{cudaErrorInvalidValue, "more than 2^29 pairs for the solver's slot records"};
-    if (npairs)
-        k_flag_contact_pairs<<<(npairs + TB - 1) / TB, TB, 0, s>>>(npairs, pd.row_count.p, pd.flags.p);
-    size_t bytes = 0;
-    cub::CountingInputIterator<uint32_t> it(0);
-    if (npairs) {
-        check_cuda(cub::DeviceSelect::Flagged(nullptr, bytes, it, pd.flags.p, pd.contact_pairs.p, pd.scalars.p + 2,
-                                              int(npairs), s), "select size");
-        pd.cub_tmp.reserve(bytes);
-        check_cuda(cub::DeviceSelect::Flagged(pd.cub_tmp.p, bytes, it, pd.flags.p, pd.contact_pairs.p,
-                                              pd.scalars.p + 2, int(npairs), s), "select");
-    }
+    if (npairs) launch_contact_list(npairs, pd, sp, status_dev, s);
     mark(5);
     // A plain world's contacts go to many blocks; with joints, and a world of a few bodies, to one
     // block with its velocities in shared memory.
@@ -2272,43 +2370,30 @@ void run_world_solver(const WorldView& w, const uint64_t* pairs, uint32_t npairs
 
 void run_cache_update(const uint64_t* pairs, uint32_t npairs, const Manifolds& old_cache, PairData& pd,
                       Manifolds& next, const uint32_t* world_of, const uint32_t* simulate_flag,
-                      const uint32_t* prev_simulate, cudaStream_t s) {
-    const int TB = 256;
-    uint32_t nold_cap = old_cache.count_host;
-    // A: surviving manifolds of the current pairs.
-    if (npairs) k_writeback<<<(npairs + TB - 1) / TB, TB, 0, s>>>(npairs, pd.row_count.p, pd.rows.p, pd.entries.p,
-                                                                  pd.flags.p);
-    cub::CountingInputIterator<uint32_t> it(0);
-    size_t bytes_a = 0, bytes_b = 0;
-    uint32_t* na_dev = pd.scalars.p + 8;
-    uint32_t* nb_dev = pd.scalars.p + 9;
-    check_cuda(cudaMemsetAsync(na_dev, 0, 2 * sizeof(uint32_t), s), "memset");
-    if (npairs)
-        check_cuda(cub::DeviceSelect::Flagged(nullptr, bytes_a, it, pd.flags.p, pd.sel_a.p, na_dev, int(npairs), s), "sel");
-    if (nold_cap)
-        check_cuda(cub::DeviceSelect::Flagged(nullptr, bytes_b, it, pd.flags.p, pd.sel_b.p, nb_dev, int(nold_cap), s), "sel");
-    pd.cub_tmp.reserve(std::max(bytes_a, bytes_b));
-    if (npairs)
-        check_cuda(cub::DeviceSelect::Flagged(pd.cub_tmp.p, bytes_a, it, pd.flags.p, pd.sel_a.p, na_dev, int(npairs), s),
-                   "sel");
-    // B: unowned old manifolds (only kept when this step does not prune).
-    if (nold_cap) {
-        // nold_cap is the exact old count: the world syncs on it before the step.
-        k_flag_unowned<<<(nold_cap + TB - 1) / TB, TB, 0, s>>>(nold_cap, pd.old_owned.p, old_cache.keys.p, world_of,
-                                                                simulate_flag, prev_simulate, pd.flags.p);
-        check_cuda(cub::DeviceSelect::Flagged(pd.cub_tmp.p, bytes_b, it, pd.flags.p, pd.sel_b.p, nb_dev, int(nold_cap), s),
-                   "sel");
-    }
-    size_t cap = size_t(npairs) + nold_cap + 1;
+                      const uint32_t* prev_simulate, uint32_t* status_dev, cudaStream_t s) {
+    // The exact old count: the world syncs on it before the step.
+    const uint32_t nold = old_cache.count_host;
+    const size_t cap = size_t(npairs) + nold + 1;
     next.keys.reserve(cap);
     next.entries.reserve(cap * ENTRY_F4);
-    uint32_t total = npairs + nold_cap;
-    if (total)
-        k_merge<<<(total + TB - 1) / TB, TB, 0, s>>>(pairs, pd.entries.p, pd.sel_a.p, na_dev, old_cache.keys.p,
-                                                      old_cache.entries.p, pd.sel_b.p, nb_dev, next.keys.p,
-                                                      next.entries.p, next.count_dev, pd.rec.merge_pos);
-    else
+    const uint32_t total = npairs + nold;
+    if (!total) {
         check_cuda(cudaMemsetAsync(next.count_dev, 0, sizeof(uint32_t), s), "memset");
+        return;
+    }
+    // Small tiles where blocks are few, so that many copy; large ones where the look-back counts.
+    const bool large = npairs > (1u << 17);
+    const uint32_t ta = std::max(large ? tile_count<4>(npairs) : tile_count<1>(npairs), 1u);
+    const uint32_t tiles = ta + (large ? tile_count<4>(nold) : tile_count<1>(nold));
+    const CacheArgs a{npairs, nold, ta, pd.row_count.p, pd.rows.p, pd.entries.p, pairs, pd.old_owned.p, old_cache.keys.p,
+                      world_of, simulate_flag, prev_simulate, pd.sel_a.p, pd.sel_b.p, pd.scalars.p,
+                      next.keys.p, next.entries.p, next.count_dev, pd.rec.merge_pos};
+    if (large) k_cache_lists<4><<<tiles, TILE_TB, 0, s>>>(a, pd.cache_scan.begin(tiles, status_dev, s));
+    else k_cache_lists<1><<<tiles, TILE_TB, 0, s>>>(a, pd.cache_scan.begin(tiles, status_dev, s));
+    k_merge<<<(total + TILE_TB - 1) / TILE_TB, TILE_TB, 0, s>>>(
+        pairs, pd.entries.p, pd.sel_a.p, pd.scalars.p + 8, old_cache.keys.p, old_cache.entries.p, pd.sel_b.p,
+        pd.scalars.p + 9, next.keys.p, next.entries.p, next.count_dev, pd.rec.merge_pos, pd.scalars.p + 12);
+    pd.old_owned.reserve(cap);  // the next step clears and fills a mark for each of its old manifolds
 }
 
 }  // namespace bgpu

@@ -91,13 +91,6 @@ void local_inertia(const Shape& s, float mass, float out[3]) {
     }
 }
 
-struct HostStats {  // pinned, written by async copies at the end of a step
-    uint32_t scalars[16];
-    uint32_t status;
-    uint32_t cache_count;
-    uint32_t simulate;
-};
-
 }  // namespace
 
 // One forward step recorded for the adjoint (the reverse solve's inputs).
@@ -218,7 +211,8 @@ struct World {
         cache[1].init();
         check_cuda(cudaMemsetAsync(cache[0].count_dev, 0, sizeof(uint32_t), stream), "memset");
         check_cuda(cudaMemsetAsync(cache[1].count_dev, 0, sizeof(uint32_t), stream), "memset");
-        pd.scalars.reserve(16);
+        pd.reserve_counters();
+        pd.old_owned.reserve(1);
         for (auto& set : ev)
             for (auto& e : set) check_cuda(cudaEventCreate(&e), "event");
     }
@@ -236,7 +230,8 @@ struct World {
                        rec_step ? rec_step->flags.p : nullptr};
     }
     bool has_mesh = false;  // some shape is a triangle mesh
-    WorldView view() { return WorldView{body_dev(), shapes_d.p, hull_d.p, n, has_mesh}; }
+    bool has_convex = false;  // some shape is a capsule or hull
+    WorldView view() { return WorldView{body_dev(), shapes_d.p, hull_d.p, n, has_mesh, has_convex}; }
 
     void sync_shapes() {
         if (!shapes_dirty) return;
@@ -307,6 +302,7 @@ struct World {
                 throw InvalidArg{"unknown shape type"};
         }
         s.cbt = contact_breaking_threshold(s.lmin, s.lmax);
+        has_convex = has_convex || type == SHAPE_CAPSULE || type == SHAPE_HULL;
         shapes_h.push_back(s);
         shapes_dirty = true;
         return uint32_t(shapes_h.size() - 1);
@@ -900,6 +896,9 @@ struct World {
         sp.info = info;
         sp.suppressed = nsuppressed ? suppressed_d.p : nullptr;
         sp.nsuppressed = nsuppressed;
+        sp.worlds = num_worlds();
+        sp.simulate = world_sim.p;
+        sp.prev_simulate = world_sim.p + sp.worlds;
         JointsDev jd = joints_dev();
         if (rec_step) {
             rec_step->flags.reserve(std::max<uint32_t>(n, 1));
@@ -912,11 +911,15 @@ struct World {
         uint32_t* simulate = world_sim.p;
         uint32_t* prev_simulate = world_sim.p + nw;
         const uint32_t* world_of = batch ? world_of_d.p : nullptr;
-        check_cuda(cudaMemsetAsync(flags.p, 0, sizeof(uint32_t), stream), "memset flags");
-        check_cuda(cudaMemsetAsync(simulate, 0, nw * sizeof(uint32_t), stream), "memset flags");
+        StepReset reset;
+        reset.add(status, 1);
+        reset.add(simulate, nw);
+        pd.add_counters(reset);
+        reset.owned = pd.old_owned.p;
+        reset.owned_n = cache[cur].count_dev;
         mark(0);
         // 1-3: velocities, predicted poses, AABBs (fused).
-        launch_integrate_velocities(b, shapes_d.p, hull_d.p, n, dt, stream);
+        launch_integrate_velocities(b, shapes_d.p, hull_d.p, n, dt, reset, stream);
         mark(1);
         // 4: broad phase (syncs once to size the pair arrays; the previous step's
         //    manifold count and timing events are read at the same point).
@@ -934,8 +937,6 @@ struct World {
         mark(3);
         // 5: pair pass
         pd.reserve(std::max<uint32_t>(npairs, 1), n, old_cache.count_host);
-        if (old_cache.count_host)
-            check_cuda(cudaMemsetAsync(pd.old_owned.p, 0, old_cache.count_host * sizeof(uint32_t), stream), "memset");
         run_pair_pass(wv, pairs.p, npairs, old_cache, pd, sp, simulate, status, stream);
         // 5a: joint rows from the current poses (step.rs:928-949)
         launch_joint_rows(b, jd, sp.inv_dt, info.erp, stream);
@@ -953,9 +954,7 @@ struct World {
                        batch ? 0u : uint32_t(bp.tree_m));
         ++step_count;
         // 6b: impulse writeback + prune
-        run_cache_update(pairs.p, npairs, old_cache, pd, next, world_of, simulate, prev_simulate, stream);
-        check_cuda(cudaMemcpyAsync(prev_simulate, simulate, nw * sizeof(uint32_t), cudaMemcpyDeviceToDevice, stream),
-                   "flag");
+        run_cache_update(pairs.p, npairs, old_cache, pd, next, world_of, simulate, prev_simulate, status, stream);
         mark(7);
         // 7a: CCD clamp fractions, from the solved velocities and the pre-integration poses
         launch_ccd_sweep(b, shapes_d.p, hull_d.p, ccd_ids_d.p, ccd_par_d.p, nccd, n, batch ? world_off_d.p : nullptr,
@@ -963,7 +962,8 @@ struct World {
                          batch ? nullptr : bp.node_rec.p, bp.leaf_body.p, batch ? 0 : bp.tree_m, bp.unbounded.p,
                          batch ? 0u : bp.nunb, ccd_scratch, stream);
         // 6c + 7 + 8: deactivation, pose integration with the split push, force clear.
-        launch_integrate_positions(b, n, dt, info.split_impulse_turn_erp, stream);
+        launch_integrate_positions(b, n, dt, info.split_impulse_turn_erp,
+                                   StepEnd{hs, pd.scalars.p, status, next.count_dev, simulate, prev_simulate, nw}, stream);
         launch_ccd_apply(b, ccd_ids_d.p, ccd_clamp_d.p, nccd, dt, stream);
         mark(8);
         if (timing) {
@@ -972,10 +972,6 @@ struct World {
         }
         check_cuda(cudaGetLastError(), "step launch");
         cur ^= 1;
-        check_cuda(cudaMemcpyAsync(hs->scalars, pd.scalars.p, 16 * sizeof(uint32_t), cudaMemcpyDeviceToHost, stream), "d2h");
-        check_cuda(cudaMemcpyAsync(&hs->status, status, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream), "d2h");
-        check_cuda(cudaMemcpyAsync(&hs->cache_count, next.count_dev, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream),
-                   "d2h");
         stats_pending = true;
         if (rec_step) finish_record();
     }
@@ -1124,6 +1120,7 @@ static void restore_snapshot(World& W, const Snapshot& S) {
     d2d(c.keys.p, S.keys.p, S.count * sizeof(uint64_t));
     d2d(c.entries.p, S.entries.p, size_t(S.count) * ENTRY_F4 * sizeof(float4));
     check_cuda(cudaMemcpyAsync(c.count_dev, &S.count, sizeof(uint32_t), cudaMemcpyHostToDevice, W.stream), "h2d");
+    W.pd.old_owned.reserve(S.count + 1);  // the next step clears as many marks as the cache has entries
     d2d(W.world_sim.p, S.sim.p, S.nsim * sizeof(uint32_t));
     check_cuda(cudaStreamSynchronize(W.stream), "sync");
     c.count_host = S.count;
@@ -2523,6 +2520,7 @@ bgpu_status bgpu_solve_contacts(bgpu_world* w, uint32_t n, const float* contacts
         }
         uint32_t G = uint32_t(keys.size());
         W.pd.reserve(std::max<uint32_t>(G, 1), W.n, 1);
+        W.pd.clear_counters(s);
         bgpu::DevBuf<uint32_t> d_first, d_cnt;
         bgpu::DevBuf<float> d_c;
         d_first.reserve(G + 1);
