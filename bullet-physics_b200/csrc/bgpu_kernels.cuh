@@ -109,6 +109,13 @@ struct StepReset {
         n[count++] = uint32_t(words);
     }
 };
+// What a step's first kernel does for the broad phase and the islands on its way over the bodies.
+// Accumulators come in pairs: the step uses one and resets the other for the next step.
+struct StepBegin {
+    int *bounds, *next_bounds;     // 6 ordered ints: min / max of the bounded proxies' centres (null: not wanted)
+    uint32_t *need, *next_need;    // Islands::need
+    uint32_t *parent, *awake;      // Islands
+};
 // What a step's last kernel hands to the host (pinned, written by the device).
 struct HostStats {
     uint32_t scalars[16];
@@ -126,6 +133,13 @@ struct StepEnd {
 // ---------------------------------------------------------------- device helpers shared by the solver and its adjoint
 constexpr unsigned int BARRIER_SPIN_LIMIT = 1u << 26;
 constexpr unsigned long long BARRIER_TIMEOUT_NS = 2000000000ull;  // 2 s: phases take microseconds
+
+// A float as an int of the same order, for integer minima and maxima.
+__device__ __forceinline__ int float_to_ordered(float f) {
+    int i = __float_as_int(f);
+    return i >= 0 ? i : i ^ 0x7fffffff;
+}
+__device__ __forceinline__ float ordered_to_float(int i) { return __int_as_float(i >= 0 ? i : i ^ 0x7fffffff); }
 
 __device__ __forceinline__ unsigned long long globaltimer_ns() {
     unsigned long long t;
@@ -216,7 +230,7 @@ constexpr uint32_t PLANE_STRIDE = 4 * 32;
 // ---------------------------------------------------------------- body kernels (k_body.cu)
 // The first kernel of a step (it also clears the step's counters) and, CCD clamps apart, the last.
 void launch_integrate_velocities(const BodyDev& b, const Shape* shapes, const float4* hull, uint32_t n, float dt,
-                                 const StepReset& reset, cudaStream_t s);
+                                 const StepReset& reset, const StepBegin& begin, cudaStream_t s);
 void launch_initial_aabbs(const BodyDev& b, const Shape* shapes, const float4* hull, uint32_t first, uint32_t n,
                           cudaStream_t s);
 void launch_integrate_positions(const BodyDev& b, uint32_t n, float dt, float turn_erp, const StepEnd& end,
@@ -245,25 +259,37 @@ void launch_pack_poses(uint32_t n, const float4* pos, const float4* quat, float*
 // against every proxy by an ordered compaction.
 struct Broadphase {
     DevBuf<uint64_t> keys, keys_alt;
-    DevBuf<uint32_t> leaf_body, parent, left, right, counts, offsets, refit_flag, flags, scan_out, unbounded;
+    DevBuf<uint32_t> leaf_body, parent, left, right, counts, offsets, refit_flag, is_unb, unbounded;
     DevBuf<uint32_t> stash, overflow;  // partners of proxies with few of them; proxies with many
+    DevBuf<uint32_t> unb_tiles;        // per unbounded proxy and tile of proxies: partners before the tile
     DevBuf<float4> node_min, node_max;
     DevBuf<uint32_t> node_maxid;       // largest body index below each node
     DevBuf<float4> node_rec;           // per internal node: both children's boxes and references
+    DevBuf<uint32_t> masks;            // all-pairs pass: bit j of row i
     DevBuf<unsigned char> cub_tmp;
-    DevBuf<int> bounds;          // 6 ordered ints: scene min/max of leaf centres
-    DevBuf<uint32_t> scalars;    // [0] total pairs, [1] proxies with more partners than the stash holds
-    uint32_t* host_scalars = nullptr;  // pinned
+    DevBuf<int> bounds;          // 2 x 6 ordered ints: scene min/max of leaf centres
+    DevBuf<uint32_t> scalars;    // [1] proxies (worlds) with more partners than the stash holds
+    TileScanBuf scan;
+    uint32_t* host_scalars = nullptr;  // pinned, written by the device: [0] total pairs, [1] proxies (worlds)
+                                       // with more partners than the stash holds
     int tree_m = 0;                    // bounded proxies in the last run's tree (0: no tree)
     uint32_t nunb = 0;                 // proxies of the last run kept out of the tree (device list `unbounded`)
+    uint32_t unb_n = 0;                // proxies and
+    std::vector<uint32_t> unb_listed;  // unbounded list that is_unb and `unbounded` hold
     Broadphase();
     ~Broadphase();
-    // Returns the pair count; pairs are written to `out` (grown as needed).
+    // Up to this many proxies every pair is tested (no tree): n^2 / 2 tests cost less than the tree's
+    // launches and climbs. Broad phase of settled piles, all pairs / tree: 1,024 bodies 57 / 118 us,
+    // 4,096 74 / 144, 8,000 97 / 197, 12,500 161 / 201, 16,250 218 / 208.
+    static constexpr uint32_t ALL_PAIRS_MAX = 12288;
+    // Returns the pair count; pairs are written to `out` (grown as needed). all_pairs: test every
+    // pair (n <= ALL_PAIRS_MAX). centres: the bounded proxies' centre bounds when a kernel before
+    // has them, else null.
     uint64_t run(const float4* aabb_min, const float4* aabb_max, uint32_t n, const std::vector<uint32_t>& unbounded_host,
-                 DevBuf<uint64_t>& out, uint32_t* status_dev, cudaStream_t s);
+                 DevBuf<uint64_t>& out, bool all_pairs, const int* centres, uint32_t* status_dev, cudaStream_t s);
     // Batched worlds: pairs only inside each world [world_off[k], world_off[k + 1]) (device array).
     uint64_t run_worlds(const float4* aabb_min, const float4* aabb_max, uint32_t n, const uint32_t* world_off,
-                        uint32_t n_worlds, DevBuf<uint64_t>& out, cudaStream_t s);
+                        uint32_t n_worlds, DevBuf<uint64_t>& out, uint32_t* status_dev, cudaStream_t s);
 };
 
 // ---------------------------------------------------------------- islands (k_islands.cu)
@@ -375,13 +401,19 @@ __device__ __forceinline__ void solve_joint_slot(const JointsDev& jd, uint32_t t
 }
 
 struct Islands {
-    DevBuf<uint32_t> parent, awake, need;
+    DevBuf<uint32_t> parent, awake, need;  // need: two words, one step's and the next's
+    void reserve(uint32_t n) {
+        parent.reserve(n);
+        awake.reserve(n);
+        need.reserve(2);
+    }
     // simulate_flag[world] is raised when the world has an active body; world_of
     // (per body) is null for a single world. Enabled joints between two dynamic bodies
-    // link their islands (islands.rs:186-196).
+    // link their islands (islands.rs:186-196). parent, awake and need_now come from the step's first
+    // kernel.
     void run(const BodyDev& b, uint32_t n, const uint64_t* pairs, uint32_t npairs, const uint32_t* world_of,
-             uint32_t* simulate_flag, uint32_t* status_dev, cudaStream_t s, const float4* joint_desc = nullptr,
-             uint32_t njoints = 0);
+             const uint32_t* need_now, uint32_t* simulate_flag, uint32_t* status_dev, cudaStream_t s,
+             const float4* joint_desc = nullptr, uint32_t njoints = 0);
 };
 
 // ---------------------------------------------------------------- pair pass + solver (k_pairs.cu, k_solver.cu)

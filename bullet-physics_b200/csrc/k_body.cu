@@ -45,17 +45,15 @@ __device__ __forceinline__ V3 gyroscopic_implicit(V3 inv, Q q, V3 w, float step)
     return rotate(q, ob - delta) - w;
 }
 
-// step.rs:306-363 + body.rs:1113-1126, 1175-1181, shapes/mod.rs:350, util.rs:52-55.
-// Also clears the step's counters (a dozen memsets otherwise, each a launch).
-__global__ void k_integrate_velocities(BodyDev b, const Shape* __restrict__ shapes, const float4* __restrict__ hull,
-                                       uint32_t n, float dt, float aabb_margin, StepReset reset) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    for (int k = 0; k < reset.count; ++k)
-        for (uint32_t t = i; t < reset.n[k]; t += gridDim.x * blockDim.x) reset.w[k][t] = 0u;
-    if (reset.owned)
-        for (uint32_t t = i, m = *reset.owned_n; t < m; t += gridDim.x * blockDim.x) reset.owned[t] = 0u;
-    if (i >= n) return;
+// step.rs:306-363 + body.rs:1113-1126, 1175-1181, shapes/mod.rs:350, util.rs:52-55, for one body; also
+// its island node, and the centre of its box for the broad phase.
+__device__ __forceinline__ void integrate_body(const BodyDev& b, const Shape* __restrict__ shapes,
+                                               const float4* __restrict__ hull, uint32_t i, float dt, float aabb_margin,
+                                               const StepBegin& begin, bool& bounded, bool& need, V3& centre) {
     uint4 info = b.info[i];
+    begin.parent[i] = i;
+    begin.awake[i] = 0u;
+    need = (info.y & (BF_STATIC | BF_KINEMATIC)) == 0u && (info.z == ACT_ISLAND_SLEEPING || info.z == ACT_WANTS_DEACTIVATION);
     float4 p4 = b.pos[i];
     float4 q4v = b.quat[i];
     float4 lv4 = b.linvel[i];
@@ -93,12 +91,60 @@ __global__ void k_integrate_velocities(BodyDev b, const Shape* __restrict__ shap
         mx = mx + splat(aabb_margin);
         b.aabb_min[i] = to4(mn, 0.0f);
         b.aabb_max[i] = to4(mx, 0.0f);
+        centre = (mn + mx) * 0.5f;
+    }
+    if (begin.bounds) {
+        const uint32_t type = shapes[info.x].type;
+        bounded = type != SHAPE_PLANE && type != SHAPE_MESH;
+        if (!active) centre = (from4(b.aabb_min[i]) + from4(b.aabb_max[i])) * 0.5f;  // a sleeper keeps its box
     }
     b.iw[3 * i + 0] = make_float4(iw.c0.x, iw.c0.y, iw.c0.z, iw.c1.x);
     b.iw[3 * i + 1] = make_float4(iw.c1.y, iw.c1.z, iw.c2.x, iw.c2.y);
     b.iw[3 * i + 2] = make_float4(iw.c2.z, ii4.w, 0.0f, 0.0f);
     b.push_lin[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     b.push_ang[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+}
+
+// The step's first kernel: it also clears the counters of the kernels after it (a dozen memsets
+// otherwise, each a launch) and bounds the proxies' centres (two launches and a second read of the boxes).
+__global__ void k_integrate_velocities(BodyDev b, const Shape* __restrict__ shapes, const float4* __restrict__ hull,
+                                       uint32_t n, float dt, float aabb_margin, StepReset reset, StepBegin begin) {
+    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < 3u && begin.next_bounds) begin.next_bounds[i] = 0x7fffffff;
+    else if (i < 6u && begin.next_bounds) begin.next_bounds[i] = int(0x80000000);
+    else if (i == 6u) *begin.next_need = 0u;
+    for (int k = 0; k < reset.count; ++k)
+        for (uint32_t t = i; t < reset.n[k]; t += gridDim.x * blockDim.x) reset.w[k][t] = 0u;
+    if (reset.owned)
+        for (uint32_t t = i, m = *reset.owned_n; t < m; t += gridDim.x * blockDim.x) reset.owned[t] = 0u;
+    __shared__ int s_bounds[6];
+    if (begin.bounds) {
+        if (threadIdx.x < 6u) s_bounds[threadIdx.x] = threadIdx.x < 3u ? 0x7fffffff : int(0x80000000);
+        __syncthreads();
+    }
+    bool bounded = false, need = false;
+    V3 centre{0.0f, 0.0f, 0.0f};
+    if (i < n) integrate_body(b, shapes, hull, i, dt, aabb_margin, begin, bounded, need, centre);
+    // The island pass is needed when some dynamic body is asleep or wants deactivation.
+    if (__ballot_sync(0xffffffffu, need) && (threadIdx.x & 31u) == 0u && *(volatile uint32_t*)begin.need == 0u)
+        atomicOr(begin.need, 1u);
+    if (!begin.bounds) return;
+    const int c[3] = {float_to_ordered(centre.x), float_to_ordered(centre.y), float_to_ordered(centre.z)};
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const bool in = bounded && (k == 0 ? centre.x == centre.x : (k == 1 ? centre.y == centre.y : centre.z == centre.z));
+        const int lo = __reduce_min_sync(0xffffffffu, in ? c[k] : 0x7fffffff);
+        const int hi = __reduce_max_sync(0xffffffffu, in ? c[k] : int(0x80000000));
+        if ((threadIdx.x & 31u) == 0u && lo <= hi) {
+            atomicMin(&s_bounds[k], lo);
+            atomicMax(&s_bounds[3 + k], hi);
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < 3u && s_bounds[threadIdx.x] <= s_bounds[3 + threadIdx.x]) {
+        atomicMin(&begin.bounds[threadIdx.x], s_bounds[threadIdx.x]);
+        atomicMax(&begin.bounds[3 + threadIdx.x], s_bounds[3 + threadIdx.x]);
+    }
 }
 
 // Static body AABBs at insertion (world.rs:548-552): pose, not predicted pose.
@@ -214,8 +260,8 @@ void launch_compute_iw(const BodyDev& b, uint32_t n, cudaStream_t s) {
 }
 
 void launch_integrate_velocities(const BodyDev& b, const Shape* shapes, const float4* hull, uint32_t n, float dt,
-                                 const StepReset& reset, cudaStream_t s) {
-    k_integrate_velocities<<<n ? (n + 255) / 256 : 1u, 256, 0, s>>>(b, shapes, hull, n, dt, 0.02f, reset);
+                                 const StepReset& reset, const StepBegin& begin, cudaStream_t s) {
+    k_integrate_velocities<<<n ? (n + 255) / 256 : 1u, 256, 0, s>>>(b, shapes, hull, n, dt, 0.02f, reset, begin);
 }
 
 void launch_initial_aabbs(const BodyDev& b, const Shape* shapes, const float4* hull, uint32_t first, uint32_t n,

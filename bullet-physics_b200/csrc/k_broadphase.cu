@@ -12,7 +12,7 @@
 // Unbounded proxies (planes) are kept out of the tree and joined by an ordered
 // flag/scan compaction.
 #include <cub/cub.cuh>
-#include "bgpu_kernels.cuh"
+#include "k_scan.cuh"
 
 namespace bgpu {
 
@@ -25,12 +25,6 @@ __device__ __forceinline__ bool overlaps(float4 amin, float4 amax, float4 bmin, 
     return amin.x <= bmax.x && amin.y <= bmax.y && amin.z <= bmax.z && bmin.x <= amax.x && bmin.y <= amax.y &&
            bmin.z <= amax.z;
 }
-
-__device__ __forceinline__ int float_to_ordered(float f) {
-    int i = __float_as_int(f);
-    return i >= 0 ? i : i ^ 0x7fffffff;
-}
-__device__ __forceinline__ float ordered_to_float(int i) { return __int_as_float(i >= 0 ? i : i ^ 0x7fffffff); }
 
 __global__ void k_reset_bounds(int* bounds) {
     if (threadIdx.x < 3) bounds[threadIdx.x] = 0x7fffffff;
@@ -78,8 +72,9 @@ __device__ __forceinline__ uint32_t quantize(float c, float lo, float hi) {
 // indices as values orders the proxies exactly as sorting (code << 32 | index) would, in
 // four 8-bit passes instead of eight.
 __global__ void k_keys(const float4* __restrict__ mn, const float4* __restrict__ mx, const uint32_t* __restrict__ is_unb,
-                       uint32_t n, const int* __restrict__ bounds, uint32_t* codes, uint32_t* index) {
+                       uint32_t n, const int* __restrict__ bounds, uint32_t* codes, uint32_t* index, uint32_t* zero) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0 && zero) *zero = 0u;  // the query's overflow count
     if (i >= n) return;
     index[i] = i;
     if (is_unb[i]) { codes[i] = 0xffffffffu; return; }
@@ -295,17 +290,175 @@ __global__ void k_query(int m, uint32_t n, const uint32_t* __restrict__ is_unb, 
     }
 }
 
-// Stashed segments (at most STASH_SLOTS partners) to their place in the pair list. Slot t
-// belongs to proxy leaf_body[t] (to proxy t when leaf_body is null).
-__global__ void k_stash_copy(int m, const uint32_t* __restrict__ leaf_body, const uint32_t* __restrict__ counts,
-                             const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ stash, uint64_t* out) {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= uint32_t(m)) return;
-    const uint32_t i = leaf_body ? leaf_body[t] : t;
-    const uint32_t c = counts[i];
-    if (c > STASH_SLOTS) return;
-    const uint64_t base = offsets[i];
-    for (uint32_t a = 0; a < c; ++a) out[base + a] = (uint64_t(i) << 32) | stash[size_t(a) * uint32_t(m) + t];
+// The partners j > h of each unbounded proxy h, tile by tile of proxies: their number (counts[h])
+// and, for the pass that writes them, how many lie before each tile (before[u tiles + tile]).
+constexpr uint32_t UNB_ROUNDS = 4;
+
+__device__ __forceinline__ uint32_t unb_ranks(uint32_t h, uint32_t base, uint32_t n, const float4* __restrict__ bmin,
+                                              const float4* __restrict__ bmax, bool (&flag)[UNB_ROUNDS],
+                                              uint32_t (&rank)[UNB_ROUNDS]) {
+    const float4 hmin = bmin[h], hmax = bmax[h];
+#pragma unroll
+    for (uint32_t r = 0; r < UNB_ROUNDS; ++r) {
+        const uint32_t j = base + r * TILE_TB + threadIdx.x;
+        flag[r] = j > h && j < n && overlaps(hmin, hmax, bmin[j], bmax[j]);
+    }
+    return tile_ranks(flag, rank);
+}
+
+__global__ void __launch_bounds__(TILE_TB) k_unb_tiles(uint32_t n, uint32_t tiles, const uint32_t* __restrict__ unb,
+                                                       const float4* __restrict__ bmin, const float4* __restrict__ bmax,
+                                                       uint32_t* before, uint32_t* counts, TileScan ts) {
+    const uint32_t tile = tile_take(ts), u = tile / tiles, t = tile % tiles;
+    bool flag[UNB_ROUNDS];
+    uint32_t rank[UNB_ROUNDS];
+    const uint32_t total = unb_ranks(unb[u], t * (TILE_TB * UNB_ROUNDS), n, bmin, bmax, flag, rank);
+    const uint32_t at = tile_prefix(ts, tile, u * tiles, total);
+    if (threadIdx.x == 0) {
+        before[tile] = at;
+        if (t + 1u == tiles) counts[unb[u]] = at + total;
+    }
+}
+
+// Where each proxy's segment starts, the number of pairs and of overflowing proxies (to the host).
+__global__ void __launch_bounds__(TILE_TB) k_segments(uint32_t n, const uint32_t* __restrict__ counts, uint32_t* offsets,
+                                                      const uint32_t* __restrict__ scalars, uint32_t* host, TileScan ts) {
+    const uint32_t tile = tile_take(ts), base = tile * (TILE_TB * 4u);
+    uint32_t v[4], before[4];
+#pragma unroll
+    for (uint32_t r = 0; r < 4; ++r) {
+        const uint32_t i = base + r * TILE_TB + threadIdx.x;
+        v[r] = i < n ? counts[i] : 0u;
+    }
+    const uint32_t total = tile_sums(v, before);
+    const uint32_t at = tile_prefix(ts, tile, 0u, total);
+#pragma unroll
+    for (uint32_t r = 0; r < 4; ++r) {
+        const uint32_t i = base + r * TILE_TB + threadIdx.x;
+        if (i < n) offsets[i] = at + before[r];
+    }
+    if (base + TILE_TB * 4u >= n && threadIdx.x == 0) {
+        host[0] = at + total;
+        host[1] = scalars[1];
+    }
+}
+
+// The segments at their place: the first stash_blocks blocks the stashed ones (slot t belongs to proxy
+// leaf_body[t], to proxy t when leaf_body is null), the others a tile of an unbounded proxy's partners.
+__global__ void __launch_bounds__(TILE_TB) k_write_pairs(int m, const uint32_t* __restrict__ leaf_body,
+                                                         const uint32_t* __restrict__ counts,
+                                                         const uint32_t* __restrict__ offsets,
+                                                         const uint32_t* __restrict__ stash, uint64_t* out,
+                                                         uint32_t stash_blocks, uint32_t n, uint32_t tiles,
+                                                         const uint32_t* __restrict__ unb, const float4* __restrict__ bmin,
+                                                         const float4* __restrict__ bmax,
+                                                         const uint32_t* __restrict__ before) {
+    if (blockIdx.x < stash_blocks) {
+        const uint32_t t = blockIdx.x * TILE_TB + threadIdx.x;
+        if (t >= uint32_t(m)) return;
+        const uint32_t i = leaf_body ? leaf_body[t] : t;
+        const uint32_t c = counts[i];
+        if (c > STASH_SLOTS) return;
+        const uint64_t base = offsets[i];
+        for (uint32_t a = 0; a < c; ++a) out[base + a] = (uint64_t(i) << 32) | stash[size_t(a) * uint32_t(m) + t];
+        return;
+    }
+    const uint32_t tile = blockIdx.x - stash_blocks, h = unb[tile / tiles], base = tile % tiles * (TILE_TB * UNB_ROUNDS);
+    bool flag[UNB_ROUNDS];
+    uint32_t rank[UNB_ROUNDS];
+    unb_ranks(h, base, n, bmin, bmax, flag, rank);
+    const uint64_t at = uint64_t(offsets[h]) + before[tile];
+#pragma unroll
+    for (uint32_t r = 0; r < UNB_ROUNDS; ++r)
+        if (flag[r]) out[at + rank[r]] = (uint64_t(h) << 32) | (base + r * TILE_TB + threadIdx.x);
+}
+
+// ---------------------------------------------------------------- all pairs (few proxies)
+// Bit j of row i: i < j and their boxes overlap. A lane holds proxy j and a warp tests 32 of them against
+// each row with one vote, so the partners come out in order and unbounded proxies are like any other. A
+// block tests 256 proxies against 128 rows staged in shared memory.
+constexpr uint32_t AP_ROWS = 128;
+
+__global__ void __launch_bounds__(256) k_all_pairs(uint32_t n, uint32_t words, const float4* __restrict__ bmin,
+                                                   const float4* __restrict__ bmax, uint32_t* masks) {
+    __shared__ float4 s_min[AP_ROWS], s_max[AP_ROWS];
+    const uint32_t i0 = blockIdx.y * AP_ROWS, j = blockIdx.x * 256u + threadIdx.x, lane = threadIdx.x & 31u;
+    if (i0 >= (blockIdx.x + 1u) * 256u) return;  // no j of the block lies above a row
+    if (threadIdx.x < AP_ROWS && i0 + threadIdx.x < n) {
+        s_min[threadIdx.x] = bmin[i0 + threadIdx.x];
+        s_max[threadIdx.x] = bmax[i0 + threadIdx.x];
+    }
+    float4 jmin = make_float4(0.f, 0.f, 0.f, 0.f), jmax = jmin;
+    if (j < n) { jmin = bmin[j]; jmax = bmax[j]; }
+    __syncthreads();
+    const uint32_t word = j >> 5;
+    if (word >= words) return;
+    for (uint32_t r0 = 0; r0 < AP_ROWS; r0 += 32u) {
+        uint32_t row = 0;
+#pragma unroll 8
+        for (uint32_t r = 0; r < 32u; ++r) {
+            const uint32_t i = i0 + r0 + r;
+            const uint32_t b = __ballot_sync(0xffffffffu, j > i && j < n && overlaps(s_min[r0 + r], s_max[r0 + r], jmin, jmax));
+            if (lane == r) row = b;
+        }
+        const uint32_t i = i0 + r0 + lane;
+        if (i < n && word >= i >> 5) masks[size_t(i) * words + word] = row;
+    }
+}
+
+// The rows' pairs, one warp a row and 64 rows a tile, as far as `out` holds them; the total to the host.
+constexpr uint32_t AP_TILE = 64;
+
+__global__ void __launch_bounds__(TILE_TB) k_all_pairs_rows(uint32_t n, uint32_t words, const uint32_t* __restrict__ masks,
+                                                            uint64_t* out, uint64_t cap, uint32_t* host, TileScan ts) {
+    __shared__ uint32_t s_cnt[AP_TILE], s_total;
+    const uint32_t tile = tile_take(ts), lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    constexpr uint32_t PER = AP_TILE / (TILE_TB / 32);
+    for (uint32_t r = 0; r < PER; ++r) {
+        const uint32_t k = warp * PER + r, i = tile * AP_TILE + k;
+        uint32_t c = 0;
+        if (i < n)
+            for (uint32_t w = (i >> 5) + lane; w < words; w += 32u) c += __popc(masks[size_t(i) * words + w]);
+        c = __reduce_add_sync(0xffffffffu, c);
+        if (lane == 0) s_cnt[k] = c;
+    }
+    __syncthreads();
+    if (warp == 0) {
+        const uint32_t a = s_cnt[2 * lane], b = s_cnt[2 * lane + 1];
+        uint32_t x = a + b;
+        for (uint32_t o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31u) s_total = x;
+        s_cnt[2 * lane] = x - a - b;
+        s_cnt[2 * lane + 1] = x - b;
+    }
+    __syncthreads();
+    const uint32_t total = s_total, at = tile_prefix(ts, tile, 0u, total);
+    if ((tile + 1u) * AP_TILE >= n && threadIdx.x == 0) {
+        host[0] = at + total;
+        host[1] = 0u;
+    }
+    if (uint64_t(at) + total > cap) return;  // the host makes room and comes again
+    for (uint32_t r = 0; r < PER; ++r) {
+        const uint32_t k = warp * PER + r, i = tile * AP_TILE + k;
+        if (i >= n) break;
+        uint64_t pos = uint64_t(at) + s_cnt[k];
+        for (uint32_t w0 = i >> 5; w0 < words; w0 += 32u) {  // uniform across the warp
+            const uint32_t w = w0 + lane;
+            uint32_t m = w < words ? masks[size_t(i) * words + w] : 0u;
+            const uint32_t c = __popc(m);
+            uint32_t x = c;
+            for (uint32_t o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= o) x += y;
+            }
+            uint64_t q = pos + x - c;
+            for (; m; m &= m - 1u) out[q++] = (uint64_t(i) << 32) | (w * 32u + uint32_t(__ffs(int(m)) - 1));
+            pos += __shfl_sync(0xffffffffu, x, 31);
+        }
+    }
 }
 
 // Unbounded proxy h: flags[j] = (j > h && overlap(h, j)) over all proxies.
@@ -443,29 +596,25 @@ __global__ void __launch_bounds__(WP_TILE) k_world_pairs_write(const float4* __r
 }  // namespace
 
 uint64_t Broadphase::run_worlds(const float4* aabb_min, const float4* aabb_max, uint32_t n, const uint32_t* world_off,
-                                uint32_t n_worlds, DevBuf<uint64_t>& out, cudaStream_t s) {
+                                uint32_t n_worlds, DevBuf<uint64_t>& out, uint32_t* status_dev, cudaStream_t s) {
     if (n == 0 || n_worlds == 0) return 0;
     counts.reserve(n);
     offsets.reserve(n);
-    scalars.reserve(4);
     stash.reserve(size_t(STASH_SLOTS) * n);
     overflow.reserve(n_worlds);
-    check_cuda(cudaMemsetAsync(scalars.p + 1, 0, sizeof(uint32_t), s), "memset");
     const uint32_t grid = std::min<uint32_t>(n_worlds, 148u * 32u);
     k_world_pairs<<<grid, WP_TILE, 0, s>>>(aabb_min, aabb_max, world_off, n_worlds, n, counts.p, stash.p, overflow.p,
                                            scalars.p + 1);
-    size_t scan_bytes = 0;
-    check_cuda(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, counts.p, offsets.p, int(n), s), "scan size");
-    cub_tmp.reserve(scan_bytes);
-    check_cuda(cub::DeviceScan::ExclusiveSum(cub_tmp.p, scan_bytes, counts.p, offsets.p, int(n), s), "scan");
-    k_total<<<1, 1, 0, s>>>(n, counts.p, offsets.p, scalars.p);
-    check_cuda(cudaMemcpyAsync(host_scalars, scalars.p, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s), "total d2h");
+    const uint32_t tiles = tile_count<4>(n);
+    k_segments<<<tiles, TILE_TB, 0, s>>>(n, counts.p, offsets.p, scalars.p, host_scalars, scan.begin(tiles, status_dev, s));
     check_cuda(cudaStreamSynchronize(s), "broadphase sync");
     uint64_t total = host_scalars[0];
     const uint32_t n_over = host_scalars[1];
     out.reserve(total + 1);
     if (total) {
-        k_stash_copy<<<(n + 255) / 256, 256, 0, s>>>(int(n), nullptr, counts.p, offsets.p, stash.p, out.p);
+        const uint32_t blocks = (n + TILE_TB - 1) / TILE_TB;
+        k_write_pairs<<<blocks, TILE_TB, 0, s>>>(int(n), nullptr, counts.p, offsets.p, stash.p, out.p, blocks, n, 1u,
+                                                 nullptr, nullptr, nullptr, nullptr);
         if (n_over)
             k_world_pairs_write<<<grid, WP_TILE, 0, s>>>(aabb_min, aabb_max, world_off, n_worlds, counts.p, offsets.p,
                                                          overflow.p, out.p);
@@ -474,6 +623,8 @@ uint64_t Broadphase::run_worlds(const float4* aabb_min, const float4* aabb_max, 
 }
 
 Broadphase::Broadphase() {
+    scalars.reserve(2);
+    bounds.reserve(12);
     check_cuda(cudaMallocHost(&host_scalars, 4 * sizeof(uint32_t)), "cudaMallocHost");
 }
 
@@ -482,9 +633,27 @@ Broadphase::~Broadphase() {
 }
 
 uint64_t Broadphase::run(const float4* aabb_min, const float4* aabb_max, uint32_t n,
-                         const std::vector<uint32_t>& unbounded_host, DevBuf<uint64_t>& out, uint32_t* status_dev,
-                         cudaStream_t s) {
+                         const std::vector<uint32_t>& unbounded_host, DevBuf<uint64_t>& out, bool all_pairs,
+                         const int* centres, uint32_t* status_dev, cudaStream_t s) {
     if (n == 0) return 0;
+    if (all_pairs) {
+        tree_m = 0;
+        nunb = 0;
+        const uint32_t words = (n + 31u) / 32u, tiles = (n + AP_TILE - 1) / AP_TILE;
+        masks.reserve(size_t(n) * words);
+        k_all_pairs<<<dim3((n + 255u) / 256u, (n + AP_ROWS - 1) / AP_ROWS), 256, 0, s>>>(n, words, aabb_min, aabb_max,
+                                                                                        masks.p);
+        // Written at once when the last step's array has room, as it does but for growth.
+        for (;;) {
+            const uint64_t cap = out.cap;
+            k_all_pairs_rows<<<tiles, TILE_TB, 0, s>>>(n, words, masks.p, out.p, cap, host_scalars,
+                                                       scan.begin(tiles, status_dev, s));
+            check_cuda(cudaStreamSynchronize(s), "broadphase sync");
+            const uint64_t total = host_scalars[0];
+            if (total <= cap) return total;
+            out.reserve(total + 1);
+        }
+    }
     const uint32_t nunb = uint32_t(unbounded_host.size());
     const int m = int(n - nunb);
     tree_m = m;
@@ -504,29 +673,31 @@ uint64_t Broadphase::run(const float4* aabb_min, const float4* aabb_max, uint32_
     node_rec.reserve(4 * size_t(n));
     counts.reserve(n);
     offsets.reserve(n);
-    flags.reserve(n);
-    scan_out.reserve(n);
-    bounds.reserve(6);
-    scalars.reserve(4);
+    is_unb.reserve(n);
     unbounded.reserve(nunb + 1);
-    if (nunb) check_cuda(cudaMemcpyAsync(unbounded.p, unbounded_host.data(), nunb * sizeof(uint32_t),
-                                         cudaMemcpyHostToDevice, s), "upload unbounded");
-    // flags doubles as the "is unbounded" marker until the unbounded pass.
-    k_clear_u32<<<grid, TB, 0, s>>>(n, flags.p);
-    if (nunb) k_set_unbounded<<<(nunb + TB - 1) / TB, TB, 0, s>>>(unbounded.p, nunb, flags.p);
-    k_reset_bounds<<<1, 32, 0, s>>>(bounds.p);
-    k_bounds<<<grid, TB, 0, s>>>(aabb_min, aabb_max, flags.p, n, bounds.p);
+    if (unb_n != n || unb_listed != unbounded_host) {  // the list changes only when bodies are added
+        unb_n = 0;
+        if (nunb) check_cuda(cudaMemcpyAsync(unbounded.p, unbounded_host.data(), nunb * sizeof(uint32_t),
+                                             cudaMemcpyHostToDevice, s), "upload unbounded");
+        k_clear_u32<<<grid, TB, 0, s>>>(n, is_unb.p);
+        if (nunb) k_set_unbounded<<<(nunb + TB - 1) / TB, TB, 0, s>>>(unbounded.p, nunb, is_unb.p);
+        unb_listed = unbounded_host;
+        unb_n = n;
+    }
+    if (!centres) {
+        k_reset_bounds<<<1, 32, 0, s>>>(bounds.p);
+        k_bounds<<<grid, TB, 0, s>>>(aabb_min, aabb_max, is_unb.p, n, bounds.p);
+        centres = bounds.p;
+    }
     // keys / keys_alt (n x 8 bytes each) hold the codes and indices and their sort buffers.
     uint32_t* codes = reinterpret_cast<uint32_t*>(keys.p);
     uint32_t* codes_alt = reinterpret_cast<uint32_t*>(keys_alt.p);
-    k_keys<<<grid, TB, 0, s>>>(aabb_min, aabb_max, flags.p, n, bounds.p, codes, codes + n);
+    k_keys<<<grid, TB, 0, s>>>(aabb_min, aabb_max, is_unb.p, n, centres, codes, codes + n, scalars.p + 1);
 
     size_t tmp_bytes = 0;
     cub::DoubleBuffer<uint32_t> dk(codes, codes_alt), dv(codes + n, codes_alt + n);
     check_cuda(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, dk, dv, int(n), 0, 32, s), "sort size");
-    size_t scan_bytes = 0;
-    check_cuda(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, counts.p, offsets.p, int(n), s), "scan size");
-    cub_tmp.reserve(std::max(tmp_bytes, scan_bytes));
+    cub_tmp.reserve(tmp_bytes);
     check_cuda(cub::DeviceRadixSort::SortPairs(cub_tmp.p, tmp_bytes, dk, dv, int(n), 0, 32, s), "sort");
     const LeafKeys sorted{dk.Current(), dv.Current()};
 
@@ -540,37 +711,29 @@ uint64_t Broadphase::run(const float4* aabb_min, const float4* aabb_max, uint32_
     // most STASH_SLOTS of them; the rest are listed and walk the tree again below.
     stash.reserve(size_t(STASH_SLOTS) * uint32_t(m > 0 ? m : 1));
     overflow.reserve(uint32_t(m > 0 ? m : 1));
-    check_cuda(cudaMemsetAsync(scalars.p, 0, 2 * sizeof(uint32_t), s), "memset");
-    k_query<Q_STASH><<<qgrid, TB, 0, s>>>(m, n, flags.p, aabb_min, aabb_max, node_rec.p, leaf_body.p, unbounded.p,
+    k_query<Q_STASH><<<qgrid, TB, 0, s>>>(m, n, is_unb.p, aabb_min, aabb_max, node_rec.p, leaf_body.p, unbounded.p,
                                           nunb, counts.p, nullptr, nullptr, status_dev, overflow.p, scalars.p + 1,
                                           stash.p);
-    // Unbounded proxies: count their segments by flag + scan.
-    for (uint32_t u = 0; u < nunb; ++u) {
-        uint32_t h = unbounded_host[u];
-        // scan_out holds the flags; the key scratch (no longer needed after the build) holds the scan.
-        k_unb_flags<<<grid, TB, 0, s>>>(h, n, aabb_min, aabb_max, scan_out.p);
-        check_cuda(cub::DeviceScan::ExclusiveSum(cub_tmp.p, scan_bytes, scan_out.p, (uint32_t*)keys_alt.p, int(n), s), "scan");
-        k_unb_count<<<1, 1, 0, s>>>(h, n, scan_out.p, (uint32_t*)keys_alt.p, counts.p);
+    const uint32_t utiles = tile_count<UNB_ROUNDS>(n), tiles = tile_count<4>(n);
+    if (nunb) {
+        unb_tiles.reserve(size_t(nunb) * utiles);
+        k_unb_tiles<<<nunb * utiles, TILE_TB, 0, s>>>(n, utiles, unbounded.p, aabb_min, aabb_max, unb_tiles.p, counts.p,
+                                                      scan.begin(nunb * utiles, status_dev, s));
     }
-    check_cuda(cub::DeviceScan::ExclusiveSum(cub_tmp.p, scan_bytes, counts.p, offsets.p, int(n), s), "scan");
-    k_total<<<1, 1, 0, s>>>(n, counts.p, offsets.p, scalars.p);
-    check_cuda(cudaMemcpyAsync(host_scalars, scalars.p, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s), "total d2h");
+    k_segments<<<tiles, TILE_TB, 0, s>>>(n, counts.p, offsets.p, scalars.p, host_scalars, scan.begin(tiles, status_dev, s));
     check_cuda(cudaStreamSynchronize(s), "broadphase sync");
     uint64_t total = host_scalars[0];
     const uint32_t n_overflow = host_scalars[1];
     out.reserve(total + 1);
     if (total) {
-        if (m > 0) k_stash_copy<<<qgrid, TB, 0, s>>>(m, leaf_body.p, counts.p, offsets.p, stash.p, out.p);
+        const uint32_t sblocks = m > 0 ? (uint32_t(m) + TILE_TB - 1) / TILE_TB : 0u;
+        k_write_pairs<<<sblocks + nunb * utiles, TILE_TB, 0, s>>>(m, leaf_body.p, counts.p, offsets.p, stash.p, out.p,
+                                                                  sblocks, n, utiles, unbounded.p, aabb_min, aabb_max,
+                                                                  unb_tiles.p);
         if (n_overflow)
             k_query<Q_WRITE><<<(n_overflow + TB - 1) / TB, TB, 0, s>>>(
-                m, n, flags.p, aabb_min, aabb_max, node_rec.p, leaf_body.p, unbounded.p, nunb, counts.p, offsets.p,
+                m, n, is_unb.p, aabb_min, aabb_max, node_rec.p, leaf_body.p, unbounded.p, nunb, counts.p, offsets.p,
                 out.p, status_dev, overflow.p, scalars.p + 1, nullptr);
-        for (uint32_t u = 0; u < nunb; ++u) {
-            uint32_t h = unbounded_host[u];
-            k_unb_flags<<<grid, TB, 0, s>>>(h, n, aabb_min, aabb_max, scan_out.p);
-            check_cuda(cub::DeviceScan::ExclusiveSum(cub_tmp.p, scan_bytes, scan_out.p, (uint32_t*)keys_alt.p, int(n), s), "scan");
-            k_unb_write<<<grid, TB, 0, s>>>(h, n, scan_out.p, (uint32_t*)keys_alt.p, offsets.p, out.p);
-        }
     }
     return total;
 }
@@ -755,7 +918,7 @@ extern "C" bgpu_status bgpu_broadphase_pairs_noalloc(const float* aabbs_dev, uin
         const int m = int(n - nunb);
         k_reset_bounds<<<1, 32, 0, s>>>(bounds);
         k_bounds<<<grid, TB, 0, s>>>(mn, mx, is_unb, n, bounds);
-        k_keys<<<grid, TB, 0, s>>>(mn, mx, is_unb, n, bounds, codes, codes + n);
+        k_keys<<<grid, TB, 0, s>>>(mn, mx, is_unb, n, bounds, codes, codes + n, nullptr);
         check_cuda(cub::DeviceRadixSort::SortPairs(tmp, sort_bytes, dk, dv, int(n), 0, 32, s), "sort");
         const LeafKeys sorted{dk.Current(), dv.Current()};
         if (m > 0) {

@@ -12,7 +12,7 @@
 //
 // When no dynamic body is asleep or wants deactivation, every island that has
 // a dynamic body is awake and the decision changes nothing, so the union-find
-// is skipped (k_island_need raises the flag that the other kernels test).
+// is skipped (the step's first kernel raises the flag that these test).
 //
 // Pairs whose two bodies are both awake (Active / DisableDeactivation) are not
 // linked. That cannot change any body's decision: a set of the thinner
@@ -22,6 +22,7 @@
 // whose awake ends it holds. So every body lands in a set with an awake member
 // exactly when its island has one, and a set with none (touched by a moving
 // kinematic or not) is the whole island.
+#include <algorithm>
 #include "bgpu_kernels.cuh"
 
 namespace bgpu {
@@ -53,7 +54,6 @@ __device__ __forceinline__ uint32_t find_root(const uint32_t* parent, uint32_t x
     return x;
 }
 
-// need = 1 when some dynamic body is island-sleeping or wants deactivation.
 // find with path halving: every visited node is pointed at its grandparent.
 // Only roots are ever linked (atomicCAS) and a node that stopped being a root
 // never becomes one again, so the grandparent is always an ancestor and the
@@ -70,23 +70,6 @@ __device__ __forceinline__ uint32_t find_halving(uint32_t* parent, uint32_t x, u
     return x;
 }
 
-__global__ void k_island_need(const uint4* __restrict__ info, uint32_t n, uint32_t* need) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    bool c = false;
-    if (i < n) {
-        uint4 in = info[i];
-        c = participates(in.y) && (in.z == ACT_ISLAND_SLEEPING || in.z == ACT_WANTS_DEACTIVATION);
-    }
-    if (__ballot_sync(0xffffffffu, c) && (threadIdx.x & 31u) == 0u && *(volatile uint32_t*)need == 0u) atomicOr(need, 1u);
-}
-
-__global__ void k_uf_init(uint32_t n, uint32_t* parent, uint32_t* awake) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    parent[i] = i;
-    awake[i] = 0;
-}
-
 __device__ __forceinline__ void link(uint32_t* parent, uint32_t a, uint32_t b, uint32_t* status) {
     for (int g = 0; g < UF_LIMIT; ++g) {
         uint32_t ra = find_halving(parent, a, status), rb = find_halving(parent, b, status);
@@ -97,24 +80,8 @@ __device__ __forceinline__ void link(uint32_t* parent, uint32_t a, uint32_t b, u
     atomicOr(status, ST_UNION_FIND_LIMIT);
 }
 
-__global__ void k_uf_link(const uint4* __restrict__ info, const uint64_t* __restrict__ pairs, uint32_t npairs,
-                          uint32_t* parent, uint32_t* status, const uint32_t* __restrict__ need) {
-    uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= npairs || !*need) return;
-    uint64_t k = pairs[p];
-    uint32_t a = key_lo(k), b = key_hi(k);
-    uint4 ia = info[a], ib = info[b];
-    if (!eligible(ia, ib) || !participates(ia.y) || !participates(ib.y)) return;
-    if (awake_member(ia) && awake_member(ib)) return;
-    link(parent, a, b, status);
-}
-
-// islands.rs:186-196: an enabled joint between two dynamic bodies links their islands
-// (whatever its collision suppression).
-__global__ void k_uf_link_joints(const uint4* __restrict__ info, const float4* __restrict__ desc, uint32_t nj,
-                                 uint32_t* parent, uint32_t* status, const uint32_t* __restrict__ need) {
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= nj || !*need) return;
+__device__ __forceinline__ void link_joint(const uint4* __restrict__ info, const float4* __restrict__ desc, uint32_t j,
+                                           uint32_t* parent, uint32_t* status) {
     const float4 h = desc[size_t(j) * JOINT_F4];
     if (__float_as_uint(h.w) & JF_DISABLED) return;
     const uint32_t a = __float_as_uint(h.y), b = __float_as_uint(h.z);
@@ -124,29 +91,29 @@ __global__ void k_uf_link_joints(const uint4* __restrict__ info, const float4* _
     link(parent, a, b, status);
 }
 
-__global__ void k_uf_flatten_awake(const uint4* __restrict__ info, uint32_t n, uint32_t* parent, uint32_t* awake,
-                                   uint32_t* status, const uint32_t* __restrict__ need) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n || !*need) return;
-    uint32_t r = find_root(parent, i, status);
-    uint4 in = info[i];
-    if (awake_member(in)) awake[r] = 1u;
-}
-
-__global__ void k_uf_store_roots(uint32_t n, uint32_t* parent, uint32_t* status, const uint32_t* __restrict__ need) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n || !*need) return;
-    // Writing the root is safe while other threads still walk: every pointer still leads to it.
-    parent[i] = find_root(parent, i, status);
+// Pairs, then joints (islands.rs:186-196: an enabled joint between two dynamic bodies links their
+// islands, whatever its collision suppression).
+__global__ void k_uf_link(const uint4* __restrict__ info, const uint64_t* __restrict__ pairs, uint32_t npairs,
+                          const float4* __restrict__ desc, uint32_t nj, uint32_t* parent, uint32_t* status,
+                          const uint32_t* __restrict__ need) {
+    uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= npairs + nj || !*need) return;
+    if (p >= npairs) {
+        link_joint(info, desc, p - npairs, parent, status);
+        return;
+    }
+    uint64_t k = pairs[p];
+    uint32_t a = key_lo(k), b = key_hi(k);
+    uint4 ia = info[a], ib = info[b];
+    if (!eligible(ia, ib) || !participates(ia.y) || !participates(ib.y)) return;
+    if (awake_member(ia) && awake_member(ib)) return;
+    link(parent, a, b, status);
 }
 
 // islands.rs:232-279 — a moving kinematic wakes every eligible island it pairs with.
-__global__ void k_kinematic_wake(const uint4* __restrict__ info, const float4* __restrict__ lv, const float4* __restrict__ av,
-                                 const uint64_t* __restrict__ pairs, uint32_t npairs, const uint32_t* __restrict__ root,
-                                 uint32_t* awake, const uint32_t* __restrict__ need) {
-    uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= npairs || !*need) return;
-    uint64_t k = pairs[p];
+__device__ __forceinline__ void kinematic_wake(const uint4* __restrict__ info, const float4* __restrict__ lv,
+                                               const float4* __restrict__ av, uint64_t k, const uint32_t* parent,
+                                               uint32_t* awake, uint32_t* status) {
     uint32_t ends[2] = {key_lo(k), key_hi(k)};
     int ks = -1;
     for (int s = 0; s < 2; ++s) {
@@ -161,7 +128,23 @@ __global__ void k_kinematic_wake(const uint4* __restrict__ info, const float4* _
     if (!eligible(ia, ib)) return;
     uint32_t other = ends[1 - ks];
     if (!participates(info[other].y)) return;
-    awake[root[other]] = 1u;
+    awake[find_root(parent, other, status)] = 1u;
+}
+
+// Every body's root, and the awake islands: those with an awake member or (the threads of the pairs) a
+// moving kinematic beside them. Writing a root is safe while other threads still walk: every pointer
+// still leads to it, and nothing links any more.
+__global__ void k_uf_awake(const uint4* __restrict__ info, const float4* __restrict__ lv, const float4* __restrict__ av,
+                           uint32_t n, const uint64_t* __restrict__ pairs, uint32_t npairs, uint32_t* parent,
+                           uint32_t* awake, uint32_t* status, const uint32_t* __restrict__ need) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (!*need) return;
+    if (i < n) {
+        const uint32_t r = find_root(parent, i, status);
+        if (awake_member(info[i])) awake[r] = 1u;
+        __stcg(&parent[i], r);
+    }
+    if (i < npairs) kinematic_wake(info, lv, av, pairs[i], parent, awake, status);
 }
 
 // islands.rs:281-294 + body.rs:578-624; also raises the `simulate` flag (step.rs:440) of the
@@ -206,26 +189,18 @@ __global__ void k_uf_apply(uint4* info, float4* lv, float4* av, float4* sleep, u
 }  // namespace
 
 void Islands::run(const BodyDev& b, uint32_t n, const uint64_t* pairs, uint32_t npairs, const uint32_t* world_of,
-                  uint32_t* simulate_flag, uint32_t* status_dev, cudaStream_t s, const float4* joint_desc,
-                  uint32_t njoints) {
+                  const uint32_t* need_now, uint32_t* simulate_flag, uint32_t* status_dev, cudaStream_t s,
+                  const float4* joint_desc, uint32_t njoints) {
     if (n == 0) return;
-    parent.reserve(n);
-    awake.reserve(n);
-    need.reserve(1);
-    check_cuda(cudaMemsetAsync(need.p, 0, sizeof(uint32_t), s), "memset");
     const int TB = 256;
-    k_island_need<<<(n + TB - 1) / TB, TB, 0, s>>>(b.info, n, need.p);
-    k_uf_init<<<(n + TB - 1) / TB, TB, 0, s>>>(n, parent.p, awake.p);
-    if (npairs) k_uf_link<<<(npairs + TB - 1) / TB, TB, 0, s>>>(b.info, pairs, npairs, parent.p, status_dev, need.p);
-    if (njoints)
-        k_uf_link_joints<<<(njoints + TB - 1) / TB, TB, 0, s>>>(b.info, joint_desc, njoints, parent.p, status_dev, need.p);
-    k_uf_flatten_awake<<<(n + TB - 1) / TB, TB, 0, s>>>(b.info, n, parent.p, awake.p, status_dev, need.p);
-    k_uf_store_roots<<<(n + TB - 1) / TB, TB, 0, s>>>(n, parent.p, status_dev, need.p);
-    if (npairs)
-        k_kinematic_wake<<<(npairs + TB - 1) / TB, TB, 0, s>>>(b.info, b.linvel, b.angvel, pairs, npairs, parent.p,
-                                                                awake.p, need.p);
+    const uint32_t links = npairs + njoints, most = std::max(n, npairs);
+    if (links)
+        k_uf_link<<<(links + TB - 1) / TB, TB, 0, s>>>(b.info, pairs, npairs, joint_desc, njoints, parent.p, status_dev,
+                                                       need_now);
+    k_uf_awake<<<(most + TB - 1) / TB, TB, 0, s>>>(b.info, b.linvel, b.angvel, n, pairs, npairs, parent.p, awake.p,
+                                                   status_dev, need_now);
     k_uf_apply<<<(n + TB - 1) / TB, TB, 0, s>>>(b.info, b.linvel, b.angvel, b.sleep, n, parent.p, awake.p, world_of,
-                                                 simulate_flag, b.rec_flags, need.p);
+                                                 simulate_flag, b.rec_flags, need_now);
 }
 
 }  // namespace bgpu

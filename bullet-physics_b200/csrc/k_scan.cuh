@@ -116,4 +116,38 @@ __device__ __forceinline__ uint32_t tile_ranks(const bool (&flag)[ROUNDS], uint3
     return s_total;
 }
 
+// Exclusive sums of the items' values over the tile in item order; returns the tile's total.
+template <uint32_t ROUNDS>
+__device__ __forceinline__ uint32_t tile_sums(const uint32_t (&value)[ROUNDS], uint32_t (&before)[ROUNDS]) {
+    constexpr uint32_t WARPS = TILE_TB / 32, N = WARPS * ROUNDS;
+    static_assert(N <= 32, "one warp scans the sums");
+    __shared__ uint32_t s_sum[32], s_total;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (uint32_t r = 0; r < ROUNDS; ++r) {
+        uint32_t x = value[r];
+        for (uint32_t o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        before[r] = x - value[r];
+        if (lane == 31u) s_sum[r * WARPS + warp] = x;
+    }
+    __syncthreads();
+    if (warp == 0) {
+        const uint32_t c = lane < N ? s_sum[lane] : 0u;
+        uint32_t x = c;
+        for (uint32_t o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        s_sum[lane] = x - c;
+        if (lane == 31u) s_total = x;
+    }
+    __syncthreads();
+#pragma unroll
+    for (uint32_t r = 0; r < ROUNDS; ++r) before[r] += s_sum[r * WARPS + warp];
+    return s_total;
+}
+
 }  // namespace bgpu

@@ -168,6 +168,7 @@ struct World {
     uint32_t standalone_groups = 0;
     DevBuf<uint64_t> standalone_keys;
     uint64_t step_count = 0;  // steps taken (seeded vs full colouring)
+    int begin_parity = 0;     // which of the paired accumulators (StepBegin) the next step uses
     static constexpr uint64_t RECOLOUR_PERIOD = 64;
     // adjoint recording: the step being recorded (null otherwise) and the pair pass's scratch
     StepRecord* rec_step = nullptr;
@@ -212,6 +213,12 @@ struct World {
         check_cuda(cudaMemsetAsync(cache[0].count_dev, 0, sizeof(uint32_t), stream), "memset");
         check_cuda(cudaMemsetAsync(cache[1].count_dev, 0, sizeof(uint32_t), stream), "memset");
         pd.reserve_counters();
+        islands.reserve(1);
+        check_cuda(cudaMemsetAsync(islands.need.p, 0, 2 * sizeof(uint32_t), stream), "memset");
+        const int none[12] = {0x7fffffff, 0x7fffffff, 0x7fffffff, int(0x80000000), int(0x80000000), int(0x80000000),
+                              0x7fffffff, 0x7fffffff, 0x7fffffff, int(0x80000000), int(0x80000000), int(0x80000000)};
+        check_cuda(cudaMemcpyAsync(bp.bounds.p, none, sizeof(none), cudaMemcpyHostToDevice, stream), "bounds");
+        check_cuda(cudaStreamSynchronize(stream), "sync");
         pd.old_owned.reserve(1);
         for (auto& set : ev)
             for (auto& e : set) check_cuda(cudaEventCreate(&e), "event");
@@ -915,16 +922,26 @@ struct World {
         reset.add(status, 1);
         reset.add(simulate, nw);
         pd.add_counters(reset);
+        reset.add(bp.scalars.p, 2);
         reset.owned = pd.old_owned.p;
         reset.owned_n = cache[cur].count_dev;
         mark(0);
         // 1-3: velocities, predicted poses, AABBs (fused).
-        launch_integrate_velocities(b, shapes_d.p, hull_d.p, n, dt, reset, stream);
+        // Few bodies: every pair is tested, with no tree (which CCD sweeps over many bodies want).
+        const bool all_pairs = !batch && n <= Broadphase::ALL_PAIRS_MAX && (nccd == 0 || n <= 1024);
+        islands.reserve(n);
+        const int now = begin_parity, next_begin = now ^ 1;
+        uint32_t* need = islands.need.p + now;
+        int* bounds = batch || all_pairs ? nullptr : bp.bounds.p + 6 * now;
+        launch_integrate_velocities(b, shapes_d.p, hull_d.p, n, dt, reset,
+                                    StepBegin{bounds, bp.bounds.p + 6 * next_begin, need, islands.need.p + next_begin,
+                                              islands.parent.p, islands.awake.p}, stream);
+        begin_parity = next_begin;
         mark(1);
         // 4: broad phase (syncs once to size the pair arrays; the previous step's
         //    manifold count and timing events are read at the same point).
-        uint64_t np = batch ? bp.run_worlds(aabb_min.p, aabb_max.p, n, world_off_d.p, nw, pairs, stream)
-                            : bp.run(aabb_min.p, aabb_max.p, n, unbounded, pairs, status, stream);
+        uint64_t np = batch ? bp.run_worlds(aabb_min.p, aabb_max.p, n, world_off_d.p, nw, pairs, status, stream)
+                            : bp.run(aabb_min.p, aabb_max.p, n, unbounded, pairs, all_pairs, bounds, status, stream);
         npairs = uint32_t(np);
         if (timing) fold(ev_cur ^ 1);
         Manifolds& old_cache = cache[cur];
@@ -933,7 +950,7 @@ struct World {
         if (rec_step) prepare_record(old_cache.count_host);
         mark(2);
         // 4b: islands
-        islands.run(b, n, pairs.p, npairs, world_of, simulate, status, stream, jd.desc, jd.n);
+        islands.run(b, n, pairs.p, npairs, world_of, need, simulate, status, stream, jd.desc, jd.n);
         mark(3);
         // 5: pair pass
         pd.reserve(std::max<uint32_t>(npairs, 1), n, old_cache.count_host);
@@ -2412,7 +2429,7 @@ bgpu_status bgpu_broadphase_pairs(const float* aabbs, uint32_t n, uint32_t* out,
             bgpu::check_cuda(cudaMemcpyAsync(dmx.p, mx.data(), n * sizeof(float4), cudaMemcpyHostToDevice, s), "h2d");
         }
         bgpu::Broadphase bp;
-        uint64_t np = bp.run(dmn.p, dmx.p, n, unb, pairs, status.p, s);
+        uint64_t np = bp.run(dmn.p, dmx.p, n, unb, pairs, n <= bgpu::Broadphase::ALL_PAIRS_MAX, nullptr, status.p, s);
         uint32_t st = 0;
         bgpu::check_cuda(cudaMemcpyAsync(&st, status.p, 4, cudaMemcpyDeviceToHost, s), "d2h");
         std::vector<uint64_t> keys(np);
