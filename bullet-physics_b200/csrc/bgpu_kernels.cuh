@@ -280,16 +280,23 @@ struct Broadphase {
     ~Broadphase();
     // Up to this many proxies every pair is tested (no tree): n^2 / 2 tests cost less than the tree's
     // launches and climbs. Broad phase of settled piles, all pairs / tree: 1,024 bodies 57 / 118 us,
-    // 4,096 74 / 144, 8,000 97 / 197, 12,500 161 / 201, 16,250 218 / 208.
+    // 4,096 74 / 144, 8,000 97 / 197, 12,500 161 / 201, 16,250 218 / 208 (the all-pairs pass has become
+    // faster since: 5,700 bodies 56 -> 34 us).
     static constexpr uint32_t ALL_PAIRS_MAX = 12288;
     // Returns the pair count; pairs are written to `out` (grown as needed). all_pairs: test every
     // pair (n <= ALL_PAIRS_MAX). centres: the bounded proxies' centre bounds when a kernel before
     // has them, else null.
     uint64_t run(const float4* aabb_min, const float4* aabb_max, uint32_t n, const std::vector<uint32_t>& unbounded_host,
                  DevBuf<uint64_t>& out, bool all_pairs, const int* centres, uint32_t* status_dev, cudaStream_t s);
-    // Batched worlds: pairs only inside each world [world_off[k], world_off[k + 1]) (device array).
-    uint64_t run_worlds(const float4* aabb_min, const float4* aabb_max, uint32_t n, const uint32_t* world_off,
-                        uint32_t n_worlds, DevBuf<uint64_t>& out, uint32_t* status_dev, cudaStream_t s);
+    // Batched worlds: pairs only inside each world [world_off[k], world_off[k + 1]) (the same offsets on the
+    // host and on the device; world_of: each body's world).
+    uint64_t run_worlds(const float4* aabb_min, const float4* aabb_max, uint32_t n,
+                        const std::vector<uint32_t>& world_off_host, const uint32_t* world_off, const uint32_t* world_of,
+                        DevBuf<uint64_t>& out, uint32_t* status_dev, cudaStream_t s);
+    DevBuf<uint32_t> mask_off;         // each world's first mask word
+    uint32_t mask_worlds = 0, mask_n = 0;  // the batch that mask_off describes
+    uint64_t mask_words = 0;           // its masks
+    static constexpr uint64_t WORLD_MASK_WORDS_MAX = 1ull << 28;  // 1 GB of masks
 };
 
 // ---------------------------------------------------------------- islands (k_islands.cu)

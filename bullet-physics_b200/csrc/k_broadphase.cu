@@ -26,6 +26,12 @@ __device__ __forceinline__ bool overlaps(float4 amin, float4 amax, float4 bmin, 
            bmin.z <= amax.z;
 }
 
+// The same without branches, for the loops in which every lane tests.
+__device__ __forceinline__ bool overlaps_all(float4 amin, float4 amax, float4 bmin, float4 bmax) {
+    return (amin.x <= bmax.x) & (amin.y <= bmax.y) & (amin.z <= bmax.z) & (bmin.x <= amax.x) & (bmin.y <= amax.y) &
+           (bmin.z <= amax.z);
+}
+
 __global__ void k_reset_bounds(int* bounds) {
     if (threadIdx.x < 3) bounds[threadIdx.x] = 0x7fffffff;
     else if (threadIdx.x < 6) bounds[threadIdx.x] = int(0x80000000);
@@ -398,7 +404,8 @@ __global__ void __launch_bounds__(256) k_all_pairs(uint32_t n, uint32_t words, c
 #pragma unroll 8
         for (uint32_t r = 0; r < 32u; ++r) {
             const uint32_t i = i0 + r0 + r;
-            const uint32_t b = __ballot_sync(0xffffffffu, j > i && j < n && overlaps(s_min[r0 + r], s_max[r0 + r], jmin, jmax));
+            const uint32_t b = __ballot_sync(0xffffffffu, (j > i) & (j < n) &
+                                                              overlaps_all(s_min[r0 + r], s_max[r0 + r], jmin, jmax));
             if (lane == r) row = b;
         }
         const uint32_t i = i0 + r0 + lane;
@@ -406,14 +413,16 @@ __global__ void __launch_bounds__(256) k_all_pairs(uint32_t n, uint32_t words, c
     }
 }
 
-// The rows' pairs, one warp a row and 64 rows a tile, as far as `out` holds them; the total to the host.
-constexpr uint32_t AP_TILE = 64;
+// The rows' pairs, one warp a row and 16 rows a tile (many blocks: 1,000 proxies took 12 us with 64), as
+// far as `out` holds them; the total to the host.
+constexpr uint32_t AP_TILE = 16;
 
 __global__ void __launch_bounds__(TILE_TB) k_all_pairs_rows(uint32_t n, uint32_t words, const uint32_t* __restrict__ masks,
                                                             uint64_t* out, uint64_t cap, uint32_t* host, TileScan ts) {
     __shared__ uint32_t s_cnt[AP_TILE], s_total;
     const uint32_t tile = tile_take(ts), lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     constexpr uint32_t PER = AP_TILE / (TILE_TB / 32);
+#pragma unroll
     for (uint32_t r = 0; r < PER; ++r) {
         const uint32_t k = warp * PER + r, i = tile * AP_TILE + k;
         uint32_t c = 0;
@@ -424,15 +433,14 @@ __global__ void __launch_bounds__(TILE_TB) k_all_pairs_rows(uint32_t n, uint32_t
     }
     __syncthreads();
     if (warp == 0) {
-        const uint32_t a = s_cnt[2 * lane], b = s_cnt[2 * lane + 1];
-        uint32_t x = a + b;
+        const uint32_t a = lane < AP_TILE ? s_cnt[lane] : 0u;
+        uint32_t x = a;
         for (uint32_t o = 1; o < 32; o <<= 1) {
             const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
             if (lane >= o) x += y;
         }
         if (lane == 31u) s_total = x;
-        s_cnt[2 * lane] = x - a - b;
-        s_cnt[2 * lane + 1] = x - b;
+        if (lane < AP_TILE) s_cnt[lane] = x - a;
     }
     __syncthreads();
     const uint32_t total = s_total, at = tile_prefix(ts, tile, 0u, total);
@@ -441,6 +449,7 @@ __global__ void __launch_bounds__(TILE_TB) k_all_pairs_rows(uint32_t n, uint32_t
         host[1] = 0u;
     }
     if (uint64_t(at) + total > cap) return;  // the host makes room and comes again
+#pragma unroll
     for (uint32_t r = 0; r < PER; ++r) {
         const uint32_t k = warp * PER + r, i = tile * AP_TILE + k;
         if (i >= n) break;
@@ -593,13 +602,136 @@ __global__ void __launch_bounds__(WP_TILE) k_world_pairs_write(const float4* __r
     }
 }
 
+// Bit j of row i of each world's masks (i < j, in the world's own numbers): their boxes overlap; counts[i]
+// the row's bits. One CTA a world, a lane a proxy j, a vote per 32 tests (k_all_pairs, world by world).
+// A thread per proxy that walked the others one by one and kept what it found took 91 us for 4,096
+// worlds of 8 to 256 bodies and 79 us for 96 of them (a ground plane's 255 partners, one store after the
+// other); this takes 41 and 12.
+constexpr uint32_t WM_TILE = 128;
+
+__global__ void __launch_bounds__(WM_TILE) k_world_masks(const float4* __restrict__ bmin, const float4* __restrict__ bmax,
+                                                         const uint32_t* __restrict__ off, uint32_t n_worlds,
+                                                         const uint32_t* __restrict__ mask_off, uint32_t* masks,
+                                                         uint32_t* counts) {
+    __shared__ float4 s_min[WM_TILE], s_max[WM_TILE];
+    __shared__ uint32_t s_cnt[WM_TILE];
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint32_t w = blockIdx.x; w < n_worlds; w += gridDim.x) {
+        const uint32_t lo = off[w], nb = off[w + 1] - lo, words = (nb + 31u) / 32u;
+        uint32_t* m = masks + mask_off[w];
+        for (uint32_t i0 = 0; i0 < nb; i0 += WM_TILE) {
+            __syncthreads();  // the tile before is done with
+            if (i0 + threadIdx.x < nb) {
+                s_min[threadIdx.x] = bmin[lo + i0 + threadIdx.x];
+                s_max[threadIdx.x] = bmax[lo + i0 + threadIdx.x];
+            }
+            s_cnt[threadIdx.x] = 0u;
+            __syncthreads();
+            const uint32_t rows = min(WM_TILE, nb - i0);
+            for (uint32_t j0 = i0; j0 < nb; j0 += WM_TILE) {
+                const uint32_t j = j0 + threadIdx.x, word = j >> 5;
+                if (word >= words) continue;  // uniform across the warp
+                float4 jmin = make_float4(0.f, 0.f, 0.f, 0.f), jmax = jmin;
+                if (j < nb) { jmin = bmin[lo + j]; jmax = bmax[lo + j]; }
+                for (uint32_t r0 = 0; r0 < rows; r0 += 32u) {
+                    if (word < (i0 + r0) >> 5) continue;  // no j of the word lies above these rows
+                    uint32_t row = 0;
+#pragma unroll 8
+                    for (uint32_t r = 0; r < 32u; ++r) {
+                        const uint32_t b = __ballot_sync(0xffffffffu, (j > i0 + r0 + r) & (j < nb) &
+                                                                          overlaps_all(s_min[r0 + r], s_max[r0 + r], jmin, jmax));
+                        if (lane == r) row = b;
+                    }
+                    if (r0 + lane < rows) {
+                        m[size_t(i0 + r0 + lane) * words + word] = row;
+                        if (row) atomicAdd(&s_cnt[r0 + lane], __popc(row));
+                    }
+                }
+            }
+            __syncthreads();
+            if (threadIdx.x < rows) counts[lo + i0 + threadIdx.x] = s_cnt[threadIdx.x];
+        }
+    }
+}
+
+// The rows' pairs: a thread a row, but rows of many partners (a ground plane's) by the whole warp.
+__global__ void __launch_bounds__(256) k_world_rows(uint32_t n, const uint32_t* __restrict__ off,
+                                                    const uint32_t* __restrict__ world_of,
+                                                    const uint32_t* __restrict__ mask_off,
+                                                    const uint32_t* __restrict__ masks, const uint32_t* __restrict__ counts,
+                                                    const uint32_t* __restrict__ offsets, uint64_t* out) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31u;
+    uint32_t cnt = 0, lo = 0, words = 0, first = 0;
+    uint64_t pos = 0;
+    if (i < n) {
+        cnt = counts[i];
+        if (cnt) {
+            const uint32_t w = world_of[i];
+            lo = off[w];
+            words = (off[w + 1] - lo + 31u) / 32u;
+            first = mask_off[w] + (i - lo) * words;
+            pos = offsets[i];
+        }
+    }
+    const bool wide = cnt > 48u;
+    if (cnt && !wide) {
+        for (uint32_t w = (i - lo) >> 5; w < words && cnt; ++w)
+            for (uint32_t m = masks[first + w]; m; m &= m - 1u, --cnt)
+                out[pos++] = (uint64_t(i) << 32) | (lo + w * 32u + uint32_t(__ffs(int(m)) - 1));
+    }
+    for (uint32_t todo = __ballot_sync(0xffffffffu, wide); todo; todo &= todo - 1u) {
+        const int src = __ffs(int(todo)) - 1;
+        const uint32_t ri = __shfl_sync(0xffffffffu, i, src), rlo = __shfl_sync(0xffffffffu, lo, src);
+        const uint32_t rwords = __shfl_sync(0xffffffffu, words, src), rfirst = __shfl_sync(0xffffffffu, first, src);
+        uint64_t rpos = __shfl_sync(0xffffffffu, static_cast<unsigned long long>(pos), src);
+        for (uint32_t w = (ri - rlo) >> 5; w < rwords; ++w) {
+            const uint32_t m = masks[rfirst + w];
+            if ((m >> lane) & 1u)
+                out[rpos + __popc(m & ((1u << lane) - 1u))] = (uint64_t(ri) << 32) | (rlo + w * 32u + lane);
+            rpos += __popc(m);
+        }
+    }
+}
+
 }  // namespace
 
-uint64_t Broadphase::run_worlds(const float4* aabb_min, const float4* aabb_max, uint32_t n, const uint32_t* world_off,
-                                uint32_t n_worlds, DevBuf<uint64_t>& out, uint32_t* status_dev, cudaStream_t s) {
+uint64_t Broadphase::run_worlds(const float4* aabb_min, const float4* aabb_max, uint32_t n,
+                                const std::vector<uint32_t>& world_off_host, const uint32_t* world_off,
+                                const uint32_t* world_of, DevBuf<uint64_t>& out, uint32_t* status_dev, cudaStream_t s) {
+    const uint32_t n_worlds = uint32_t(world_off_host.size() - 1);
     if (n == 0 || n_worlds == 0) return 0;
     counts.reserve(n);
     offsets.reserve(n);
+    if (mask_worlds != n_worlds || mask_n != n) {  // worlds were added
+        std::vector<uint32_t> first(n_worlds);
+        mask_words = 0;
+        for (uint32_t k = 0; k < n_worlds; ++k) {
+            const uint64_t nb = world_off_host[k + 1] - world_off_host[k];
+            first[k] = uint32_t(mask_words);
+            mask_words += nb * ((nb + 31u) / 32u);
+        }
+        mask_off.reserve(n_worlds);
+        check_cuda(cudaMemcpyAsync(mask_off.p, first.data(), n_worlds * sizeof(uint32_t), cudaMemcpyHostToDevice, s), "h2d");
+        check_cuda(cudaStreamSynchronize(s), "sync");
+        mask_worlds = n_worlds;
+        mask_n = n;
+    }
+    if (mask_words <= WORLD_MASK_WORDS_MAX) {
+        masks.reserve(mask_words);
+        k_world_masks<<<std::min<uint32_t>(n_worlds, 148u * 32u), WM_TILE, 0, s>>>(aabb_min, aabb_max, world_off, n_worlds,
+                                                                                 mask_off.p, masks.p, counts.p);
+        const uint32_t tiles = tile_count<4>(n);
+        k_segments<<<tiles, TILE_TB, 0, s>>>(n, counts.p, offsets.p, scalars.p, host_scalars,
+                                             scan.begin(tiles, status_dev, s));
+        check_cuda(cudaStreamSynchronize(s), "broadphase sync");
+        const uint64_t total = host_scalars[0];
+        out.reserve(total + 1);
+        if (total)
+            k_world_rows<<<(n + 255) / 256, 256, 0, s>>>(n, world_off, world_of, mask_off.p, masks.p, counts.p, offsets.p,
+                                                         out.p);
+        return total;
+    }
+    // Masks of more than a gigabyte (a world of some 90,000 bodies): the stash pass.
     stash.reserve(size_t(STASH_SLOTS) * n);
     overflow.reserve(n_worlds);
     const uint32_t grid = std::min<uint32_t>(n_worlds, 148u * 32u);

@@ -139,6 +139,11 @@ struct World {
     // (threads per CTA, largest world solved by one warp), and the per-world batch records
     WorldPlan wplan;
     uint32_t wplan_block = 128, wplan_tau = 64;  // 0 threads: the global (all-worlds) solver
+    // Until a caller tunes, worlds of a few bodies more than wplan_tau run one per warp too: a block's other
+    // warps would only wait (1,024 worlds of 64 boxes and a plane: 200 us a solve in blocks of 128
+    // threads, four waves of them, 145 us one per warp).
+    static constexpr uint32_t UNTUNED_WARP_WORLD_BODIES = 96;
+    bool wplan_tuned = false;
     DevBuf<uint32_t> wcol;
     DevBuf<uint32_t> plain_off_d;    // a plain world's {0, n}, for the per-world solver
     static constexpr uint32_t PLAIN_WORLD_SOLVER_MAX_BODIES = 1024;
@@ -593,7 +598,8 @@ struct World {
         }
         if (wplan_block == 0) return;
         wcol.reserve(size_t(num_worlds()) * WS_STRIDE + 1);
-        build_world_plan(world_off_h, wplan_block, wplan_tau, wplan, stream);
+        build_world_plan(world_off_h, wplan_block,
+                         wplan_tuned ? wplan_tau : std::max(wplan_tau, UNTUNED_WARP_WORLD_BODIES), wplan, stream);
     }
 
     bool use_world_solver() const { return wplan.valid && (joints_h.empty() || !batch); }
@@ -940,7 +946,8 @@ struct World {
         mark(1);
         // 4: broad phase (syncs once to size the pair arrays; the previous step's
         //    manifold count and timing events are read at the same point).
-        uint64_t np = batch ? bp.run_worlds(aabb_min.p, aabb_max.p, n, world_off_d.p, nw, pairs, status, stream)
+        uint64_t np = batch ? bp.run_worlds(aabb_min.p, aabb_max.p, n, world_off_h, world_off_d.p, world_of_d.p, pairs, status,
+                                            stream)
                             : bp.run(aabb_min.p, aabb_max.p, n, unbounded, pairs, all_pairs, bounds, status, stream);
         npairs = uint32_t(np);
         if (timing) fold(ev_cur ^ 1);
@@ -1171,6 +1178,7 @@ static void autotune_batch(World& W, float dt, uint32_t steps) {
     check_cuda(cudaEventCreate(&e0), "event");
     check_cuda(cudaEventCreate(&e1), "event");
     Cand best{W.wplan_block, W.wplan_tau};
+    W.wplan_tuned = true;
     float best_ms = 0.0f, global_ms = 0.0f;
     uint32_t timed = 0;
     for (const Cand& c : cands) {
@@ -1734,6 +1742,7 @@ bgpu_status bgpu_batch_set_tuning(bgpu_world* w, uint32_t threads_per_cta, uint3
         W.finish_stats();
         W.wplan_block = threads_per_cta;
         W.wplan_tau = warp_world_max_bodies;
+        W.wplan_tuned = true;
         W.rebuild_world_plan();
         return BGPU_OK;
     });
