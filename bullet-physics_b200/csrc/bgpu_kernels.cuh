@@ -462,7 +462,9 @@ struct PairDataDev {
 
 constexpr uint32_t ROUTE_COUNT0 = 16;  // first per-route counter in PairData::scalars
 constexpr uint32_t CAPTURE_COUNT = ROUTE_COUNT0 + NP_MESH + 1;  // detections with points (capture list length)
+constexpr uint32_t EPA_COUNT = CAPTURE_COUNT + 1;               // convex pairs whose cores overlap (EPA list length)
 constexpr uint32_t CAPTURE_LIST = NP_MESH;  // the capture list is route_list region [8 P, 9 P)
+constexpr uint32_t EPA_LIST = NP_MESH + 1;  // and the EPA list [9 P, 10 P)
 
 struct PairData {
     // Per pair (indexed like the sorted pair array).
@@ -535,9 +537,9 @@ struct PairData {
         detect_n.reserve(npairs);
         row_count.reserve(npairs);
         rows.reserve(npairs * 4 * ROW_F4);
-        route_list.reserve(size_t(CAPTURE_LIST + 1) * npairs);
+        route_list.reserve(size_t(EPA_LIST + 1) * npairs);
         old_owned.reserve(old_manifolds + 1);
-        static_assert(CAPTURE_COUNT < 32, "counters");
+        static_assert(EPA_COUNT < 32, "counters");
         reserve_counters();
         contact_pairs.reserve(npairs);
         colour.reserve(npairs);

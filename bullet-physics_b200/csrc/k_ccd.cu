@@ -107,11 +107,6 @@ struct Inflated {
     }
 };
 
-__device__ __forceinline__ bool same_bits(V3 a, V3 b) {
-    return __float_as_uint(a.x) == __float_as_uint(b.x) && __float_as_uint(a.y) == __float_as_uint(b.y) &&
-           __float_as_uint(a.z) == __float_as_uint(b.z);
-}
-
 // Equal walk states between two iterations (at most three points are kept there).
 __device__ __forceinline__ bool same_state(const Simplex& a, V3 av, const Simplex& b, V3 bv) {
     return a.n == b.n && same_bits(av, bv) && same_bits(a.p[0], b.p[0]) && (a.n < 2 || same_bits(a.p[1], b.p[1])) &&

@@ -538,6 +538,39 @@ __device__ __noinline__ void collide_convex(const Shape& sa, V3 pa, Q qa, const 
     mf_push(m, point_a - n * depth, n, depth);
 }
 
+// collide_convex up to the EPA: 2 means that the cores overlap (simplex holds the enclosing
+// tetrahedron), else m is complete.
+__device__ __forceinline__ int collide_convex_gjk(const Shape& sa, V3 pa, Q qa, const Shape& sb, V3 pb, Q qb,
+                                                  bool has_seed, V3 seed, const float4* __restrict__ hull, Manifold& m,
+                                                  V3* simplex) {
+    m.n = 0;
+    ConvexPair cp;
+    cp.sa = &sa; cp.sb = &sb; cp.pa = pa; cp.pb = pb; cp.qa = qa; cp.qb = qb; cp.hull = hull;
+    const GjkResult g = gjk_contact(cp, has_seed, seed, fminf(sa.cbt, sb.cbt));
+    if (g.kind == 1) mf_push(m, g.point_on_b, g.normal, -g.distance);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) simplex[k] = g.simplex[k];
+    return g.kind;
+}
+
+// collide_convex's EPA part by a whole warp (scratch in shared memory, the warp's own).
+__device__ __forceinline__ void collide_convex_epa(const Shape& sa, V3 pa, Q qa, const Shape& sb, V3 pb, Q qb,
+                                                   const float4* __restrict__ hull, const V3* simplex, EpaScratch& scratch,
+                                                   Manifold& m, uint32_t* status) {
+    m.n = 0;
+    ConvexPair cp;
+    cp.sa = &sa; cp.sb = &sb; cp.pa = pa; cp.pb = pb; cp.qa = qa; cp.qb = qb; cp.hull = hull;
+    V3 n;
+    float core_depth;
+    if (epa_penetration_warp(cp, simplex, scratch, n, core_depth) && (threadIdx.x & 31u) == 0u)
+        atomicOr(status, ST_EPA_CAPACITY);
+    __syncwarp();  // the scratch is free again
+    if (core_depth <= 0.0f) return;
+    const float depth = core_depth + sa.margin + sb.margin;
+    const V3 point_a = support_world(sa, pa, qa, n, hull);
+    mf_push(m, point_a - n * depth, n, depth);
+}
+
 // ---------------------------------------------------------------- convex vs static mesh
 // narrowphase/convex_mesh.rs:26-153. The convex's world AABB, swept into the mesh frame, picks
 // candidate triangles from the mesh BVH (bvh.rs:45-66, the same stack walk: left pushed first,
@@ -808,11 +841,17 @@ __global__ __launch_bounds__(NARROW_ANALYTIC_TB) void k_narrow_analytic(BodyDev 
     }
 }
 
-__global__ void k_narrow_convex(BodyDev b, const Shape* __restrict__ shapes, const float4* __restrict__ hull,
-                                const uint64_t* __restrict__ pairs, uint32_t npairs, PairDataDev pd, uint32_t* status) {
+// The GJK part of the convex route, a thread a pair. Pairs whose cores overlap go on to k_narrow_epa
+// with their tetrahedron in the detection's place: as one kernel a few lanes' polytopes (up to 255
+// expansions each, in 12 KB of local memory a thread) held up every warp. The 16,384-body mixed pile
+// (16,000 pairs, 750 of them overlapping): 368 us as one kernel, 76 + 47 us as two. A quarter or an
+// eighth of the lanes a warp is no faster: what is left is one walk's chain of some 16 supports and
+// reductions, not the warps' divergence.
+__global__ void __launch_bounds__(64) k_narrow_convex(BodyDev b, const Shape* __restrict__ shapes,
+                                                      const float4* __restrict__ hull, const uint64_t* __restrict__ pairs,
+                                                      uint32_t npairs, PairDataDev pd) {
     uint32_t cnt = pd.scalars[ROUTE_COUNT0 + NP_CONVEX];
     if (blockIdx.x == 0 && threadIdx.x == 0) pd.scalars[1] = cnt;  // convex detections (step statistics)
-    EpaScratch scratch;
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < cnt; t += gridDim.x * blockDim.x) {
         uint32_t p = pd.route_list[size_t(NP_CONVEX - 1) * npairs + t];
         uint64_t key = pairs[p];
@@ -822,31 +861,199 @@ __global__ void k_narrow_convex(BodyDev b, const Shape* __restrict__ shapes, con
         V3 seed = V3{0.f, 0.f, 0.f};
         bool has_seed = entry_seed(pd.entries + size_t(p) * ENTRY_F4, seed);
         Manifold m;
-        collide_convex(sa, from4(b.pred[i]), q4(b.quat[i]), sb, from4(b.pred[j]), q4(b.quat[j]), has_seed, seed, hull,
-                       scratch, m, status);
-        store_detection(pd, p, npairs, m);
+        V3 simplex[4];
+        if (collide_convex_gjk(sa, from4(b.pred[i]), q4(b.quat[i]), sb, from4(b.pred[j]), q4(b.quat[j]), has_seed, seed,
+                               hull, m, simplex) == 2) {
+            for (int k = 0; k < 4; ++k) pd.detect[size_t(p) * 8 + k] = to4(simplex[k], 0.0f);
+            const uint32_t slot = claim_route_slot(&pd.scalars[EPA_COUNT], 0u);
+            pd.route_list[size_t(EPA_LIST) * npairs + slot] = p;
+        } else {
+            store_detection(pd, p, npairs, m);
+        }
     }
 }
 
-// The mesh route of the pair pass: one warp per pair. Lane 0 walks the mesh BVH and lists the
-// candidate triangles (those whose own box overlaps the query) in walk order; the lanes run the
-// per-triangle detectors side by side; lane 0 then keeps the hits in candidate order and reduces
-// them (the same points, in the same order, as collide_mesh's single pass).
+// The EPA part, a warp a pair. What bounds it: the chain of expansions (a support, the horizon, the new
+// faces: some 1,500 cycles each); two warps a block, for 23 KB of scratch, leave 18 on an SM.
+constexpr int EPA_WARPS = 2;
+
+__global__ void __launch_bounds__(32 * EPA_WARPS) k_narrow_epa(BodyDev b, const Shape* __restrict__ shapes,
+                                                               const float4* __restrict__ hull,
+                                                               const uint64_t* __restrict__ pairs, uint32_t npairs,
+                                                               PairDataDev pd, uint32_t* status) {
+    __shared__ EpaScratch s_epa[EPA_WARPS];
+    const uint32_t cnt = pd.scalars[EPA_COUNT], wi = threadIdx.x >> 5;
+    for (uint32_t t = blockIdx.x * EPA_WARPS + wi; t < cnt; t += gridDim.x * EPA_WARPS) {
+        const uint32_t p = pd.route_list[size_t(EPA_LIST) * npairs + t];
+        const uint64_t key = pairs[p];
+        const uint32_t i = key_lo(key), j = key_hi(key);
+        const Shape sa = shapes[b.info[i].x], sb = shapes[b.info[j].x];
+        V3 simplex[4];
+        for (int k = 0; k < 4; ++k) simplex[k] = from4(pd.detect[size_t(p) * 8 + k]);
+        __syncwarp();  // every lane has the tetrahedron before lane 0 writes the detection over it
+        Manifold m;
+        collide_convex_epa(sa, from4(b.pred[i]), q4(b.quat[i]), sb, from4(b.pred[j]), q4(b.quat[j]), hull, simplex,
+                           s_epa[wi], m, status);
+        if ((threadIdx.x & 31u) == 0u) store_detection(pd, p, npairs, m);
+        __syncwarp();
+    }
+}
+
+// The mesh route of the pair pass, a block a pair. Its first warp walks the mesh BVH and lists the
+// candidate triangles (those whose own box overlaps the query) in walk order; they are dealt to the
+// warps, each of which runs the GJK of its own side by side and gives the triangles whose cores
+// overlap the whole warp's EPA one after the other; thread 0 then keeps the hits in candidate order and
+// reduces them (the same points, in the same order, as collide_mesh's single pass). 500 bodies on the
+// terrain (250 pairs of up to 8 triangles, up to 6 of them overlapping): 140 us with a warp a pair, a
+// lane walking (30,000 cycles, now 7,000) and a thread's EPA in local memory; 56 us so.
 constexpr int MESH_WARPS = 4;
 constexpr int MESH_MAX_TRIS = 128;  // candidate triangles per pair (more: ST_MESH_CANDIDATES)
+constexpr uint32_t MESH_FRONT = 256;  // nodes in one generation of the walk
+static_assert(MESH_MAX_TRIS == 32 * MESH_WARPS, "one candidate a thread");
+
+// convex_mesh.rs:37-60 query box, bvh.rs:45-66 walk, triangle box filter, by one warp: a generation of
+// the walk at a time, each node that the box meets replaced in its place by its children, the second
+// first, which is the order in which a stack would come to them. A lane a node: the walk waits for
+// memory once a generation instead of once a node. Queries that meet more nodes than the lists hold
+// take the stack. Returns the number of candidates (slots in `slot`).
+__device__ __noinline__ uint32_t mesh_candidates(const Shape& cv, V3 pc, Q qc, const Shape& ms, V3 pm, Q qm,
+                                                 const float4* __restrict__ hull, uint32_t (*front)[MESH_FRONT],
+                                                 uint32_t* slot, uint32_t* status) {
+    const uint32_t lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
+    V3 wmn, wmx;
+    world_aabb(cv, pc, qc, hull, wmn, wmx);
+    const Q inv_m = qinv(qm);
+    const V3 c = (wmn + wmx) * 0.5f, e = (wmx - wmn) * 0.5f;
+    V3 lmin = splat(INFINITY), lmax = splat(-INFINITY);
+    for (int k = 0; k < 8; ++k) {
+        const V3 corner = V3{(k & 1) == 0 ? c.x + e.x : c.x - e.x, (k & 2) == 0 ? c.y + e.y : c.y - e.y,
+                             (k & 4) == 0 ? c.z + e.z : c.z - e.z};
+        const V3 q = rotate(inv_m, corner - pm);
+        lmin = vmin(lmin, q);
+        lmax = vmax(lmax, q);
+    }
+    auto overlaps = [&](V3 a0, V3 a1) {
+        return bool((a0.x <= lmax.x) & (a0.y <= lmax.y) & (a0.z <= lmax.z) & (lmin.x <= a1.x) & (lmin.y <= a1.y) &
+                    (lmin.z <= a1.z));
+    };
+    const uint32_t tri_base = mesh_tri_base(ms);
+    uint32_t nc = 0, n = ms.hull_cnt ? 1u : 0u, cur = 0;
+    if (lane == 0) front[0][0] = 0;
+    __syncwarp();
+    // Entries are nodes, or leaves that were met already (MESH_LEAF set: their node without the flag).
+    bool inner = n != 0, over = false;
+    for (int round = 0; inner && !over; ++round) {
+        uint32_t out = 0;
+        inner = false;
+        for (uint32_t f0 = 0; f0 < n; f0 += 32) {
+            const bool in = f0 + lane < n;
+            const uint32_t k = in ? front[cur][f0 + lane] : MESH_LEAF;
+            uint32_t kids = in ? 1u : 0u, a = k, b = 0;
+            if (!(k & MESH_LEAF)) {
+                const float4 n0 = hull[ms.hull_off + 2 * k], n1 = hull[ms.hull_off + 2 * k + 1];
+                const uint32_t na = __float_as_uint(n0.w);
+                kids = 0;
+                if (overlaps(from4(n0), from4(n1))) {
+                    const bool leaf = (na & MESH_LEAF) != 0u;
+                    kids = leaf ? 1u : 2u;
+                    a = leaf ? k | MESH_LEAF : __float_as_uint(n1.w);
+                    b = na;
+                }
+            }
+            const uint32_t one = __ballot_sync(0xffffffffu, kids >= 1u), two = __ballot_sync(0xffffffffu, kids == 2u);
+            const uint32_t at = out + __popc(one & below) + __popc(two & below);
+            out += __popc(one) + __popc(two);
+            inner = inner || two != 0u;
+            over = out > MESH_FRONT || round == MESH_STACK - 2;
+            if (over) break;
+            if (kids >= 1u) front[cur ^ 1u][at] = a;
+            if (kids == 2u) front[cur ^ 1u][at + 1] = b;
+        }
+        __syncwarp();
+        cur ^= 1u;
+        n = out;
+    }
+    if (!over) {
+        for (uint32_t f0 = 0; f0 < n; f0 += 32) {
+            uint32_t start = 0, hit = 0;  // a leaf's triangles, four at most
+            if (f0 + lane < n) {
+                const uint32_t k = front[cur][f0 + lane] & ~MESH_LEAF;
+                start = __float_as_uint(hull[ms.hull_off + 2 * k].w) & ~MESH_LEAF;
+                const uint32_t nb = __float_as_uint(hull[ms.hull_off + 2 * k + 1].w);
+                for (uint32_t q = 0; q < nb; ++q) {
+                    const uint32_t o = tri_base + 3 * (start + q);
+                    const V3 ta = from4(hull[o]), tb = from4(hull[o + 1]), tc = from4(hull[o + 2]);
+                    hit |= uint32_t(overlaps(vmin(ta, vmin(tb, tc)), vmax(ta, vmax(tb, tc)))) << q;
+                }
+            }
+            const uint32_t cnt = __popc(hit);
+            uint32_t at = cnt;
+#pragma unroll
+            for (uint32_t d = 1; d < 32; d <<= 1) {
+                const uint32_t v = __shfl_up_sync(0xffffffffu, at, d);
+                if (lane >= d) at += v;
+            }
+            const uint32_t total = __shfl_sync(0xffffffffu, at, 31);
+            at += nc - cnt;
+            for (; hit; hit &= hit - 1u, ++at) {
+                if (at < MESH_MAX_TRIS) slot[at] = start + __ffs(int(hit)) - 1;
+                else atomicOr(status, ST_MESH_CANDIDATES);
+            }
+            nc = min(nc + total, uint32_t(MESH_MAX_TRIS));
+        }
+        return nc;
+    }
+    if (lane == 0) {
+        uint32_t stack[MESH_STACK];
+        int sp = 0;
+        stack[sp++] = 0;
+        while (sp > 0) {
+            const uint32_t k = stack[--sp];
+            const float4 n0 = hull[ms.hull_off + 2 * k], n1 = hull[ms.hull_off + 2 * k + 1];
+            if (!overlaps(from4(n0), from4(n1))) continue;
+            const uint32_t na = __float_as_uint(n0.w), nb = __float_as_uint(n1.w);
+            if (!(na & MESH_LEAF)) {
+                if (sp + 2 > MESH_STACK) {
+                    atomicOr(status, ST_TRAVERSAL_STACK);
+                    continue;
+                }
+                stack[sp++] = na;
+                stack[sp++] = nb;
+                continue;
+            }
+            const uint32_t start = na & ~MESH_LEAF;
+            for (uint32_t s = start; s < start + nb; ++s) {
+                const uint32_t o = tri_base + 3 * s;
+                const V3 ta = from4(hull[o]), tb = from4(hull[o + 1]), tc = from4(hull[o + 2]);
+                if (!overlaps(vmin(ta, vmin(tb, tc)), vmax(ta, vmax(tb, tc)))) continue;
+                if (nc == MESH_MAX_TRIS) {
+                    atomicOr(status, ST_MESH_CANDIDATES);
+                    continue;
+                }
+                slot[nc++] = s;
+            }
+        }
+    }
+    return __shfl_sync(0xffffffffu, nc, 0);
+}
 
 __global__ void __launch_bounds__(32 * MESH_WARPS) k_narrow_mesh(BodyDev b, const Shape* __restrict__ shapes,
                                                                  const float4* __restrict__ hull,
                                                                  const uint64_t* __restrict__ pairs, uint32_t npairs,
                                                                  PairDataDev pd, uint32_t* status) {
-    __shared__ uint32_t s_slot[MESH_WARPS][MESH_MAX_TRIS];
-    __shared__ float4 s_pt[MESH_WARPS][MESH_MAX_TRIS], s_nr[MESH_WARPS][MESH_MAX_TRIS];
-    __shared__ uint32_t s_n[MESH_WARPS];
+    __shared__ uint32_t s_slot[MESH_MAX_TRIS];
+    __shared__ uint32_t s_n;
+    __shared__ __align__(16) EpaScratch s_epa[MESH_WARPS];
+    // The walk's lists and the candidates' results lie in the scratch, before and after its use.
+    uint32_t(*s_front)[MESH_FRONT] = reinterpret_cast<uint32_t(*)[MESH_FRONT]>(&s_epa[0]);
+    float4* s_pt = reinterpret_cast<float4*>(&s_epa[1]);
+    float4* s_nr = s_pt + MESH_MAX_TRIS;
+    static_assert(sizeof(EpaScratch) % 16 == 0 && sizeof(EpaScratch) >= 2 * MESH_MAX_TRIS * sizeof(float4) &&
+                      sizeof(EpaScratch) >= 2 * MESH_FRONT * sizeof(uint32_t), "lists in the scratch");
     const uint32_t cnt = pd.scalars[ROUTE_COUNT0 + NP_MESH];
     if (blockIdx.x == 0 && threadIdx.x == 0) pd.scalars[1] += cnt;  // with the convex detections (statistics)
     const uint32_t wi = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    EpaScratch scratch;
-    for (uint32_t t = blockIdx.x * MESH_WARPS + wi; t < cnt; t += gridDim.x * MESH_WARPS) {
+    for (uint32_t t = blockIdx.x; t < cnt; t += gridDim.x) {
         const uint32_t p = pd.route_list[size_t(NP_MESH - 1) * npairs + t];
         const uint64_t key = pairs[p];
         const uint32_t i = key_lo(key), j = key_hi(key);
@@ -861,104 +1068,88 @@ __global__ void __launch_bounds__(32 * MESH_WARPS) k_narrow_mesh(BodyDev b, cons
         const bool has_seed = entry_seed(pd.entries + size_t(p) * ENTRY_F4, seed);
         const float thr = fminf(cv.cbt, ms.cbt);
         const uint32_t tri_base = mesh_tri_base(ms);
-        if (lane == 0) {  // convex_mesh.rs:37-60 query box, bvh.rs:45-66 walk, triangle box filter
-            V3 wmn, wmx;
-            world_aabb(cv, pc, qc, hull, wmn, wmx);
-            const Q inv_m = qinv(qm);
-            const V3 c = (wmn + wmx) * 0.5f, e = (wmx - wmn) * 0.5f;
-            V3 lmin = splat(INFINITY), lmax = splat(-INFINITY);
-            for (int k = 0; k < 8; ++k) {
-                const V3 corner = V3{(k & 1) == 0 ? c.x + e.x : c.x - e.x, (k & 2) == 0 ? c.y + e.y : c.y - e.y,
-                                     (k & 4) == 0 ? c.z + e.z : c.z - e.z};
-                const V3 q = rotate(inv_m, corner - pm);
-                lmin = vmin(lmin, q);
-                lmax = vmax(lmax, q);
-            }
-            auto overlaps = [&](V3 a0, V3 a1) {
-                return a0.x <= lmax.x && a0.y <= lmax.y && a0.z <= lmax.z && lmin.x <= a1.x && lmin.y <= a1.y &&
-                       lmin.z <= a1.z;
-            };
-            uint32_t nc = 0;
-            uint32_t stack[MESH_STACK];
-            int sp = 0;
-            if (ms.hull_cnt) stack[sp++] = 0;
-            while (sp > 0) {
-                const uint32_t k = stack[--sp];
-                const float4 n0 = hull[ms.hull_off + 2 * k], n1 = hull[ms.hull_off + 2 * k + 1];
-                if (!overlaps(from4(n0), from4(n1))) continue;
-                const uint32_t na = __float_as_uint(n0.w), nb = __float_as_uint(n1.w);
-                if (!(na & MESH_LEAF)) {
-                    if (sp + 2 > MESH_STACK) {
-                        atomicOr(status, ST_TRAVERSAL_STACK);
-                        continue;
-                    }
-                    stack[sp++] = na;
-                    stack[sp++] = nb;
-                    continue;
-                }
-                const uint32_t start = na & ~MESH_LEAF;
-                for (uint32_t slot = start; slot < start + nb; ++slot) {
-                    const uint32_t o = tri_base + 3 * slot;
-                    const V3 ta = from4(hull[o]), tb = from4(hull[o + 1]), tc = from4(hull[o + 2]);
-                    if (!overlaps(vmin(ta, vmin(tb, tc)), vmax(ta, vmax(tb, tc)))) continue;
-                    if (nc == MESH_MAX_TRIS) {
-                        atomicOr(status, ST_MESH_CANDIDATES);
-                        continue;
-                    }
-                    s_slot[wi][nc++] = slot;
-                }
-            }
-            s_n[wi] = nc;
+        __syncthreads();  // the lists of the block's last pair have been read
+        if (wi == 0) {
+            const uint32_t n = mesh_candidates(cv, pc, qc, ms, pm, qm, hull, s_front, s_slot, status);
+            if (lane == 0) s_n = n;
         }
-        __syncwarp();
-        const uint32_t nc = s_n[wi];
+        __syncthreads();
+        const uint32_t nc = s_n;
+        if (nc == 0) {
+            if (threadIdx.x == 0) {
+                Manifold m;
+                m.n = 0;
+                store_detection(pd, p, npairs, m);
+            }
+            continue;
+        }
         const bool sphere = cv.type == SHAPE_SPHERE;
-        const V3 center = rotate(qinv(qm), pc - pm);
         Shape tri;
         tri.type = SHAPE_HULL;
         tri.hull_cnt = 3;
         tri.margin = 0.0f;
         tri.cbt = thr;
-        for (uint32_t k = lane; k < nc; k += 32) {
-            const uint32_t o = tri_base + 3 * s_slot[wi][k];
-            V3 pt = V3{0.f, 0.f, 0.f}, nl = V3{0.f, 0.f, 0.f};
-            float pen = 0.0f;
-            bool hit = false;
-            if (sphere) {
-                if (sphere_triangle(center, cv.p0, thr, from4(hull[o]), from4(hull[o + 1]), from4(hull[o + 2]), pt, nl,
-                                    pen)) {
-                    pt = pm + rotate(qm, pt);
-                    nl = rotate(qm, -nl);
-                    hit = true;
-                }
-            } else {
-                tri.hull_off = o;
-                Manifold one;
-                collide_convex(cv, pc, qc, tri, pm, qm, has_seed, seed, hull, scratch, one, status);
-                if (one.n) {
-                    pt = one.pos[0];
-                    nl = one.nrm[0];
-                    pen = one.pen[0];
-                    hit = true;
-                }
+        const uint32_t k = lane * MESH_WARPS + wi, o = k < nc ? tri_base + 3 * s_slot[k] : tri_base;
+        V3 pt = V3{0.f, 0.f, 0.f}, nl = V3{0.f, 0.f, 0.f};
+        float pen = 0.0f;
+        bool hit = false, deep = false;
+        V3 simplex[4] = {};
+        if (k < nc && sphere) {
+            const V3 center = rotate(qinv(qm), pc - pm);
+            if (sphere_triangle(center, cv.p0, thr, from4(hull[o]), from4(hull[o + 1]), from4(hull[o + 2]), pt, nl,
+                                pen)) {
+                pt = pm + rotate(qm, pt);
+                nl = rotate(qm, -nl);
+                hit = true;
             }
-            s_pt[wi][k] = to4(pt, pen);
-            s_nr[wi][k] = to4(nl, hit ? 1.0f : 0.0f);
+        } else if (k < nc) {
+            tri.hull_off = o;
+            Manifold one;
+            deep = collide_convex_gjk(cv, pc, qc, tri, pm, qm, has_seed, seed, hull, one, simplex) == 2;
+            if (one.n) {
+                pt = one.pos[0];
+                nl = one.nrm[0];
+                pen = one.pen[0];
+                hit = true;
+            }
         }
         __syncwarp();
-        if (lane == 0) {
+        for (uint32_t todo = __ballot_sync(0xffffffffu, deep); todo; todo &= todo - 1u) {
+            const int src = __ffs(int(todo)) - 1;
+            V3 sx[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                sx[q] = V3{__shfl_sync(0xffffffffu, simplex[q].x, src), __shfl_sync(0xffffffffu, simplex[q].y, src),
+                           __shfl_sync(0xffffffffu, simplex[q].z, src)};
+            tri.hull_off = __shfl_sync(0xffffffffu, o, src);
+            Manifold one;
+            collide_convex_epa(cv, pc, qc, tri, pm, qm, hull, sx, s_epa[wi], one, status);
+            if (int(lane) == src && one.n) {
+                pt = one.pos[0];
+                nl = one.nrm[0];
+                pen = one.pen[0];
+                hit = true;
+            }
+        }
+        __syncthreads();  // the scratch is free
+        if (k < nc) {
+            s_pt[k] = to4(pt, pen);
+            s_nr[k] = to4(nl, hit ? 1.0f : 0.0f);
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
             MeshCandidates cand;
             cand.n = 0;
-            for (uint32_t k = 0; k < nc; ++k) {
-                const float4 nr = s_nr[wi][k];
+            for (uint32_t q = 0; q < nc; ++q) {
+                const float4 nr = s_nr[q];
                 if (nr.w == 0.0f) continue;
                 if (cand.n == MESH_MAX_CAND) {
                     atomicOr(status, ST_MESH_CANDIDATES);
                     break;
                 }
-                const float4 pt = s_pt[wi][k];
-                cand.pos[cand.n] = from4(pt);
-                cand.pen[cand.n] = pt.w;
+                const float4 pq = s_pt[q];
+                cand.pos[cand.n] = from4(pq);
+                cand.pen[cand.n] = pq.w;
                 cand.nrm[cand.n] = from4(nr);
                 ++cand.n;
             }
@@ -967,7 +1158,6 @@ __global__ void __launch_bounds__(32 * MESH_WARPS) k_narrow_mesh(BodyDev b, cons
             if (mesh_a) mf_flip(m);
             store_detection(pd, p, npairs, m);
         }
-        __syncwarp();  // the warp's shared lists are reused by its next pair
     }
 }
 
@@ -1098,14 +1288,14 @@ void run_pair_pass(const WorldView& w, const uint64_t* pairs, uint32_t npairs, c
     k_narrow_analytic<<<grid, NARROW_ANALYTIC_TB, 0, s>>>(w.b, w.shapes, w.hull, pairs, npairs, d);
     if (w.has_convex) {
         uint32_t cgrid = std::min<uint32_t>((npairs + 63) / 64, 148u * 8u);
-        k_narrow_convex<<<cgrid, 64, 0, s>>>(w.b, w.shapes, w.hull, pairs, npairs, d, status_dev);
+        k_narrow_convex<<<cgrid, 64, 0, s>>>(w.b, w.shapes, w.hull, pairs, npairs, d);
+        k_narrow_epa<<<std::min<uint32_t>((npairs + EPA_WARPS - 1) / EPA_WARPS, 148u * 8u), 32 * EPA_WARPS, 0, s>>>(
+            w.b, w.shapes, w.hull, pairs, npairs, d, status_dev);
     }
     if (w.has_mesh) {
-        const uint32_t mgrid = std::min<uint32_t>((npairs + MESH_WARPS - 1) / MESH_WARPS, 148u * 8u);
+        const uint32_t mgrid = std::min<uint32_t>(npairs, 148u * 16u);
         k_narrow_mesh<<<mgrid, 32 * MESH_WARPS, 0, s>>>(w.b, w.shapes, w.hull, pairs, npairs, d, status_dev);
     }
-    // The GJK/EPA kernels keep their polytopes in local memory (12-15 KB a thread): a launch
-    // the device cannot back with local memory fails here rather than dropping detections.
     check_cuda(cudaGetLastError(), "narrow phase launch");
     k_capture<<<(npairs + CAPTURE_TB - 1) / CAPTURE_TB < 148u * 16u ? (npairs + CAPTURE_TB - 1) / CAPTURE_TB : 148u * 16u,
                 CAPTURE_TB, 0, s>>>(w.b, w.shapes, pairs, npairs, sp, d);

@@ -1,0 +1,83 @@
+"""The convex and mesh routes of a step (GJK by the thread, EPA by the warp) against the oracle, in
+lockstep: one pair, around a warp's and a block's share of the EPA list, hulls below and above a
+warp's 32 points, and terrain queries of a few triangles, of a few dozen (several leaves a lane of
+the walk) and of more than the lists hold, which the step reports by its status.
+
+Tolerances are those of a single step (test_gpu_lockstep.py): pairs bit for bit, state 1e-5.
+"""
+import numpy as np
+import pytest
+
+import oracle_api as orc
+from test_gpu_lockstep import lockstep
+
+pytestmark = pytest.mark.gpu
+
+
+def _hull(rng, n, r):
+    p = rng.normal(size=(n, 3))
+    return (r * p / np.linalg.norm(p, axis=1, keepdims=True)).astype(np.float32)
+
+
+def _quat(rng):
+    q = rng.normal(size=4)
+    return tuple(q / np.linalg.norm(q))
+
+
+def _both(gpu):
+    return gpu.World(), orc.OracleWorld("f32")
+
+
+@pytest.mark.parametrize("pairs,points", [(1, 24), (2, 8), (3, 33), (31, 24), (65, 40)])
+def test_overlapping_hulls(gpu, pairs, points):
+    rng = np.random.default_rng(100 * pairs + points)
+    w, o = _both(gpu)
+    pts = _hull(rng, points, 0.5)
+    kinds = []
+    for x in (w, o):
+        kinds.append([x.hull(pts), x.box([0.4, 0.3, 0.35]), x.capsule(0.25, 0.3)])
+    assert kinds[0] == kinds[1]
+    for k in range(pairs):
+        base = np.array([3.0 * (k % 8), 3.0 * (k // 8), 0.0])
+        off = _hull(rng, 1, 0.55)[0]
+        qa, qb = _quat(rng), _quat(rng)
+        for x in (w, o):
+            x.add_body(kinds[0][0], tuple(base), qa, mass=1.0)
+            x.add_body(kinds[0][k % 3], tuple(base + off), qb, mass=1.0)
+    lockstep(w, o, 1.0 / 60.0, 4, f"{pairs} hulls")
+    assert len(w.pairs()) == pairs
+
+
+@pytest.mark.parametrize("count,half", [(1, 0.1), (5, 0.3), (40, 0.45)])
+def test_bodies_in_terrain(gpu, count, half):
+    import scenes
+
+    rng = np.random.default_rng(count)
+    w, o = _both(gpu)
+    v, idx = scenes.wavy_grid_mesh(60, 60, (-6.0, -6.0), (0.2, 0.2), 0.3, 0.4, 0.3)
+    pts = _hull(rng, 40, half)
+    for x in (w, o):
+        assert x.mesh(v, idx) == 0
+        assert [x.box([half, 0.1, half]), x.hull(pts), x.capsule(half, 0.1)] == [1, 2, 3]
+        x.add_body(0, (0.0, 0.0, 0.0), mass=0.0)
+    cells = rng.permutation(100)[:count]
+    for k, c in enumerate(cells):
+        p = (-5.0 + 1.05 * (c % 10), 0.2, -5.0 + 1.05 * (c // 10))
+        q = _quat(rng)
+        for x in (w, o):
+            x.add_body(1 + k % 3, p, q, mass=1.0)
+    lockstep(w, o, 1.0 / 60.0, 4, f"{count} on terrain")
+
+
+def test_terrain_query_beyond_the_lists(gpu):
+    import scenes
+
+    w = gpu.World()
+    v, idx = scenes.wavy_grid_mesh(60, 60, (-6.0, -6.0), (0.2, 0.2), 0.01, 0.4, 0.3)
+    w.mesh(v, idx)
+    w.box([4.0, 0.1, 4.0])
+    w.add_body(0, (0.0, 0.0, 0.0), mass=0.0)
+    w.add_body(1, (0.0, 0.05, 0.0), mass=1.0)
+    with pytest.raises(gpu.BgpuError, match="device status bits 0x100"):  # more candidates than a pair keeps
+        w.step(1.0 / 60.0)
+    assert np.isfinite(w.state()).all()
