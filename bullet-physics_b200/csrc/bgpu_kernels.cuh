@@ -251,6 +251,8 @@ void launch_ccd_sweep(const BodyDev& b, const Shape* shapes, const float4* hull,
 void launch_ccd_apply(const BodyDev& b, const uint32_t* ids, const float* clamp, uint32_t m, float dt, cudaStream_t s);
 // Host-facing layouts: n x 3 floats -> float4 lanes, and poses -> n x 7 floats.
 void launch_unpack3(uint32_t n, const float* src, float4* dst, cudaStream_t s);
+// pos/quat/velocities/activation/timer -> n x 15 floats, the layout of bgpu_read_state.
+void launch_pack_state(uint32_t n, const BodyDev& b, float* out, cudaStream_t s);
 void launch_pack_poses(uint32_t n, const float4* pos, const float4* quat, float* out, cudaStream_t s);
 
 // ---------------------------------------------------------------- broad phase (k_broadphase.cu)

@@ -284,6 +284,19 @@ __global__ void k_unpack3(uint32_t n, const float* __restrict__ src, float4* dst
     dst[i] = make_float4(src[3 * i], src[3 * i + 1], src[3 * i + 2], 0.0f);
 }
 
+// The caller's state layout. Bound by the copy to the host that follows: one, where each array's own copy
+// took some 8 us of the host's time however few bodies (one body's state: 66 us, now 22 us).
+__global__ void k_pack_state(uint32_t n, BodyDev b, float* out) {
+    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const float4 p = b.pos[i], q = b.quat[i], l = b.linvel[i], a = b.angvel[i];
+    float* o = out + size_t(i) * 15;
+    o[0] = p.x; o[1] = p.y; o[2] = p.z; o[3] = q.x; o[4] = q.y; o[5] = q.z; o[6] = q.w;
+    o[7] = l.x; o[8] = l.y; o[9] = l.z; o[10] = a.x; o[11] = a.y; o[12] = a.z;
+    o[13] = float(b.info[i].z);
+    o[14] = b.sleep[i].x;
+}
+
 // position + orientation -> n x 7 floats (x y z qx qy qz qw).
 __global__ void k_pack_poses(uint32_t n, const float4* __restrict__ pos, const float4* __restrict__ quat, float* out) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -297,6 +310,10 @@ __global__ void k_pack_poses(uint32_t n, const float4* __restrict__ pos, const f
 
 void launch_unpack3(uint32_t n, const float* src, float4* dst, cudaStream_t s) {
     if (n) k_unpack3<<<(n + 255) / 256, 256, 0, s>>>(n, src, dst);
+}
+
+void launch_pack_state(uint32_t n, const BodyDev& b, float* out, cudaStream_t s) {
+    if (n) k_pack_state<<<(n + 255) / 256, 256, 0, s>>>(n, b, out);
 }
 
 void launch_pack_poses(uint32_t n, const float4* pos, const float4* quat, float* out, cudaStream_t s) {

@@ -1876,25 +1876,13 @@ bgpu_status bgpu_read_state(bgpu_world* w, float* state) {
     return guarded([&]() -> bgpu_status {
         World& W = w->impl;
         uint32_t n = W.n;
-        std::vector<float4> p(n), q(n), lv(n), av(n), sl(n);
-        std::vector<uint4> in(n);
+        if (!n) return BGPU_OK;
         cudaStream_t s = W.stream;
-        bgpu::check_cuda(cudaMemcpyAsync(p.data(), W.pos.p, n * sizeof(float4), cudaMemcpyDeviceToHost, s), "d2h");
-        bgpu::check_cuda(cudaMemcpyAsync(q.data(), W.quat.p, n * sizeof(float4), cudaMemcpyDeviceToHost, s), "d2h");
-        bgpu::check_cuda(cudaMemcpyAsync(lv.data(), W.linvel.p, n * sizeof(float4), cudaMemcpyDeviceToHost, s), "d2h");
-        bgpu::check_cuda(cudaMemcpyAsync(av.data(), W.angvel.p, n * sizeof(float4), cudaMemcpyDeviceToHost, s), "d2h");
-        bgpu::check_cuda(cudaMemcpyAsync(sl.data(), W.sleep.p, n * sizeof(float4), cudaMemcpyDeviceToHost, s), "d2h");
-        bgpu::check_cuda(cudaMemcpyAsync(in.data(), W.info_d.p, n * sizeof(uint4), cudaMemcpyDeviceToHost, s), "d2h");
+        W.host_io.reserve(size_t(n) * 15);
+        bgpu::launch_pack_state(n, W.body_dev(), W.host_io.p, s);
+        bgpu::check_cuda(cudaMemcpyAsync(state, W.host_io.p, size_t(n) * 15 * sizeof(float), cudaMemcpyDeviceToHost, s),
+                         "d2h");
         bgpu::check_cuda(cudaStreamSynchronize(s), "sync");
-        for (uint32_t i = 0; i < n; ++i) {
-            float* o = state + size_t(i) * 15;
-            o[0] = p[i].x; o[1] = p[i].y; o[2] = p[i].z;
-            o[3] = q[i].x; o[4] = q[i].y; o[5] = q[i].z; o[6] = q[i].w;
-            o[7] = lv[i].x; o[8] = lv[i].y; o[9] = lv[i].z;
-            o[10] = av[i].x; o[11] = av[i].y; o[12] = av[i].z;
-            o[13] = float(in[i].z);
-            o[14] = sl[i].x;
-        }
         return BGPU_OK;
     });
 }

@@ -77,3 +77,23 @@ def test_a_sleeping_world_keeps_manifolds_of_vanished_pairs():
         assert np.abs(st[:, :13] - r[:, :13]).max() < 2e-3, step
         o.set_state(st)
     assert (g.state()[1:, 13] != 2).any()
+
+
+@pytest.mark.parametrize("n", [1, 255, 256, 257, 1025])
+def test_state_is_every_column_of_every_body(gpu, n):
+    """A written state reads back whole: poses, velocities, activation and deactivation timer, around
+    a block of the packing kernel; and again after a second, larger world state has used the staging."""
+    rng = np.random.default_rng(n)
+    w = gpu.World()
+    w.box([0.1, 0.1, 0.1])
+    for k in range(n):
+        w.add_body(0, (1.0 * k, 0.0, 0.0), mass=1.0)
+    s = rng.normal(size=(n, 15)).astype(np.float32)
+    s[:, 3:7] /= np.linalg.norm(s[:, 3:7], axis=1, keepdims=True)
+    s[:, 13] = rng.integers(1, 6, size=n)
+    s[:, 14] = rng.random(n)
+    w.set_state(s)
+    np.testing.assert_array_equal(w.state(), s)
+    np.testing.assert_array_equal(w.poses(), s[:, :7])
+    w.apply_forces(np.ones((n, 3), np.float32), np.ones((n, 3), np.float32))
+    np.testing.assert_array_equal(w.state(), s)
