@@ -97,3 +97,29 @@ def test_state_is_every_column_of_every_body(gpu, n):
     np.testing.assert_array_equal(w.poses(), s[:, :7])
     w.apply_forces(np.ones((n, 3), np.float32), np.ones((n, 3), np.float32))
     np.testing.assert_array_equal(w.state(), s)
+
+
+@pytest.mark.parametrize("n,leave", [(3, 1), (127, 64), (129, 128), (520, 400), (1300, 3), (1300, 700)])
+def test_old_manifolds_are_found(gpu, n, leave):
+    """Boxes on one static box settle, then all but a few leave at once: the pairs of a block look for
+    their manifolds among few old keys, among more than a block stages, and where none is left. In
+    lockstep with the oracle, whose impulses start from the same manifolds."""
+    import oracle_api as orc
+    from test_gpu_lockstep import lockstep
+
+    side = int(np.ceil(np.sqrt(n)))
+    w, o = gpu.World(), orc.OracleWorld("f32")
+    for x in (w, o):
+        assert [x.box([1.5 * side, 0.5, 1.5 * side]), x.box([0.5, 0.5, 0.5])] == [0, 1]
+        x.add_body(0, (0.0, -0.5, 0.0), mass=0.0)
+        for k in range(n):
+            x.add_body(1, (1.25 * (k % side - side / 2), 0.499, 1.25 * (k // side - side / 2)), mass=1.0)
+    lockstep(w, o, 1.0 / 60.0, 3, "settle")
+    s = w.state()
+    stay = np.zeros(n + 1, bool)
+    stay[0] = True
+    stay[1 + np.linspace(0, n - 1, leave).astype(int)] = True
+    s[~stay, 1] += 50.0
+    w.set_state(s)
+    lockstep(w, o, 1.0 / 60.0, 2, "after")
+    assert len(w.pairs()) == leave
