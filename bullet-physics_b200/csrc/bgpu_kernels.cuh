@@ -265,7 +265,6 @@ struct Broadphase {
     DevBuf<uint32_t> stash, overflow;  // partners of proxies with few of them; proxies with many
     DevBuf<uint32_t> unb_tiles;        // per unbounded proxy and tile of proxies: partners before the tile
     DevBuf<float4> node_min, node_max;
-    DevBuf<uint32_t> node_maxid;       // largest body index below each node
     DevBuf<float4> node_rec;           // per internal node: both children's boxes and references
     DevBuf<uint32_t> masks;            // all-pairs pass: bit j of row i
     DevBuf<unsigned char> cub_tmp;

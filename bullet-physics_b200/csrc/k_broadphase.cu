@@ -111,7 +111,6 @@ __global__ void k_build(LeafKeys k, int m, uint32_t* left, uint32_t* right, uint
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < m) leaf_body[i] = k.index[i];
     if (i >= m - 1) return;
-    refit_flag[i] = 0;
     int d = (delta(k, m, i, i + 1) - delta(k, m, i, i - 1)) >= 0 ? 1 : -1;
     int dmin = delta(k, m, i, i - d);
     int lmax = 2;
@@ -133,6 +132,7 @@ __global__ void k_build(LeafKeys k, int m, uint32_t* left, uint32_t* right, uint
     uint32_t rc = (hi == gamma + 1) ? uint32_t(m - 1 + gamma + 1) : uint32_t(gamma + 1);
     left[i] = lc;
     right[i] = rc;
+    refit_flag[i] = uint32_t(j) << 2;  // the other end of the node's leaves; low bits: children that arrived
     parent[lc] = uint32_t(i);
     parent[rc] = uint32_t(i);
 }
@@ -144,39 +144,97 @@ constexpr uint32_t LEAF_REF = 0x80000000u;
 // node's record (4 float4: left child min | ref, left max | ref of right, right min | largest
 // body index under left, right max | largest under right) is written by the thread that
 // completes it, so a query reads one 64-byte record per node it visits.
-__global__ void k_refit(int m, const uint32_t* __restrict__ leaf_body, const uint32_t* __restrict__ parent,
-                        const uint32_t* __restrict__ left, const uint32_t* __restrict__ right, uint32_t* refit_flag,
-                        const float4* __restrict__ bmin, const float4* __restrict__ bmax, float4* nmin, float4* nmax,
-                        uint32_t* nid, float4* rec) {
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= m) return;
-    uint32_t node = uint32_t(m - 1 + t);
-    uint32_t body = leaf_body[t];
-    nmin[node] = bmin[body];
-    nmax[node] = bmax[body];
-    nid[node] = body;
-    if (m == 1) return;
-    __threadfence();
-    uint32_t cur = parent[node];
+// What bounds it: the climb, a fence, an atomic and two dependent loads a level. A node's number is one end of
+// its leaves, so a node whose other end is in the same block of leaves has its whole subtree there: such
+// nodes meet in shared memory, and only the climb from the blocks to the root goes through L2.
+// There the records are written after the atomic, which has only the boxes to wait for, and the children's
+// numbers are loaded with it. 16,384 / 60,000 / 131,072 leaves: 47 / 44 / 54 us with every node in L2,
+// 37 / 38 / 47 us with blocks of 512 (256: 37 / 40 / 48, 128: 38 / 41 / 48), 30 / 31 / 38 us so.
+constexpr int REFIT_TB = 512;
+
+__global__ void __launch_bounds__(REFIT_TB) k_refit(int m, const uint32_t* __restrict__ leaf_body,
+                                                    const uint32_t* __restrict__ parent, const uint32_t* __restrict__ left,
+                                                    const uint32_t* __restrict__ right, uint32_t* refit_flag,
+                                                    const float4* __restrict__ bmin, const float4* __restrict__ bmax,
+                                                    float4* nmin, float4* nmax, float4* rec) {
+    // The block's leaves, then its nodes; w of a minimum: the largest body index.
+    __shared__ float4 s_min[2 * REFIT_TB], s_max[2 * REFIT_TB];
+    __shared__ uint32_t s_left[REFIT_TB], s_right[REFIT_TB], s_parent[REFIT_TB], s_count[REFIT_TB];
+    constexpr uint32_t ELSEWHERE = 1u << 31;  // in s_count: a node that other blocks' leaves belong to
+    const uint32_t base = blockIdx.x * REFIT_TB, x = threadIdx.x, t = base + x, leaf0 = uint32_t(m - 1);
+    uint32_t cur = 0, me = leaf0 + t;
+    float4 lo{}, hi{};
+    if (t < leaf0) {
+        s_left[x] = left[t];
+        s_right[x] = right[t];
+        s_parent[x] = t ? parent[t] : 0u;
+        s_count[x] = (refit_flag[t] >> 2) / REFIT_TB == blockIdx.x ? 0u : ELSEWHERE;
+    }
+    if (t < uint32_t(m)) {
+        const uint32_t body = leaf_body[t];
+        lo = bmin[body];
+        hi = bmax[body];
+        lo.w = __uint_as_float(body);
+        s_min[x] = lo;
+        s_max[x] = hi;
+        if (m > 1) cur = parent[me];
+    }
+    __syncthreads();
+    if (t >= uint32_t(m) || m == 1) return;
+    constexpr uint32_t NONE = 0xffffffffu;
+    uint32_t rec_of = NONE;  // a node whose record (q0 .. q3) is not written yet
+    float4 q0{}, q1{}, q2{}, q3{};
+    auto slot = [&](uint32_t node) { return node >= leaf0 ? node - leaf0 - base : REFIT_TB + node - base; };
     for (int guard = 0; guard < 128; ++guard) {
-        if (atomicAdd(&refit_flag[cur], 1u) == 0) return;  // first child to arrive stops
-        __threadfence();
-        uint32_t l = left[cur], r = right[cur];
-        float4 a0 = __ldcg(&nmin[l]), a1 = __ldcg(&nmax[l]), b0 = __ldcg(&nmin[r]), b1 = __ldcg(&nmax[r]);
-        const uint32_t il = __ldcg(&nid[l]), ir = __ldcg(&nid[r]);
-        nmin[cur] = make_float4(fminf(a0.x, b0.x), fminf(a0.y, b0.y), fminf(a0.z, b0.z), 0.f);
-        nmax[cur] = make_float4(fmaxf(a1.x, b1.x), fmaxf(a1.y, b1.y), fmaxf(a1.z, b1.z), 0.f);
-        nid[cur] = il > ir ? il : ir;
-        const uint32_t lref = l >= uint32_t(m - 1) ? (LEAF_REF | il) : l;
-        const uint32_t rref = r >= uint32_t(m - 1) ? (LEAF_REF | ir) : r;
-        float4* rc = rec + size_t(cur) * 4;
-        rc[0] = make_float4(a0.x, a0.y, a0.z, __uint_as_float(lref));
-        rc[1] = make_float4(a1.x, a1.y, a1.z, __uint_as_float(rref));
-        rc[2] = make_float4(b0.x, b0.y, b0.z, __uint_as_float(il));
-        rc[3] = make_float4(b1.x, b1.y, b1.z, __uint_as_float(ir));
-        __threadfence();
+        const bool here = cur - base < uint32_t(REFIT_TB) && !(s_count[cur - base] & ELSEWHERE);
+        uint32_t l, r, up;
+        float4 a0, a1, b0, b1;
+        if (here) {
+            __threadfence_block();
+            if (atomicAdd(&s_count[cur - base], 1u) == 0u) return;  // first child to arrive stops
+            __threadfence_block();
+            l = s_left[cur - base];
+            r = s_right[cur - base];
+            up = s_parent[cur - base];
+            a0 = s_min[slot(l)]; a1 = s_max[slot(l)]; b0 = s_min[slot(r)]; b1 = s_max[slot(r)];
+        } else {
+            nmin[me] = lo;
+            nmax[me] = hi;
+            l = left[cur];  // on their way with the atomic
+            r = right[cur];
+            up = parent[cur];
+            uint32_t arrived;
+            asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(arrived) : "l"(refit_flag + cur) : "memory");
+            if (rec_of != NONE) {  // the last node's record: nobody waits for it
+                float4* rc = rec + size_t(rec_of) * 4;
+                rc[0] = q0; rc[1] = q1; rc[2] = q2; rc[3] = q3;
+                rec_of = NONE;
+            }
+            if ((arrived & 3u) == 0u) return;
+            a0 = __ldcg(&nmin[l]); a1 = __ldcg(&nmax[l]); b0 = __ldcg(&nmin[r]); b1 = __ldcg(&nmax[r]);
+        }
+        const uint32_t il = __float_as_uint(a0.w), ir = __float_as_uint(b0.w);
+        lo = make_float4(fminf(a0.x, b0.x), fminf(a0.y, b0.y), fminf(a0.z, b0.z), __uint_as_float(il > ir ? il : ir));
+        hi = make_float4(fmaxf(a1.x, b1.x), fmaxf(a1.y, b1.y), fmaxf(a1.z, b1.z), 0.f);
+        const uint32_t lref = l >= leaf0 ? (LEAF_REF | il) : l;
+        const uint32_t rref = r >= leaf0 ? (LEAF_REF | ir) : r;
+        q0 = make_float4(a0.x, a0.y, a0.z, __uint_as_float(lref));
+        q1 = make_float4(a1.x, a1.y, a1.z, __uint_as_float(rref));
+        q2 = make_float4(b0.x, b0.y, b0.z, __uint_as_float(il));
+        q3 = make_float4(b1.x, b1.y, b1.z, __uint_as_float(ir));
+        rec_of = cur;
+        if (here || cur == 0) {
+            float4* rc = rec + size_t(cur) * 4;
+            rc[0] = q0; rc[1] = q1; rc[2] = q2; rc[3] = q3;
+            rec_of = NONE;
+        }
         if (cur == 0) return;
-        cur = parent[cur];
+        me = cur;
+        if (here) {
+            s_min[REFIT_TB + cur - base] = lo;
+            s_max[REFIT_TB + cur - base] = hi;
+        }
+        cur = up;
     }
 }
 
@@ -801,7 +859,6 @@ uint64_t Broadphase::run(const float4* aabb_min, const float4* aabb_max, uint32_
     refit_flag.reserve(n);
     node_min.reserve(2 * size_t(n));
     node_max.reserve(2 * size_t(n));
-    node_maxid.reserve(2 * size_t(n));
     node_rec.reserve(4 * size_t(n));
     counts.reserve(n);
     offsets.reserve(n);
@@ -835,8 +892,8 @@ uint64_t Broadphase::run(const float4* aabb_min, const float4* aabb_max, uint32_
 
     if (m > 0) {
         k_build<<<(m + TB - 1) / TB, TB, 0, s>>>(sorted, m, left.p, right.p, parent.p, leaf_body.p, refit_flag.p);
-        k_refit<<<(m + TB - 1) / TB, TB, 0, s>>>(m, leaf_body.p, parent.p, left.p, right.p, refit_flag.p, aabb_min,
-                                                 aabb_max, node_min.p, node_max.p, node_maxid.p, node_rec.p);
+        k_refit<<<(m + REFIT_TB - 1) / REFIT_TB, REFIT_TB, 0, s>>>(m, leaf_body.p, parent.p, left.p, right.p, refit_flag.p, aabb_min,
+                                                 aabb_max, node_min.p, node_max.p, node_rec.p);
     }
     const uint32_t qgrid = m > 0 ? (uint32_t(m) + TB - 1) / TB : 1u;
     // One traversal per proxy: counts, plus the sorted partners of every proxy with at
@@ -1003,11 +1060,10 @@ extern "C" bgpu_status bgpu_broadphase_pairs_noalloc(const float* aabbs_dev, uin
         float4* node_min = sb.take<float4>(2 * size_t(n));
         float4* node_max = sb.take<float4>(2 * size_t(n));
         float4* node_rec = sb.take<float4>(4 * size_t(n));
-        uint32_t* node_maxid = sb.take<uint32_t>(2 * size_t(n));
         int* bounds = sb.take<int>(8);
         uint32_t* scalars = sb.take<uint32_t>(8);
         const void* taken[] = {mn, mx, keys, keys_alt, is_unb, leaf_body, parent, left, right, refit_flag, counts,
-                               offsets, flags, scan, unb_list, node_min, node_max, node_rec, node_maxid, bounds, scalars};
+                               offsets, flags, scan, unb_list, node_min, node_max, node_rec, bounds, scalars};
         for (const void* t : taken)
             if (!t) {
                 set_last_error("allocation-free broad phase: scratch array too small");
@@ -1055,8 +1111,8 @@ extern "C" bgpu_status bgpu_broadphase_pairs_noalloc(const float* aabbs_dev, uin
         const LeafKeys sorted{dk.Current(), dv.Current()};
         if (m > 0) {
             k_build<<<(m + TB - 1) / TB, TB, 0, s>>>(sorted, m, left, right, parent, leaf_body, refit_flag);
-            k_refit<<<(m + TB - 1) / TB, TB, 0, s>>>(m, leaf_body, parent, left, right, refit_flag, mn, mx, node_min,
-                                                     node_max, node_maxid, node_rec);
+            k_refit<<<(m + REFIT_TB - 1) / REFIT_TB, REFIT_TB, 0, s>>>(m, leaf_body, parent, left, right, refit_flag, mn, mx, node_min,
+                                                     node_max, node_rec);
         }
         uint32_t* status = scalars + 1;
         const uint32_t qgrid = m > 0 ? (uint32_t(m) + TB - 1) / TB : 1u;

@@ -80,3 +80,30 @@ def test_a_world_that_grows_across_the_limit_and_sleeps(n):
         # rounding of the box edges may differ by an ulp: all but touching boxes agree
         assert len(np.setxor1d(g, e)) <= 3
         assert w.stats()["device_status"] == 0
+
+
+@pytest.mark.parametrize("n", [2, 3, 511, 512, 513, 1024, 1025, 3000])
+def test_tree_at_the_edges_of_a_refit_block(n):
+    """The allocation-free entry takes the tree at every size: one block of leaves, its remainders, a
+    last block of one leaf, and a third of the boxes identical (equal keys, a deep subtree across blocks)."""
+    import ctypes
+
+    import torch
+
+    import bgpu
+    from test_zz_no_alloc import _entry
+
+    rng = np.random.default_rng(n)
+    c = rng.uniform(0.0, max(2.0, n ** (1.0 / 3.0)), size=(n, 3))
+    h = rng.uniform(0.1, 0.5, size=(n, 3))
+    c[n // 3: n // 3 + min(n // 3, 600)] = c[n // 3]
+    h[n // 3: n // 3 + min(n // 3, 600)] = 0.01
+    a = np.concatenate([c - h, c + h], axis=1).astype(np.float32)
+    want = _expected(a)
+    dev = torch.from_numpy(a).cuda()
+    out = torch.full((len(want) + 8, 2), -1, dtype=torch.int32, device="cuda")
+    got = ctypes.c_uint64(0)
+    torch.cuda.synchronize()
+    assert _entry(bgpu)(dev.data_ptr(), n, out.data_ptr(), len(want) + 8, ctypes.byref(got), None) == 0
+    torch.cuda.synchronize()
+    np.testing.assert_array_equal(out[: got.value].cpu().numpy().view(np.uint32), want)
