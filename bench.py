@@ -223,11 +223,11 @@ def count_launches(w, dt, nsteps=2):
 
 def solve_traffic(contacts):
     """DRAM bytes of the PGS launches of one step, from the committed ncu capture of the same
-    kernels (profiles/k_solve_chunks_large_pile_131072.md, a shorter-settled pile), scaled to
+    kernel (profiles/k_solve_flow_large_pile.md, a shorter-settled pile), scaled to
     this step by its contact count (the kernels' traffic grows with the rows they sweep)."""
     import re
 
-    path = os.path.join(ROOT, "profiles", "k_solve_chunks_large_pile_131072.md")
+    path = os.path.join(ROOT, "profiles", "k_solve_flow_large_pile.md")
     try:
         text = open(path).read()
         dram = float(re.search(r"dram_bytes_per_launch:\s*([0-9.eE+]+)", text).group(1))
@@ -548,7 +548,7 @@ def main():
                        "pairs": st["num_pairs"], "contacts": st["num_contacts"],
                        "contact_pairs": st["num_contact_pairs"], "colours": st["num_colours"],
                        "stage_ms_per_step": [x / launches for x in st["stage_ms"]]},
-            "roofline": {"kernel": "k_solve_chunks (chunked colour-batched PGS)", "bound": "hbm",
+            "roofline": {"kernel": "k_solve_flow (chunked colour-batched PGS)", "bound": "hbm",
                          "achieved": achieved, "peak": hbm, "unit": "GB/s",
                          "frac": (achieved / hbm) if achieved else None, "traffic": traffic,
                          "traffic_source": traffic_src, "peak_kind": peak_kind,
