@@ -607,8 +607,9 @@ __device__ __forceinline__ bool same_bits(V3 a, V3 b) {
             (__float_as_uint(a.z) ^ __float_as_uint(b.z))) == 0u;
 }
 
-// The walk is a function of the simplex alone, so a simplex that comes back comes back for ever: such a
-// walk runs into the iteration limit and reports nothing, which the check against the simplex kept at
+// The walk is a function of the reduced simplex and its closest point (the same edge of two triangles can
+// have closest points that differ in the last bit), so a state that comes back comes back for ever: such
+// a walk runs into the iteration limit and reports nothing, which the check against the state kept at
 // iteration 4, 8, 12, 16, 24, 32 and 48 says at once. Walks end within 20 iterations or not at all: of
 // 16,000 pairs of the 16,384-body mixed pile 50 ran to the 64th, and each held its warp that long.
 static __device__ __forceinline__ GjkResult gjk_contact(const ConvexPair& cp, bool has_seed, V3 seed, float thr) {
@@ -623,7 +624,7 @@ static __device__ __forceinline__ GjkResult gjk_contact(const ConvexPair& cp, bo
     int n = 1;
     V3 dir = -first.w;
     float touch2 = TOUCH2 * fmaxf(len2(first.w), 1.0f);
-    V3 K0{}, K1{}, K2{};  // the kept simplex: reduced, so of at most three points
+    V3 K0{}, K1{}, K2{}, Kv{};  // the kept state: a reduced simplex has at most three points
     int kn = 0;
     GjkResult out;
     out.kind = 0;
@@ -649,11 +650,12 @@ static __device__ __forceinline__ GjkResult gjk_contact(const ConvexPair& cp, bo
             }
             return out;
         }
-        if (n == kn && same_bits(B0.w, K0) && (n < 2 || same_bits(B1.w, K1)) && (n < 3 || same_bits(B2.w, K2))) break;
+        if (n == kn && same_bits(v, Kv) && same_bits(B0.w, K0) && (n < 2 || same_bits(B1.w, K1)) && (n < 3 || same_bits(B2.w, K2))) break;
         if (it >= 4 && (it & 3) == 0 && (it <= 16 || (it & 7) == 0) && (it <= 32 || it == 48)) {
             K0 = B0.w;
             K1 = B1.w;
             K2 = B2.w;
+            Kv = v;
             kn = n;
         }
         dir = -v;

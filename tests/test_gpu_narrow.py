@@ -81,3 +81,18 @@ def test_terrain_query_beyond_the_lists(gpu):
     with pytest.raises(gpu.BgpuError, match="device status bits 0x100"):  # more candidates than a pair keeps
         w.step(1.0 / 60.0)
     assert np.isfinite(w.state()).all()
+
+
+@pytest.mark.parametrize("seed,spread", [(1, 0.45), (2, 0.6)])
+def test_walks_that_come_back(gpu, seed, spread):
+    """Walks that never settle (3 in 1,000 pairs) end early on the device and at the limit in the oracle;
+    the rest must not be taken for one of them: point counts equal, points within 1e-5."""
+    from test_gpu_parity import _narrow_case
+
+    rng = np.random.default_rng(seed)
+    w, o = _both(gpu)
+    pts = [_hull(rng, 24, 0.45), _hull(rng, 8, 0.5)]
+    for x in (w, o):
+        assert [x.hull(pts[0]), x.hull(pts[1]), x.capsule(0.2, 0.4), x.box([0.4, 0.3, 0.2])] == [0, 1, 2, 3]
+    mism, err = _narrow_case(w, o, [0, 1, 2, 3], rng, 20000, spread)
+    assert not mism and err <= 1e-5, (mism[:10], err)
