@@ -654,7 +654,7 @@ struct SolveArgs {
     float4* vtab;             // velocity contact table (VT_PLANES planes)
     float4* stab;             // split contact table (ST_PLANES planes)
     float4* srec;             // adjoint recording (else null): per (sweep, slot, contact) vn, impulse, clamp bits
-    unsigned int* bar;        // [0] velocity-team barrier counter, [1] split-team counter
+    unsigned int* bar;        // [0] velocity-team barrier counter, [1] split-team counter, [8] flow_by_barriers
     uint32_t* status;
     float inv_dt;
     float restitution_threshold;
@@ -1233,6 +1233,28 @@ __global__ void __launch_bounds__(256) k_flow_table(SolveArgs a) {
     }
 }
 
+// The same solve with a grid barrier after every phase, for a colouring that overflowed: its surplus groups
+// share the last colour with others at one body, so a colour is no longer one version of a body and a wait
+// for one may never end. Every group is solved; only the order (and, as they run side by side, the velocity
+// updates) of those at that one body is left open. A slot's table entries stay with one thread (the deal
+// depends on the colour alone). Some 3 us a phase: 128 colours and 20 sweeps take 8 ms, under an error status.
+template <uint32_t TB>
+__device__ __noinline__ void flow_by_barriers(const SolveArgs& a, const FlowArgs& f) {
+    const uint32_t ncol = a.scalars[4], iters = a.iterations;
+    const uint32_t first = blockIdx.x * TB + threadIdx.x, stride = gridDim.x * TB;
+    uint32_t nbar = 0;
+    for (uint32_t sw = 0; sw <= iters; ++sw)
+        for (uint32_t c = 0; c < ncol; ++c) {
+            for (uint32_t t = a.offset[c] + first; t < a.end[c]; t += stride)
+                run_item<true>(a, sw, iters, t, __ldg(&a.batch_rec[t]));
+            const uint32_t* soff = f.soff + size_t(c) * (f.P + 1);
+            if (sw)
+                for (uint32_t t = soff[0] + first; t < soff[f.P]; t += stride)
+                    run_item<false>(a, sw - 1u, iters - 1u, t, __ldg(&a.split_rec[t]));
+            team_barrier(a.bar + 8, ++nbar * gridDim.x, a.status);
+        }
+}
+
 // The items of a warp: 32 lanes of a phase (sweep, colour) of its chunk. A phase's lanes are its
 // velocity lanes (a group of 4 or 3 rows takes 4 lanes, of 2 rows 2, of 1 row one), padded to a
 // whole warp, then one lane per split group; split sweep s runs in the phases of velocity sweep
@@ -1274,6 +1296,10 @@ __global__ void __launch_bounds__(TB, 1) k_solve_flow(SolveArgs a, FlowArgs f) {
     __shared__ uint4 s_end[MAX_COLOURS];
     const uint32_t ncol = a.scalars[4];
     const uint32_t iters = a.iterations;
+    if (*a.status & ST_COLOUR_OVERFLOW) {  // set by the colouring, before this launch: the same for all blocks
+        flow_by_barriers<TB>(a, f);
+        return;
+    }
     const uint32_t b = blockIdx.x / f.bpc, lane = threadIdx.x & 31u;  // the chunk
     const uint32_t nwarps = f.bpc * (TB / 32u), warp = (blockIdx.x % f.bpc) * (TB / 32u) + (threadIdx.x >> 5);
     for (uint32_t c = threadIdx.x; c < ncol; c += TB) {

@@ -8,6 +8,7 @@ BGPU_PGS=team selects the team kernel (read once per process), hence the child p
 import os
 import subprocess
 import sys
+import time
 
 import numpy as np
 import pytest
@@ -18,6 +19,7 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 CHILD = r"""
 import sys
+import time
 sys.path[:0] = [sys.argv[1] + "/bullet-physics_b200"]
 import numpy as np
 import bgpu, scenes
@@ -95,3 +97,49 @@ def test_worlds_of_different_sizes_step_side_by_side(gpu_oracle):
     for w in (big, small, big):
         w.step(1.0 / 60.0, 30)
         assert w.stats()["device_status"] == 0
+
+
+@pytest.mark.parametrize("balls,layers,iters", [(70, 3, 10), (70, 3, 0), (140, 11, 20)])
+def test_a_body_with_more_neighbours_than_colours(gpu_oracle, balls, layers, iters):
+    """A heavy tray with more balls on it than a colouring has colours (64 and 128), one in three of them sunk
+    deep enough for a split row, no gravity: the step reports the overflow and nothing else, at once, every
+    group is still solved (the balls stop, the sunk ones are pushed out), and a pile beside the tray
+    moves as it does without it, bit for bit."""
+    bgpu, _, scenes = gpu_oracle
+    is_box, ppos, pquat = scenes.large_pile_arrays(10, 10, layers, 4, 1.0)
+    ppos = ppos + np.array([40.0, 0.0, 0.0])
+    pile = len(ppos)
+    k = np.arange(balls)
+    sunk = k % 3 == 0
+    bpos = np.stack([(k % 12) * 0.5 - 2.75, np.where(sunk, 5.395, 5.445), (k // 12) * 0.5 - 2.75], axis=1)
+
+    def world(tray):
+        w = bgpu.World(gravity=(0.0, 0.0, 0.0), num_iterations=iters)
+        plane, box, sph = w.plane([0.0, 1.0, 0.0], 0.0), w.box([0.5, 0.5, 0.5]), w.sphere(0.5)
+        shape = np.concatenate([[plane], np.where(is_box, box, sph)])
+        pos, quat = np.concatenate([np.zeros((1, 3)), ppos]), np.concatenate([[[0, 0, 0, 1]], pquat])
+        mass = np.concatenate([[0.0], np.ones(pile)])
+        vel = np.zeros((1 + pile, 3))
+        if tray:
+            shape = np.concatenate([shape, [w.box([4.0, 0.25, 4.0])], np.full(balls, w.sphere(0.2))])
+            pos = np.concatenate([pos, [[0.0, 5.0, 0.0]], bpos])
+            quat = np.concatenate([quat, np.tile([0, 0, 0, 1], (balls + 1, 1))])
+            mass = np.concatenate([mass, [1e5], np.ones(balls)])
+            vel = np.concatenate([vel, np.zeros((1, 3)), np.tile([0.0, -0.1, 0.0], (balls, 1))])
+        w.add_bodies_array(shape, pos, quat, linvel=vel, mass=mass)
+        return w
+
+    w, alone = world(True), world(False)
+    for step in range(3):
+        alone.step(1.0 / 60.0)
+        t0 = time.perf_counter()
+        with pytest.raises(bgpu.BgpuError, match="device status bits 0x8$"):
+            w.step(1.0 / 60.0)
+        assert step == 0 or time.perf_counter() - t0 < 1.0
+        assert w.stats()["device_status"] == 8 and w.stats()["num_contact_pairs"] >= balls
+        np.testing.assert_array_equal(w.state()[:pile + 1], alone.state())
+    assert alone.stats()["num_contacts"] > 0
+    ball = w.state()[pile + 2:]
+    if iters:  # (without a sweep there are no impulses)
+        assert (ball[:, 8] > -0.02).all() and (ball[:, 1] > bpos[:, 1] - 2e-3).all()
+        assert (ball[sunk, 1] > bpos[sunk, 1] + 1e-3).all()
