@@ -709,6 +709,10 @@ __global__ void __launch_bounds__(CCD_CAST_THREADS) k_ccd_cast(BodyDev b, const 
     const uint32_t g = total <= CCD_WARP_CASTS ? 32u : (total <= 2u * CCD_WARP_CASTS ? 16u : 8u);
     const uint32_t td = g == 32u ? 4u : (g == 16u ? 3u : 2u), bd = td + 1u;
     const uint32_t segs = 32u / g, sl = lane % g;
+    const uint32_t mine = (g == 32u ? 0xffffffffu : (1u << g) - 1u) << (lane - sl);  // the segment's lanes
+    // A walk takes at most 258 steps (the first support point, 64 iterations of at most four, the end), a
+    // cast 41 rounds of them, and each vote is a step of every walk: the loop below ends before `left` does.
+    uint32_t left = (total / (nwarps * segs) + 1u) * (41u * 258u);
     // The segment's cast (the same values on all its lanes) and the lane's walk.
     enum { TERNARY, CLOSEST, BISECT, IDLE };
     int phase = IDLE;
@@ -721,7 +725,7 @@ __global__ void __launch_bounds__(CCD_CAST_THREADS) k_ccd_cast(BodyDev b, const 
     w.d2 = 0.0f;
     bool ready = true;   // the segment's round is over and its decisions are taken
     uint32_t seen = 0u;  // the last vote on the walks that are done
-    for (;;) {
+    for (;; --left) {
         if (ready) {
             // The next round of probes: of this cast, or of the segment's next one.
             w.done = true;
@@ -737,6 +741,7 @@ __global__ void __launch_bounds__(CCD_CAST_THREADS) k_ccd_cast(BodyDev b, const 
                 if (ended) {
                     // Fractions are not negative, so their bits order as they do.
                     if (sl == 0u) atomicMin(reinterpret_cast<unsigned int*>(&clamp[entry]), __float_as_uint(f));
+                    __syncwarp(mine);
                     ended = false;
                     phase = IDLE;
                     continue;
@@ -747,8 +752,12 @@ __global__ void __launch_bounds__(CCD_CAST_THREADS) k_ccd_cast(BodyDev b, const 
                     if (x >= off[q]) { r = q; at = x - off[q]; }
                 x += nwarps * segs;
                 const uint4 it = items.items[size_t(r) * items.m + at];
-                // A hit may have overtaken the cast's bound.
-                if (!(__uint_as_float(it.z) < *(volatile float*)&clamp[it.x])) continue;
+                // A hit may have overtaken the cast's bound. One lane reads for the segment, which has to go
+                // one way: other warps lower the clamp meanwhile.
+                float reach = 0.0f;
+                if (sl == 0u) reach = *(volatile float*)&clamp[it.x];
+                reach = __shfl_sync(mine, reach, 0, int(g));
+                if (!(__uint_as_float(it.z) < reach)) continue;
                 entry = it.x;
                 const uint32_t i = ids[entry];
                 from = from4(b.pos[i]);
@@ -787,6 +796,10 @@ __global__ void __launch_bounds__(CCD_CAST_THREADS) k_ccd_cast(BodyDev b, const 
             }
         }
         if (!__any_sync(0xffffffffu, phase != IDLE)) break;
+        if (left == 0u) {
+            if (lane == 0u) atomicOr(status, ST_BARRIER_TIMEOUT);
+            break;
+        }
         if (!w.done) w.step(t);
         // Follow the decisions as far as their probes are done: a round ends with the probes on the
         // taken path, whatever the walks beside it are still at.
@@ -810,19 +823,19 @@ __global__ void __launch_bounds__(CCD_CAST_THREADS) k_ccd_cast(BodyDev b, const 
                 ready = false;
                 continue;
             }
-            bool left;
+            bool lower;
             if (phase == TERNARY) {
                 const float m1 = l + (h - l) / 3.0f, m2 = h - (h - l) / 3.0f;
-                left = d1 < d2;
-                if (left) h = m2;
+                lower = d1 < d2;
+                if (lower) h = m2;
                 else l = m1;
             } else {
                 const float mid = (l + h) * 0.5f;
-                left = d1 <= 1e-8f;
-                if (left) h = mid;
+                lower = d1 <= 1e-8f;
+                if (lower) h = mid;
                 else l = mid;
             }
-            n = 2u * n + (left ? 1u : 2u);
+            n = 2u * n + (lower ? 1u : 2u);
         }
         if (!ready) continue;
         lo = l;

@@ -260,3 +260,31 @@ def test_ccd_with_more_candidates_than_the_casting_kernel_takes(gpu):
         t.ccd(t.body(sph, (x, 1.5, 0.0), linvel=(0.0, -400.0, 0.0), mass=1.0), 0.05, 0.15)
     t.step()
     assert (t.g.ccd_clamps() < 1.0).sum() == 2
+
+
+@pytest.mark.parametrize("n", [100, 250, 500])
+def test_ccd_casts_of_one_body_side_by_side(gpu, n):
+    """Eight candidates a body (plates one below the other, one of them a mesh), whose casts lower the body's
+    clamp while others of its candidates test their bounds against it: 800, 2,000 and 4,000 casts (a
+    warp, half and a quarter of one each) give the fractions of 12 bodies at a time, bit for bit."""
+    rng = np.random.default_rng(n)
+    pos = np.stack([rng.uniform(-0.6, 0.6, n), rng.uniform(0.9, 1.1, n), rng.uniform(-0.6, 0.6, n)], axis=1)
+    vel = np.stack([rng.uniform(-9, 9, n), rng.uniform(-600, -240, n), np.zeros(n)], axis=1)
+
+    def clamps(lo, hi):
+        w = gpu.World(gravity=(0.0, 0.0, 0.0))
+        plate, sph = w.add_shape(orc.BOX, [2.0, 0.01, 2.0]), w.add_shape(orc.SPHERE, [0.1])
+        mesh = w.mesh([[-2, 0, -2], [2, 0, -2], [2, 0, 2], [-2, 0, 2]], [0, 2, 1, 0, 3, 2])
+        for k in range(8):  # overlapping bounding balls: every bound is 0 or near it
+            w.add_body(mesh if k == 3 else plate, (0.0, 0.5 - 0.25 * ((5 * k) % 8), 0.0), mass=0.0)
+        for k in range(lo, hi):
+            w.add_body(sph, pos[k], linvel=vel[k], mass=1.0, group=2, mask=1)
+        w.set_ccd(8, np.full(hi - lo, 0.05), np.full(hi - lo, 0.1))
+        w.step(DT)
+        assert w.stats()["device_status"] == 0
+        return w.ccd_clamps()[8:]
+
+    together = clamps(0, n)
+    apart = np.concatenate([clamps(lo, min(lo + 12, n)) for lo in range(0, n, 12)])
+    assert (together < 1.0).all()
+    np.testing.assert_array_equal(together, apart)
