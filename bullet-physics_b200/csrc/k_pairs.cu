@@ -952,14 +952,19 @@ __global__ void __launch_bounds__(32 * EPA_WARPS) k_narrow_epa(BodyDev b, const 
     }
 }
 
-// The mesh route of the pair pass, a block a pair. Its first warp walks the mesh BVH and lists the
-// candidate triangles (those whose own box overlaps the query) in walk order; they are dealt to the
-// warps, each of which runs the GJK of its own side by side and gives the triangles whose cores
-// overlap the whole warp's EPA one after the other; thread 0 then keeps the hits in candidate order and
-// reduces them (the same points, in the same order, as collide_mesh's single pass). 500 bodies on the
-// terrain (250 pairs of up to 8 triangles, up to 6 of them overlapping): 140 us with a warp a pair, a
-// lane walking (30,000 cycles, now 7,000) and a thread's EPA in local memory; 56 us so.
-constexpr int MESH_WARPS = 4;
+// The mesh route of the pair pass, a block a pair, or with many pairs a warp. The first warp walks the mesh
+// BVH and lists the candidate triangles (those whose own box overlaps the query) in walk order; they
+// are dealt to the warps, each of which runs the GJK of its own side by side and gives the triangles
+// whose cores overlap the whole warp's EPA one after the other; one lane then keeps the hits in
+// candidate order and reduces them (the same points, in the same order, as collide_mesh's single
+// pass). 500 bodies on the terrain (250 pairs of up to 8 triangles, up to 6 of them overlapping): 140 us
+// with a warp a pair, a lane walking (30,000 cycles, now 7,000) and a thread's EPA in local
+// memory; 56 us so.
+constexpr uint32_t MESH_WARPS = 4;
+// A block's scratch (48 KB) leaves four on an SM: two waves of them, then a warp a pair has four times as
+// many pairs under way. The whole pair pass, block / warp a pair, on terrain: 254 pairs 105 / 130 us,
+// 947 148 / 165, 1,600 180 / 157, 2,500 170 / 123, 10,000 447 / 246, 40,000 1,615 / 924.
+constexpr uint32_t MESH_BLOCK_PAIRS = 2 * 4 * 148;
 constexpr int MESH_MAX_TRIS = 128;  // candidate triangles per pair (more: ST_MESH_CANDIDATES)
 constexpr uint32_t MESH_FRONT = 256;  // nodes in one generation of the walk
 static_assert(MESH_MAX_TRIS == 32 * MESH_WARPS, "one candidate a thread");
@@ -1094,19 +1099,29 @@ __global__ void __launch_bounds__(32 * MESH_WARPS) k_narrow_mesh(BodyDev b, cons
                                                                  const float4* __restrict__ hull,
                                                                  const uint64_t* __restrict__ pairs, uint32_t npairs,
                                                                  PairDataDev pd, uint32_t* status) {
-    __shared__ uint32_t s_slot[MESH_MAX_TRIS];
+    __shared__ uint32_t s_slots[MESH_WARPS][MESH_MAX_TRIS];
     __shared__ uint32_t s_n;
     __shared__ __align__(16) EpaScratch s_epa[MESH_WARPS];
-    // The walk's lists and the candidates' results lie in the scratch, before and after its use.
-    uint32_t(*s_front)[MESH_FRONT] = reinterpret_cast<uint32_t(*)[MESH_FRONT]>(&s_epa[0]);
-    float4* s_pt = reinterpret_cast<float4*>(&s_epa[1]);
-    float4* s_nr = s_pt + MESH_MAX_TRIS;
     static_assert(sizeof(EpaScratch) % 16 == 0 && sizeof(EpaScratch) >= 2 * MESH_MAX_TRIS * sizeof(float4) &&
                       sizeof(EpaScratch) >= 2 * MESH_FRONT * sizeof(uint32_t), "lists in the scratch");
     const uint32_t cnt = pd.scalars[ROUTE_COUNT0 + NP_MESH];
     if (blockIdx.x == 0 && threadIdx.x == 0) pd.scalars[1] += cnt;  // with the convex detections (statistics)
     const uint32_t wi = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    for (uint32_t t = blockIdx.x; t < cnt; t += gridDim.x) {
+    // W warps a pair: the block, or a warp for itself.
+    const bool whole = cnt <= MESH_BLOCK_PAIRS;
+    const uint32_t W = whole ? MESH_WARPS : 1u, rank = whole ? wi : 0u, own = whole ? 0u : wi;
+    const bool leader = lane == 0u && rank == 0u;
+    auto sync = [&] {
+        if (whole) __syncthreads();
+        else __syncwarp();
+    };
+    // The walk's lists and the candidates' results lie in the scratch, before and after its use.
+    uint32_t(*s_front)[MESH_FRONT] = reinterpret_cast<uint32_t(*)[MESH_FRONT]>(&s_epa[own]);
+    float4* s_pt = reinterpret_cast<float4*>(&s_epa[whole ? 1u : wi]);
+    float4* s_nr = s_pt + 32u * W;
+    uint32_t* s_slot = s_slots[own];
+    const uint32_t stride = whole ? gridDim.x : gridDim.x * MESH_WARPS;
+    for (uint32_t t = whole ? blockIdx.x : blockIdx.x * MESH_WARPS + wi; t < cnt; t += stride) {
         const uint32_t p = pd.route_list[size_t(NP_MESH - 1) * npairs + t];
         const uint64_t key = pairs[p];
         const uint32_t i = key_lo(key), j = key_hi(key);
@@ -1121,93 +1136,89 @@ __global__ void __launch_bounds__(32 * MESH_WARPS) k_narrow_mesh(BodyDev b, cons
         const bool has_seed = entry_seed(pd.entries + size_t(p) * ENTRY_F4, seed);
         const float thr = fminf(cv.cbt, ms.cbt);
         const uint32_t tri_base = mesh_tri_base(ms);
-        __syncthreads();  // the lists of the block's last pair have been read
-        if (wi == 0) {
-            const uint32_t n = mesh_candidates(cv, pc, qc, ms, pm, qm, hull, s_front, s_slot, status);
-            if (lane == 0) s_n = n;
+        sync();  // the last pair's lists have been read
+        uint32_t nc = 0;
+        if (rank == 0u) {
+            nc = mesh_candidates(cv, pc, qc, ms, pm, qm, hull, s_front, s_slot, status);
+            if (whole && lane == 0) s_n = nc;
         }
-        __syncthreads();
-        const uint32_t nc = s_n;
-        if (nc == 0) {
-            if (threadIdx.x == 0) {
-                Manifold m;
-                m.n = 0;
-                store_detection(pd, p, npairs, m);
-            }
-            continue;
-        }
+        sync();
+        if (whole) nc = s_n;
+        MeshCandidates cand;  // the leader's
+        cand.n = 0;
         const bool sphere = cv.type == SHAPE_SPHERE;
         Shape tri;
         tri.type = SHAPE_HULL;
         tri.hull_cnt = 3;
         tri.margin = 0.0f;
         tri.cbt = thr;
-        const uint32_t k = lane * MESH_WARPS + wi, o = k < nc ? tri_base + 3 * s_slot[k] : tri_base;
-        V3 pt = V3{0.f, 0.f, 0.f}, nl = V3{0.f, 0.f, 0.f};
-        float pen = 0.0f;
-        bool hit = false, deep = false;
-        V3 simplex[4] = {};
-        if (k < nc && sphere) {
-            const V3 center = rotate(qinv(qm), pc - pm);
-            if (sphere_triangle(center, cv.p0, thr, from4(hull[o]), from4(hull[o + 1]), from4(hull[o + 2]), pt, nl,
-                                pen)) {
-                pt = pm + rotate(qm, pt);
-                nl = rotate(qm, -nl);
-                hit = true;
-            }
-        } else if (k < nc) {
-            tri.hull_off = o;
-            Manifold one;
-            deep = collide_convex_gjk(cv, pc, qc, tri, pm, qm, has_seed, seed, hull, one, simplex) == 2;
-            if (one.n) {
-                pt = one.pos[0];
-                nl = one.nrm[0];
-                pen = one.pen[0];
-                hit = true;
-            }
-        }
-        __syncwarp();
-        for (uint32_t todo = __ballot_sync(0xffffffffu, deep); todo; todo &= todo - 1u) {
-            const int src = __ffs(int(todo)) - 1;
-            V3 sx[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-                sx[q] = V3{__shfl_sync(0xffffffffu, simplex[q].x, src), __shfl_sync(0xffffffffu, simplex[q].y, src),
-                           __shfl_sync(0xffffffffu, simplex[q].z, src)};
-            tri.hull_off = __shfl_sync(0xffffffffu, o, src);
-            Manifold one;
-            collide_convex_epa(cv, pc, qc, tri, pm, qm, hull, sx, s_epa[wi], one, status);
-            if (int(lane) == src && one.n) {
-                pt = one.pos[0];
-                nl = one.nrm[0];
-                pen = one.pen[0];
-                hit = true;
-            }
-        }
-        __syncthreads();  // the scratch is free
-        if (k < nc) {
-            s_pt[k] = to4(pt, pen);
-            s_nr[k] = to4(nl, hit ? 1.0f : 0.0f);
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            MeshCandidates cand;
-            cand.n = 0;
-            for (uint32_t q = 0; q < nc; ++q) {
-                const float4 nr = s_nr[q];
-                if (nr.w == 0.0f) continue;
-                if (cand.n == MESH_MAX_CAND) {
-                    atomicOr(status, ST_MESH_CANDIDATES);
-                    break;
+        for (uint32_t k0 = 0; k0 < nc; k0 += 32u * W) {
+            const uint32_t k = k0 + lane * W + rank, o = k < nc ? tri_base + 3 * s_slot[k] : tri_base;
+            V3 pt = V3{0.f, 0.f, 0.f}, nl = V3{0.f, 0.f, 0.f};
+            float pen = 0.0f;
+            bool hit = false, deep = false;
+            V3 simplex[4] = {};
+            if (k < nc && sphere) {
+                const V3 center = rotate(qinv(qm), pc - pm);
+                if (sphere_triangle(center, cv.p0, thr, from4(hull[o]), from4(hull[o + 1]), from4(hull[o + 2]), pt, nl,
+                                    pen)) {
+                    pt = pm + rotate(qm, pt);
+                    nl = rotate(qm, -nl);
+                    hit = true;
                 }
-                const float4 pq = s_pt[q];
-                cand.pos[cand.n] = from4(pq);
-                cand.pen[cand.n] = pq.w;
-                cand.nrm[cand.n] = from4(nr);
-                ++cand.n;
+            } else if (k < nc) {
+                tri.hull_off = o;
+                Manifold one;
+                deep = collide_convex_gjk(cv, pc, qc, tri, pm, qm, has_seed, seed, hull, one, simplex) == 2;
+                if (one.n) {
+                    pt = one.pos[0];
+                    nl = one.nrm[0];
+                    pen = one.pen[0];
+                    hit = true;
+                }
             }
+            __syncwarp();
+            for (uint32_t todo = __ballot_sync(0xffffffffu, deep); todo; todo &= todo - 1u) {
+                const int src = __ffs(int(todo)) - 1;
+                V3 sx[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    sx[q] = V3{__shfl_sync(0xffffffffu, simplex[q].x, src), __shfl_sync(0xffffffffu, simplex[q].y, src),
+                               __shfl_sync(0xffffffffu, simplex[q].z, src)};
+                tri.hull_off = __shfl_sync(0xffffffffu, o, src);
+                Manifold one;
+                collide_convex_epa(cv, pc, qc, tri, pm, qm, hull, sx, s_epa[wi], one, status);
+                if (int(lane) == src && one.n) {
+                    pt = one.pos[0];
+                    nl = one.nrm[0];
+                    pen = one.pen[0];
+                    hit = true;
+                }
+            }
+            sync();  // the scratch is free
+            s_pt[lane * W + rank] = to4(pt, pen);
+            s_nr[lane * W + rank] = to4(nl, hit ? 1.0f : 0.0f);
+            sync();
+            if (leader)
+                for (uint32_t q = 0; q < min(nc - k0, 32u * W); ++q) {
+                    const float4 nr = s_nr[q];
+                    if (nr.w == 0.0f) continue;
+                    if (cand.n == MESH_MAX_CAND) {
+                        atomicOr(status, ST_MESH_CANDIDATES);
+                        break;
+                    }
+                    const float4 pq = s_pt[q];
+                    cand.pos[cand.n] = from4(pq);
+                    cand.pen[cand.n] = pq.w;
+                    cand.nrm[cand.n] = from4(nr);
+                    ++cand.n;
+                }
+            sync();  // the results have been read
+        }
+        if (leader) {
             Manifold m;
-            reduce_to_manifold(cand, m);
+            m.n = 0;
+            if (nc) reduce_to_manifold(cand, m);
             if (mesh_a) mf_flip(m);
             store_detection(pd, p, npairs, m);
         }

@@ -69,6 +69,29 @@ def test_bodies_in_terrain(gpu, count, half):
     lockstep(w, o, 1.0 / 60.0, 4, f"{count} on terrain")
 
 
+@pytest.mark.parametrize("count", [1184, 1185])
+def test_terrain_pairs_on_both_sides_of_a_block_a_pair(gpu, count):
+    """As many mesh pairs as take a block each, and one more (a warp each), of up to some 70 triangles
+    (more than a warp's lanes)."""
+    import scenes
+
+    rng = np.random.default_rng(7)
+    w, o = _both(gpu)
+    v, idx = scenes.wavy_grid_mesh(180, 180, (-22.5, -22.5), (0.25, 0.25), 0.2, 0.4, 0.3)
+    pts = _hull(rng, 12, 0.45)
+    for x in (w, o):
+        assert x.mesh(v, idx) == 0
+        assert [x.box([0.45, 0.1, 0.45]), x.hull(pts), x.sphere(0.3)] == [1, 2, 3]
+        x.add_body(0, (0.0, 0.0, 0.0), mass=0.0)
+    for k in range(count):
+        p = (-21.0 + 1.2 * (k % 35), 0.15, -21.0 + 1.2 * (k // 35))
+        q = _quat(rng)
+        for x in (w, o):
+            x.add_body(1 + k % 3, p, q, mass=1.0)
+    lockstep(w, o, 1.0 / 60.0, 2, f"{count} on terrain")
+    assert (w.pairs()[:, 0] == 0).sum() == count
+
+
 def test_terrain_query_beyond_the_lists(gpu):
     import scenes
 
