@@ -1238,6 +1238,7 @@ __global__ void __launch_bounds__(256) k_flow_table(SolveArgs a) {
 // for one may never end. Every group is solved; only the order (and, as they run side by side, the velocity
 // updates) of those at that one body is left open. A slot's table entries stay with one thread (the deal
 // depends on the colour alone). Some 3 us a phase: 128 colours and 20 sweeps take 8 ms, under an error status.
+// (The caller's parameters are __grid_constant__: a copy of them to pass on here cost every solve 1 to 2 %.)
 template <uint32_t TB>
 __device__ __noinline__ void flow_by_barriers(const SolveArgs& a, const FlowArgs& f) {
     const uint32_t ncol = a.scalars[4], iters = a.iterations;
@@ -1288,7 +1289,8 @@ struct FlowItem {
 // flight (1,785 us). One group a lane instead of one contact a lane halves the instructions but holds
 // a warp up for the slowest of 32 groups (1,887 us at 160 threads, the most its staging allows).
 template <uint32_t TB>
-__global__ void __launch_bounds__(TB, 1) k_solve_flow(SolveArgs a, FlowArgs f) {
+__global__ void __launch_bounds__(TB, 1) k_solve_flow(const __grid_constant__ SolveArgs a,
+                                                      const __grid_constant__ FlowArgs f) {
     extern __shared__ float4 s_pl[];  // [stage][plane][thread]
     // Per colour: the chunk's part of the batches, and the ends of its velocity lanes on 4 and on 2
     // lanes a group, of all of them, and the phase's lanes with the split groups.
