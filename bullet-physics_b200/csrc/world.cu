@@ -139,11 +139,24 @@ struct World {
     // (threads per CTA, largest world solved by one warp), and the per-world batch records
     WorldPlan wplan;
     uint32_t wplan_block = 128, wplan_tau = 64;  // 0 threads: the global (all-worlds) solver
-    // Until a caller tunes, worlds of a few bodies more than wplan_tau run one per warp too: a block's other
-    // warps would only wait (1,024 worlds of 64 boxes and a plane: 200 us a solve in blocks of 128
-    // threads, four waves of them, 145 us one per warp).
-    static constexpr uint32_t UNTUNED_WARP_WORLD_BODIES = 96;
+    // Until a caller tunes, worlds of a few bodies more than wplan_tau run one per warp too if there are more
+    // of them than the GPU holds blocks (128 threads of 128 registers: four an SM); up to there a block a
+    // world has the SMs to itself. Solve in us, a block / a warp a world: 96 worlds of 65 bodies 141 / 222,
+    // 592 222 / 243, 650 320 / 249, 1,024 382 / 275; worlds of 65 to 96 bodies, 8 of them 93 / 191, 592 192 /
+    // 256, 900 185 / 183, 4,096 937 / 670; of 8 to 256 bodies, 96 103 / 128, 2,048 (230 of the sizes in
+    // question) 251 / 284.
+    static constexpr uint32_t UNTUNED_WARP_WORLD_BODIES = 96, UNTUNED_BLOCKS = 4 * 148;
     bool wplan_tuned = false;
+    // Worlds of up to this many bodies are solved by one warp.
+    uint32_t warp_world_max() const {
+        if (wplan_tuned || !batch) return wplan_tau;
+        uint32_t k = 0;
+        for (size_t w = 0; w + 1 < world_off_h.size(); ++w) {
+            const uint32_t nb = world_off_h[w + 1] - world_off_h[w];
+            k += nb > wplan_tau && nb <= UNTUNED_WARP_WORLD_BODIES ? 1u : 0u;
+        }
+        return k > UNTUNED_BLOCKS ? UNTUNED_WARP_WORLD_BODIES : wplan_tau;
+    }
     DevBuf<uint32_t> wcol;
     DevBuf<uint32_t> plain_off_d;    // a plain world's {0, n}, for the per-world solver
     static constexpr uint32_t PLAIN_WORLD_SOLVER_MAX_BODIES = 1024;
@@ -598,8 +611,7 @@ struct World {
         }
         if (wplan_block == 0) return;
         wcol.reserve(size_t(num_worlds()) * WS_STRIDE + 1);
-        build_world_plan(world_off_h, wplan_block,
-                         wplan_tuned ? wplan_tau : std::max(wplan_tau, UNTUNED_WARP_WORLD_BODIES), wplan, stream);
+        build_world_plan(world_off_h, wplan_block, warp_world_max(), wplan, stream);
     }
 
     bool use_world_solver() const { return wplan.valid && (joints_h.empty() || !batch); }
@@ -1177,7 +1189,10 @@ static void autotune_batch(World& W, float dt, uint32_t steps) {
     } release{e0, e1};
     check_cuda(cudaEventCreate(&e0), "event");
     check_cuda(cudaEventCreate(&e1), "event");
-    Cand best{W.wplan_block, W.wplan_tau};
+    Cand best{W.wplan_block, W.warp_world_max()};  // the shape in use
+    if (std::none_of(cands.begin(), cands.end(),
+                     [&](const Cand& c) { return c.block == best.block && (!c.block || c.tau == best.tau); }))
+        cands.push_back(best);
     W.wplan_tuned = true;
     float best_ms = 0.0f, global_ms = 0.0f;
     uint32_t timed = 0;
@@ -1752,7 +1767,7 @@ bgpu_status bgpu_batch_get_tuning(bgpu_world* w, bgpu_batch_tuning* out) {
     if (!w || !out) return bad_args("bgpu_batch_get_tuning");
     World& W = w->impl;
     out->threads_per_cta = W.wplan_block;
-    out->warp_world_max_bodies = W.wplan_tau;
+    out->warp_world_max_bodies = W.warp_world_max();
     out->ctas = W.use_world_solver() ? W.wplan.ncta : 0u;
     out->candidates = W.tuned_candidates;
     out->ms_per_step = W.tuned_ms;

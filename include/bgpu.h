@@ -322,8 +322,8 @@ typedef struct bgpu_batch_tuning {
 } bgpu_batch_tuning;
 /* Autotuner: from the batch's current state, times steps_per_candidate steps of
  * every candidate launch shape (threads per CTA 32 / 64 / 128 / 256 x warp-world
- * limits 0 / 32 / 64 / 128 / all, and the global solver), keeps the fastest, and
- * puts the batch back in the state it started from. out may be NULL. */
+ * limits 0 / 32 / 64 / 128 / all, the global solver, and the shape in use), keeps
+ * the fastest, and puts the batch back in the state it started from. out may be NULL. */
 bgpu_status bgpu_batch_autotune(bgpu_world* w, float dt, uint32_t steps_per_candidate, bgpu_batch_tuning* out);
 bgpu_status bgpu_batch_set_tuning(bgpu_world* w, uint32_t threads_per_cta, uint32_t warp_world_max_bodies);
 bgpu_status bgpu_batch_get_tuning(bgpu_world* w, bgpu_batch_tuning* out);

@@ -238,6 +238,26 @@ def test_batch_autotune_keeps_the_state_and_the_parity(gpu):
 
 
 @gpu_only
+@pytest.mark.parametrize("worlds,bodies,limit", [(4, 65, 64), (592, 65, 64), (593, 65, 96), (593, 96, 96), (593, 97, 64),
+                                                 (593, 64, 64)])
+def test_batch_tuning_reports_the_shape_in_use(gpu, worlds, bodies, limit):
+    """An untuned batch runs its worlds of 65 to 96 bodies one per warp when there are more of them than the GPU
+    holds blocks; the shape it reports, handed back, is the shape it runs."""
+    w = gpu.World(batch=True)
+    box = w.box([0.5, 0.5, 0.5])
+    n = worlds * bodies
+    pos = np.zeros((n, 3))
+    pos[:, 0] = 2.0 * np.tile(np.arange(bodies), worlds)
+    w.add_worlds_array([bodies] * worlds, np.full(n, box), pos, np.tile([0.0, 0.0, 0.0, 1.0], (n, 1)), mass=np.ones(n))
+    w.step(1.0 / 60.0)
+    t = w.tuning()
+    assert t["threads_per_cta"] == 128 and t["warp_world_max_bodies"] == limit
+    assert t["ctas"] == (worlds if bodies > limit else -(-worlds // 4))
+    w.set_tuning(t["threads_per_cta"], t["warp_world_max_bodies"])
+    assert w.tuning() == t
+
+
+@gpu_only
 def test_batch_set_tuning_rejects_bad_shapes(gpu):
     import bgpu
     import scenes
