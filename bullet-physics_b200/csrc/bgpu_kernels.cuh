@@ -269,10 +269,10 @@ struct Broadphase {
     DevBuf<uint32_t> masks;            // all-pairs pass: bit j of row i
     DevBuf<unsigned char> cub_tmp;
     DevBuf<int> bounds;          // 2 x 6 ordered ints: scene min/max of leaf centres
-    DevBuf<uint32_t> scalars;    // [1] proxies (worlds) with more partners than the stash holds
+    DevBuf<uint32_t> scalars;    // [1] proxies with more partners than the stash holds
     TileScanBuf scan;
-    uint32_t* host_scalars = nullptr;  // pinned, written by the device: [0] total pairs, [1] proxies (worlds)
-                                       // with more partners than the stash holds
+    uint32_t* host_scalars = nullptr;  // pinned, written by the device: [0] total pairs, [1] proxies with more
+                                       // partners than the stash holds
     int tree_m = 0;                    // bounded proxies in the last run's tree (0: no tree)
     uint32_t nunb = 0;                 // proxies of the last run kept out of the tree (device list `unbounded`)
     uint32_t unb_n = 0;                // proxies and
@@ -294,10 +294,13 @@ struct Broadphase {
     uint64_t run_worlds(const float4* aabb_min, const float4* aabb_max, uint32_t n,
                         const std::vector<uint32_t>& world_off_host, const uint32_t* world_off, const uint32_t* world_of,
                         DevBuf<uint64_t>& out, uint32_t* status_dev, cudaStream_t s);
-    DevBuf<uint32_t> mask_off;         // each world's first mask word
+    DevBuf<uint64_t> mask_off;         // each world's first mask word
     uint32_t mask_worlds = 0, mask_n = 0;  // the batch that mask_off describes
     uint64_t mask_words = 0;           // its masks
-    static constexpr uint64_t WORLD_MASK_WORDS_MAX = 1ull << 28;  // 1 GB of masks
+    // 256 MB of masks: one world of 46,340 bodies, two of 32,768. Beyond, the masks are made a part at a time
+    // and the tests twice, first to count (with a limit of 64 MB two worlds of 20,000 bodies took 94 ms a step
+    // for 42).
+    static constexpr uint64_t WORLD_MASK_WORDS_MAX = 1ull << 26;
 };
 
 // ---------------------------------------------------------------- islands (k_islands.cu)

@@ -408,7 +408,7 @@ __global__ void __launch_bounds__(TILE_TB) k_segments(uint32_t n, const uint32_t
 }
 
 // The segments at their place: the first stash_blocks blocks the stashed ones (slot t belongs to proxy
-// leaf_body[t], to proxy t when leaf_body is null), the others a tile of an unbounded proxy's partners.
+// leaf_body[t]), the others a tile of an unbounded proxy's partners.
 __global__ void __launch_bounds__(TILE_TB) k_write_pairs(int m, const uint32_t* __restrict__ leaf_body,
                                                          const uint32_t* __restrict__ counts,
                                                          const uint32_t* __restrict__ offsets,
@@ -420,7 +420,7 @@ __global__ void __launch_bounds__(TILE_TB) k_write_pairs(int m, const uint32_t* 
     if (blockIdx.x < stash_blocks) {
         const uint32_t t = blockIdx.x * TILE_TB + threadIdx.x;
         if (t >= uint32_t(m)) return;
-        const uint32_t i = leaf_body ? leaf_body[t] : t;
+        const uint32_t i = leaf_body[t];
         const uint32_t c = counts[i];
         if (c > STASH_SLOTS) return;
         const uint64_t base = offsets[i];
@@ -566,118 +566,29 @@ __global__ void k_set_unbounded(const uint32_t* __restrict__ unb, uint32_t nunb,
     if (u < nunb) is_unb[unb[u]] = 1;
 }
 
-// Batched worlds: world k owns proxies [off[k], off[k + 1]) and pairs only form
-// inside a world. One CTA per world tests every (i < j) of the world against
-// the other proxies staged in shared memory, tile by tile in ascending j, so
-// each proxy's partners come out in ascending order, as in the tree query. The
-// pass fills counts[i] and stashes the partners of every proxy with at most
-// STASH_SLOTS of them (stash[a * n + i]); a world with a proxy over that (a
-// ground plane under a pile) sets wover[w] and adds one to *n_over.
-constexpr int WP_TILE = 64;
-
-__global__ void __launch_bounds__(WP_TILE) k_world_pairs(const float4* __restrict__ bmin, const float4* __restrict__ bmax,
-                                                           const uint32_t* __restrict__ off, uint32_t n_worlds, uint32_t n,
-                                                           uint32_t* counts, uint32_t* stash, uint32_t* wover,
-                                                           uint32_t* n_over) {
-    __shared__ float4 smin[WP_TILE], smax[WP_TILE];
-    for (uint32_t w = blockIdx.x; w < n_worlds; w += gridDim.x) {
-        const uint32_t lo = off[w], hi = off[w + 1];
-        bool over = false;
-        for (uint32_t ibase = lo; ibase < hi; ibase += WP_TILE) {
-            const uint32_t i = ibase + threadIdx.x;
-            const bool has = i < hi;
-            float4 qmin = make_float4(0.f, 0.f, 0.f, 0.f), qmax = qmin;
-            if (has) { qmin = bmin[i]; qmax = bmax[i]; }
-            uint32_t cnt = 0;
-            for (uint32_t jbase = ibase; jbase < hi; jbase += WP_TILE) {
-                __syncthreads();
-                const uint32_t j = jbase + threadIdx.x;
-                if (j < hi) { smin[threadIdx.x] = bmin[j]; smax[threadIdx.x] = bmax[j]; }
-                __syncthreads();
-                const uint32_t jn = min(uint32_t(WP_TILE), hi - jbase);
-                if (!has) continue;
-                for (uint32_t q = 0; q < jn; ++q) {
-                    const uint32_t jj = jbase + q;
-                    if (jj > i && overlaps(qmin, qmax, smin[q], smax[q])) {
-                        if (cnt < STASH_SLOTS) stash[size_t(cnt) * n + i] = jj;
-                        ++cnt;
-                    }
-                }
-            }
-            if (has) {
-                counts[i] = cnt;
-                over |= cnt > STASH_SLOTS;
-            }
-        }
-        const int any = __syncthreads_or(over ? 1 : 0);
-        if (threadIdx.x == 0) {
-            wover[w] = any ? 1u : 0u;
-            if (any) atomicAdd(n_over, 1u);
-        }
-    }
-}
-
-// The segments of the proxies that k_world_pairs could not stash, in the worlds it
-// flagged. The CTA takes those proxies one at a time and tests 64 candidates j at
-// once; a ballot per warp ranks the hits, so the segment is written in ascending j.
-__global__ void __launch_bounds__(WP_TILE) k_world_pairs_write(const float4* __restrict__ bmin,
-                                                                 const float4* __restrict__ bmax,
-                                                                 const uint32_t* __restrict__ off, uint32_t n_worlds,
-                                                                 const uint32_t* __restrict__ counts,
-                                                                 const uint32_t* __restrict__ offsets,
-                                                                 const uint32_t* __restrict__ wover, uint64_t* out) {
-    static_assert(WP_TILE == 64, "two warps a CTA");
-    __shared__ uint32_t s_mask[2], s_hits[2];
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    for (uint32_t w = blockIdx.x; w < n_worlds; w += gridDim.x) {
-        if (!wover[w]) continue;  // uniform across the CTA
-        const uint32_t lo = off[w], hi = off[w + 1];
-        for (uint32_t ibase = lo; ibase < hi; ibase += WP_TILE) {
-            const uint32_t me = ibase + threadIdx.x;
-            const uint32_t m = __ballot_sync(0xffffffffu, me < hi && counts[me] > STASH_SLOTS);
-            __syncthreads();  // the previous tile's readers of s_mask are done
-            if (lane == 0) s_mask[warp] = m;
-            __syncthreads();
-            unsigned long long todo = (static_cast<unsigned long long>(s_mask[1]) << 32) | s_mask[0];
-            while (todo) {
-                const uint32_t i = ibase + uint32_t(__ffsll(static_cast<long long>(todo)) - 1);
-                todo &= todo - 1ull;
-                const float4 qmin = bmin[i], qmax = bmax[i];
-                uint64_t pos = offsets[i];
-                for (uint32_t jbase = i + 1; jbase < hi; jbase += WP_TILE) {
-                    const uint32_t j = jbase + threadIdx.x;
-                    const bool hit = j < hi && overlaps(qmin, qmax, bmin[j], bmax[j]);
-                    const uint32_t b = __ballot_sync(0xffffffffu, hit);
-                    if (lane == 0) s_hits[warp] = __popc(b);
-                    __syncthreads();
-                    const uint32_t h0 = s_hits[0], h1 = s_hits[1];
-                    if (hit) out[pos + (warp ? h0 : 0u) + __popc(b & ((1u << lane) - 1u))] = (uint64_t(i) << 32) | j;
-                    pos += h0 + h1;
-                    __syncthreads();  // s_hits is rewritten next round
-                }
-            }
-        }
-    }
-}
-
+// Batched worlds: world k owns proxies [off[k], off[k + 1]) and pairs only form inside a world.
+//
 // Bit j of row i of each world's masks (i < j, in the world's own numbers): their boxes overlap; counts[i]
-// the row's bits. One CTA a world, a lane a proxy j, a vote per 32 tests (k_all_pairs, world by world).
+// the row's bits. One CTA a world, a lane a proxy j, a vote per 32 tests (k_all_pairs, world by world). Rows
+// [r0, r1) of the batch, which lie in worlds [w0, w1) and start at a multiple of 128 in theirs; without masks
+// they are only counted.
 // A thread per proxy that walked the others one by one and kept what it found took 91 us for 4,096
 // worlds of 8 to 256 bodies and 79 us for 96 of them (a ground plane's 255 partners, one store after the
 // other); this takes 41 and 12.
 constexpr uint32_t WM_TILE = 128;
 
 __global__ void __launch_bounds__(WM_TILE) k_world_masks(const float4* __restrict__ bmin, const float4* __restrict__ bmax,
-                                                         const uint32_t* __restrict__ off, uint32_t n_worlds,
-                                                         const uint32_t* __restrict__ mask_off, uint32_t* masks,
-                                                         uint32_t* counts) {
+                                                         const uint32_t* __restrict__ off, uint32_t w0, uint32_t w1,
+                                                         uint32_t r0, uint32_t r1, const uint64_t* __restrict__ mask_off,
+                                                         uint64_t mask_base, uint32_t* masks, uint32_t* counts) {
     __shared__ float4 s_min[WM_TILE], s_max[WM_TILE];
     __shared__ uint32_t s_cnt[WM_TILE];
     const uint32_t lane = threadIdx.x & 31u;
-    for (uint32_t w = blockIdx.x; w < n_worlds; w += gridDim.x) {
+    for (uint32_t w = w0 + blockIdx.x; w < w1; w += gridDim.x) {
         const uint32_t lo = off[w], nb = off[w + 1] - lo, words = (nb + 31u) / 32u;
-        uint32_t* m = masks + mask_off[w];
-        for (uint32_t i0 = 0; i0 < nb; i0 += WM_TILE) {
+        const uint32_t to = min(r1 - lo, nb);
+        const uint64_t m = mask_off[w] - mask_base;  // (may be below 0 for rows that are not asked for)
+        for (uint32_t i0 = r0 > lo ? r0 - lo : 0u; i0 < to; i0 += WM_TILE) {
             __syncthreads();  // the tile before is done with
             if (i0 + threadIdx.x < nb) {
                 s_min[threadIdx.x] = bmin[lo + i0 + threadIdx.x];
@@ -685,24 +596,24 @@ __global__ void __launch_bounds__(WM_TILE) k_world_masks(const float4* __restric
             }
             s_cnt[threadIdx.x] = 0u;
             __syncthreads();
-            const uint32_t rows = min(WM_TILE, nb - i0);
+            const uint32_t rows = min(WM_TILE, to - i0);
             for (uint32_t j0 = i0; j0 < nb; j0 += WM_TILE) {
                 const uint32_t j = j0 + threadIdx.x, word = j >> 5;
                 if (word >= words) continue;  // uniform across the warp
                 float4 jmin = make_float4(0.f, 0.f, 0.f, 0.f), jmax = jmin;
                 if (j < nb) { jmin = bmin[lo + j]; jmax = bmax[lo + j]; }
-                for (uint32_t r0 = 0; r0 < rows; r0 += 32u) {
-                    if (word < (i0 + r0) >> 5) continue;  // no j of the word lies above these rows
+                for (uint32_t q0 = 0; q0 < rows; q0 += 32u) {
+                    if (word < (i0 + q0) >> 5) continue;  // no j of the word lies above these rows
                     uint32_t row = 0;
 #pragma unroll 8
-                    for (uint32_t r = 0; r < 32u; ++r) {
-                        const uint32_t b = __ballot_sync(0xffffffffu, (j > i0 + r0 + r) & (j < nb) &
-                                                                          overlaps_all(s_min[r0 + r], s_max[r0 + r], jmin, jmax));
-                        if (lane == r) row = b;
+                    for (uint32_t q = 0; q < 32u; ++q) {
+                        const uint32_t b = __ballot_sync(0xffffffffu, (j > i0 + q0 + q) & (j < nb) &
+                                                                          overlaps_all(s_min[q0 + q], s_max[q0 + q], jmin, jmax));
+                        if (lane == q) row = b;
                     }
-                    if (r0 + lane < rows) {
-                        m[size_t(i0 + r0 + lane) * words + word] = row;
-                        if (row) atomicAdd(&s_cnt[r0 + lane], __popc(row));
+                    if (q0 + lane < rows) {
+                        if (masks) masks[m + uint64_t(i0 + q0 + lane) * words + word] = row;
+                        if (row) atomicAdd(&s_cnt[q0 + lane], __popc(row));
                     }
                 }
             }
@@ -713,21 +624,21 @@ __global__ void __launch_bounds__(WM_TILE) k_world_masks(const float4* __restric
 }
 
 // The rows' pairs: a thread a row, but rows of many partners (a ground plane's) by the whole warp.
-__global__ void __launch_bounds__(256) k_world_rows(uint32_t n, const uint32_t* __restrict__ off,
+__global__ void __launch_bounds__(256) k_world_rows(uint32_t r0, uint32_t r1, const uint32_t* __restrict__ off,
                                                     const uint32_t* __restrict__ world_of,
-                                                    const uint32_t* __restrict__ mask_off,
+                                                    const uint64_t* __restrict__ mask_off, uint64_t mask_base,
                                                     const uint32_t* __restrict__ masks, const uint32_t* __restrict__ counts,
                                                     const uint32_t* __restrict__ offsets, uint64_t* out) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31u;
-    uint32_t cnt = 0, lo = 0, words = 0, first = 0;
-    uint64_t pos = 0;
-    if (i < n) {
+    const uint32_t i = r0 + blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31u;
+    uint32_t cnt = 0, lo = 0, words = 0;
+    uint64_t pos = 0, first = 0;
+    if (i < r1) {
         cnt = counts[i];
         if (cnt) {
             const uint32_t w = world_of[i];
             lo = off[w];
             words = (off[w + 1] - lo + 31u) / 32u;
-            first = mask_off[w] + (i - lo) * words;
+            first = mask_off[w] - mask_base + uint64_t(i - lo) * words;
             pos = offsets[i];
         }
     }
@@ -740,7 +651,8 @@ __global__ void __launch_bounds__(256) k_world_rows(uint32_t n, const uint32_t* 
     for (uint32_t todo = __ballot_sync(0xffffffffu, wide); todo; todo &= todo - 1u) {
         const int src = __ffs(int(todo)) - 1;
         const uint32_t ri = __shfl_sync(0xffffffffu, i, src), rlo = __shfl_sync(0xffffffffu, lo, src);
-        const uint32_t rwords = __shfl_sync(0xffffffffu, words, src), rfirst = __shfl_sync(0xffffffffu, first, src);
+        const uint32_t rwords = __shfl_sync(0xffffffffu, words, src);
+        const uint64_t rfirst = __shfl_sync(0xffffffffu, static_cast<unsigned long long>(first), src);
         uint64_t rpos = __shfl_sync(0xffffffffu, static_cast<unsigned long long>(pos), src);
         for (uint32_t w = (ri - rlo) >> 5; w < rwords; ++w) {
             const uint32_t m = masks[rfirst + w];
@@ -761,53 +673,61 @@ uint64_t Broadphase::run_worlds(const float4* aabb_min, const float4* aabb_max, 
     counts.reserve(n);
     offsets.reserve(n);
     if (mask_worlds != n_worlds || mask_n != n) {  // worlds were added
-        std::vector<uint32_t> first(n_worlds);
+        std::vector<uint64_t> first(n_worlds);
         mask_words = 0;
         for (uint32_t k = 0; k < n_worlds; ++k) {
             const uint64_t nb = world_off_host[k + 1] - world_off_host[k];
-            first[k] = uint32_t(mask_words);
+            first[k] = mask_words;
             mask_words += nb * ((nb + 31u) / 32u);
         }
         mask_off.reserve(n_worlds);
-        check_cuda(cudaMemcpyAsync(mask_off.p, first.data(), n_worlds * sizeof(uint32_t), cudaMemcpyHostToDevice, s), "h2d");
+        check_cuda(cudaMemcpyAsync(mask_off.p, first.data(), n_worlds * sizeof(uint64_t), cudaMemcpyHostToDevice, s), "h2d");
         check_cuda(cudaStreamSynchronize(s), "sync");
         mask_worlds = n_worlds;
         mask_n = n;
     }
-    if (mask_words <= WORLD_MASK_WORDS_MAX) {
-        masks.reserve(mask_words);
-        k_world_masks<<<std::min<uint32_t>(n_worlds, 148u * 32u), WM_TILE, 0, s>>>(aabb_min, aabb_max, world_off, n_worlds,
-                                                                                 mask_off.p, masks.p, counts.p);
-        const uint32_t tiles = tile_count<4>(n);
-        k_segments<<<tiles, TILE_TB, 0, s>>>(n, counts.p, offsets.p, scalars.p, host_scalars,
-                                             scan.begin(tiles, status_dev, s));
-        check_cuda(cudaStreamSynchronize(s), "broadphase sync");
-        const uint64_t total = host_scalars[0];
-        out.reserve(total + 1);
-        if (total)
-            k_world_rows<<<(n + 255) / 256, 256, 0, s>>>(n, world_off, world_of, mask_off.p, masks.p, counts.p, offsets.p,
-                                                         out.p);
-        return total;
-    }
-    // Masks of more than a gigabyte (a world of some 90,000 bodies): the stash pass.
-    stash.reserve(size_t(STASH_SLOTS) * n);
-    overflow.reserve(n_worlds);
-    const uint32_t grid = std::min<uint32_t>(n_worlds, 148u * 32u);
-    k_world_pairs<<<grid, WP_TILE, 0, s>>>(aabb_min, aabb_max, world_off, n_worlds, n, counts.p, stash.p, overflow.p,
-                                           scalars.p + 1);
+    auto make = [&](uint32_t w0, uint32_t w1, uint32_t r0, uint32_t r1, uint64_t base, uint32_t* to) {
+        k_world_masks<<<std::min<uint32_t>(w1 - w0, 148u * 32u), WM_TILE, 0, s>>>(aabb_min, aabb_max, world_off, w0, w1, r0, r1,
+                                                                               mask_off.p, base, to, counts.p);
+    };
+    auto write = [&](uint32_t r0, uint32_t r1, uint64_t base) {
+        k_world_rows<<<(r1 - r0 + 255) / 256, 256, 0, s>>>(r0, r1, world_off, world_of, mask_off.p, base, masks.p, counts.p,
+                                                           offsets.p, out.p);
+    };
+    const bool whole = mask_words <= WORLD_MASK_WORDS_MAX;
+    if (whole) masks.reserve(mask_words);
+    make(0, n_worlds, 0, n, 0, whole ? masks.p : nullptr);
     const uint32_t tiles = tile_count<4>(n);
     k_segments<<<tiles, TILE_TB, 0, s>>>(n, counts.p, offsets.p, scalars.p, host_scalars, scan.begin(tiles, status_dev, s));
     check_cuda(cudaStreamSynchronize(s), "broadphase sync");
-    uint64_t total = host_scalars[0];
-    const uint32_t n_over = host_scalars[1];
+    const uint64_t total = host_scalars[0];
     out.reserve(total + 1);
-    if (total) {
-        const uint32_t blocks = (n + TILE_TB - 1) / TILE_TB;
-        k_write_pairs<<<blocks, TILE_TB, 0, s>>>(int(n), nullptr, counts.p, offsets.p, stash.p, out.p, blocks, n, 1u,
-                                                 nullptr, nullptr, nullptr, nullptr);
-        if (n_over)
-            k_world_pairs_write<<<grid, WP_TILE, 0, s>>>(aabb_min, aabb_max, world_off, n_worlds, counts.p, offsets.p,
-                                                         overflow.p, out.p);
+    if (!total) return 0;
+    if (whole) {
+        write(0, n, 0);
+        return total;
+    }
+    // Too many masks: counted above, the tests are made again for as many rows at a time as the masks hold
+    // (whole worlds, or a multiple of 128 rows of one; 128 rows at least).
+    uint32_t k = 0, row = 0;  // the first world and its row still to do
+    uint64_t base = 0;        // their mask word
+    while (k < n_worlds) {
+        const uint32_t w0 = k, r0 = world_off_host[k] + row;
+        uint64_t words = 0;
+        for (; k < n_worlds; ++k, row = 0) {
+            const uint32_t nb = world_off_host[k + 1] - world_off_host[k], per = (nb + 31u) / 32u;
+            const uint64_t fit = per ? (WORLD_MASK_WORDS_MAX - std::min(words, WORLD_MASK_WORDS_MAX)) / per : nb;
+            uint32_t take = nb - row;
+            if (take > fit) take = std::max(uint32_t(fit) / WM_TILE * WM_TILE, words ? 0u : std::min(take, WM_TILE));
+            words += uint64_t(take) * per;
+            row += take;
+            if (row < nb) break;
+        }
+        const uint32_t r1 = k < n_worlds ? world_off_host[k] + row : n;
+        masks.reserve(words);
+        make(w0, std::min(k + 1u, n_worlds), r0, r1, base, masks.p);
+        write(r0, r1, base);
+        base += words;
     }
     return total;
 }

@@ -148,6 +148,45 @@ def test_batch_pairs_of_crowded_proxies(gpu):
 
 
 @gpu_only
+@pytest.mark.parametrize("sizes", [[300, 46400, 40], [46336, 46336], [33, 1100, 44000, 20000]])
+def test_batch_pairs_of_worlds_whose_masks_come_in_parts(gpu, sizes):
+    """Worlds with more mask words than are kept at once (2^26): the parts end inside a world, at a world's end
+    and span several; rows of a few partners and crowded ones (plane, large boxes). Each world's pairs
+    equal those of the same bodies in a plain world (all pairs or the tree), in ascending order."""
+    assert sum(n * -(-n // 32) for n in sizes) > 1 << 26
+    rng = np.random.default_rng(3)
+
+    def shapes(w):
+        return [w.plane([0.0, 1.0, 0.0], 0.0), w.box([3.0, 3.0, 3.0]), w.sphere(0.2)]
+
+    batch = gpu.World(gravity=(0.0, 0.0, 0.0), batch=True, num_iterations=1)
+    ids = shapes(batch)
+    parts, plain = [], []
+    for n in sizes:
+        e = (n * 0.4) ** (1.0 / 3.0)
+        kind = np.full(n, ids[2])
+        kind[0] = ids[0]
+        kind[5:n:997] = ids[1]
+        pos = rng.uniform(0.0, e, (n, 3)) + np.array([0.0, 0.1, 0.0])
+        pos[0] = 0.0
+        mass = np.where(kind == ids[2], 1.0, 0.0)
+        parts.append((kind, pos, mass))
+        w = gpu.World(gravity=(0.0, 0.0, 0.0), num_iterations=1)
+        assert shapes(w) == ids
+        w.add_bodies_array(kind, pos, np.tile([0.0, 0.0, 0.0, 1.0], (n, 1)), mass=mass)
+        w.step(1.0 / 240.0)
+        plain.append(w.pairs().astype(np.int64))
+        w.close()
+    kind, pos, mass = (np.concatenate(x) for x in zip(*parts))
+    batch.add_worlds_array(sizes, kind, pos, np.tile([0.0, 0.0, 0.0, 1.0], (len(pos), 1)), mass=mass)
+    batch.step(1.0 / 240.0)
+    off = np.concatenate([[0], np.cumsum(sizes)])
+    want = np.concatenate([p + o for p, o in zip(plain, off)])
+    assert all(len(p) > 0 for p in plain) and np.bincount(want[:, 0]).max() > 48
+    np.testing.assert_array_equal(batch.pairs().astype(np.int64), want)
+
+
+@gpu_only
 def test_batch_rejects_plain_body_insertion(gpu):
     import bgpu
 
