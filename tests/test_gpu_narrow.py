@@ -48,6 +48,25 @@ def test_overlapping_hulls(gpu, pairs, points):
     assert len(w.pairs()) == pairs
 
 
+@pytest.mark.parametrize("n,h,d,off", [(64, 0.8, 0.003, 5e-4), (80, 3.0, 0.003, 5e-4), (90, 0.8, 0.001, 1e-3),
+                                       (100, 1.5, 0.001, 2e-4), (100, 3.0, 0.001, 5e-4)])
+def test_horizons_wider_than_a_warp(gpu, n, h, d, off):
+    """A hull of two cones on a ring of n points, with one more point just outside the lower cone next to its tip,
+    about a capsule of no length (a point with a margin): the polytope's expansion finds that point last, when it sees
+    half of the lower cone's n faces, so the horizon has some n / 2 edges (42 to 50 from n = 80 on)."""
+    a = 2 * np.pi * np.arange(n) / n + 0.01
+    pts = np.concatenate([np.stack([np.cos(a), np.zeros(n), np.sin(a)], axis=1),
+                          [[0, h, 0], [0, -h, 0], [d, -h + 1e-4, 0]]]).astype(np.float32)
+    w, o = _both(gpu)
+    for x in (w, o):
+        x.set_gravity((0.0, 0.0, 0.0))
+        assert [x.hull(pts), x.capsule(0.3, 0.0)] == [0, 1]
+        x.add_body(0, (0.0, 0.0, 0.0), mass=1.0)
+        x.add_body(1, (off, -0.3 * off, 0.0), mass=0.0)
+    lockstep(w, o, 1.0 / 60.0, 1, f"ring of {n}")
+    assert w.stats()["num_contacts"] == 1
+
+
 @pytest.mark.parametrize("count,half", [(1, 0.1), (5, 0.3), (40, 0.45)])
 def test_bodies_in_terrain(gpu, count, half):
     import scenes
@@ -90,6 +109,32 @@ def test_terrain_pairs_on_both_sides_of_a_block_a_pair(gpu, count):
             x.add_body(1 + k % 3, p, q, mass=1.0)
     lockstep(w, o, 1.0 / 60.0, 2, f"{count} on terrain")
     assert (w.pairs()[:, 0] == 0).sum() == count
+
+
+@pytest.mark.parametrize("shape", ["box", "hull", "sphere"])
+def test_walks_wider_than_the_lists(gpu, shape):
+    """1,600 triangles that cross at the origin, along x and along z in turn: each leaf's box reaches the far
+    corner where the body lies on a patch of floor, none of the leaves' triangles does, so the walk meets more
+    nodes than its lists hold (256) for a few candidates."""
+    v = [[-10, 0, -0.5], [10, 0, -0.5], [0, 0, 1], [-0.5, 0, -10], [-0.5, 0, 10], [1, 0, 0]]
+    idx = [[0, 2, 1], [3, 4, 5]] * 800
+    for i in range(3):
+        for k in range(3):
+            v.append([6.5 + i, 0, 6.5 + k])
+    for i in range(2):
+        for k in range(2):
+            q = 6 + 3 * i + k
+            idx += [[q, q + 1, q + 4], [q, q + 4, q + 3]]
+    v, idx = np.asarray(v, np.float32), np.asarray(idx, np.uint32)
+    w, o = _both(gpu)
+    for x in (w, o):
+        assert x.mesh(v, idx) == 0
+        assert {"box": lambda: x.box([0.5, 0.5, 0.5]), "hull": lambda: x.hull(_hull(np.random.default_rng(1), 24, 0.5)),
+                "sphere": lambda: x.sphere(0.5)}[shape]() == 1
+        x.add_body(0, (0.0, 0.0, 0.0), mass=0.0)
+        x.add_body(1, (7.6, 0.48, 7.4), (0.0, 0.1, 0.0, 0.995), mass=1.0)
+    lockstep(w, o, 1.0 / 60.0, 3, f"{shape} far from the leaves")
+    assert w.stats()["num_contacts"] > 0 and w.stats()["device_status"] == 0
 
 
 def test_terrain_query_beyond_the_lists(gpu):
