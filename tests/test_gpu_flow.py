@@ -24,7 +24,7 @@ sys.path[:0] = [sys.argv[1] + "/bullet-physics_b200"]
 import numpy as np
 import bgpu, scenes
 kind, iters, steps = sys.argv[2], int(sys.argv[3]), int(sys.argv[4])
-if kind == "boxes":        # 1,050 bodies: the smallest worlds the kernel takes, a few groups a chunk
+if kind == "boxes":        # 1,050 bodies: the smallest worlds cut into chunks, a few groups a chunk
     s = scenes.falling_box_stack(7, 6, 25, seed=9)
 elif kind == "mixed":      # every row count, deep overlaps at the start (split groups, many colours)
     s = scenes.mixed_convex_pile(1500, seed=8, extent=9.0)
@@ -76,6 +76,73 @@ def test_plain_worlds_on_both_sides_of_the_lines(gpu_oracle, n):
         a, b = g.state(), o.state()
         assert np.abs(a[:, :13] - b[:, :13]).max() <= 1e-5 * max(1.0, np.abs(b[:, :13]).max())
     assert g.num_bodies == n and g.stats()["num_contacts"] > n and g.stats()["device_status"] == 0
+
+
+def _plain_and_one_block(bgpu, s, kinematic):
+    """The scene as a plain world and as a batch of one world, which one block solves."""
+    a = s.arrays()
+    d = bgpu.desc_array(a["shape"], a["pos"], a["quat"], a["linvel"], a["angvel"], a["mass"], a["friction"],
+                        a["restitution"])
+    if kinematic:
+        d["mass"][-1], d["flags"][-1], d["linear_velocity"][-1] = 0.0, bgpu.KINEMATIC, (0.5, 0.0, 0.0)
+    out = []
+    for batch in (False, True):
+        w = bgpu.World(gravity=s.gravity, batch=batch, num_iterations=s.iterations)
+        import scenes
+        scenes.add_shapes(w, s.shapes)
+        first, n = bgpu.ctypes.c_uint32(), bgpu.ctypes.c_uint32(len(d))
+        p = d.ctypes.data_as(bgpu.ctypes.POINTER(bgpu.BodyDesc))
+        if batch:
+            bgpu.check(w.L.bgpu_batch_add_worlds(w.h, 1, bgpu.ctypes.byref(n), p, bgpu.ctypes.byref(first)), "add_worlds")
+            w.set_tuning(256, 0)
+        else:
+            bgpu.check(w.L.bgpu_add_bodies(w.h, len(d), p, bgpu.ctypes.byref(first)), "add_bodies")
+        out.append(w)
+    return out
+
+
+@pytest.mark.parametrize("kind,iters", [("boxes", 10), ("boxes", 0), ("boxes", 1), ("mixed", 0), ("mixed", 1),
+                                        ("mixed", 10), ("pile", 25)])
+def test_many_blocks_equal_one(gpu_oracle, kind, iters):
+    """Worlds of 256 to 1,024 bodies, solved by many blocks, against one block, bit for bit: a kinematic body,
+    deep overlaps (split groups), groups of every row count, no velocity sweep, one and many."""
+    bgpu, _, scenes = gpu_oracle
+    s = {"boxes": lambda: scenes.falling_box_stack(7, 6, 7, seed=9),
+         "mixed": lambda: scenes.mixed_convex_pile(700, seed=8, extent=7.0),
+         "pile": lambda: scenes.large_pile(10, 10, 10, seed=7, spacing=1.0)}[kind]()
+    s.iterations = iters
+    plain, one = _plain_and_one_block(bgpu, s, kind == "boxes")
+    assert 256 <= plain.num_bodies <= 1024
+    split = 0
+    for step in range(60 if kind == "boxes" else 30):
+        plain.step(s.dt)
+        one.step(s.dt)
+        np.testing.assert_array_equal(plain.state(), one.state(), err_msg=f"step {step}")
+        split += plain.stats()["num_split_pairs"]
+    assert plain.stats()["num_contacts"] > 0 and (kind != "mixed" or split > 0)
+
+
+@pytest.mark.parametrize("n", [200, 300, 1000])
+def test_gradients_of_a_plain_world(gpu_oracle, n):
+    """A tape over a plain world (one block up to 255 bodies, many beyond) against the same world as a batch of one.
+    The reverse pass adds up a body's terms in its colours' order either way; only the friction and
+    restitution gradients add theirs by atomics, whose order is free: 1e-5 of the largest."""
+    bgpu, _, scenes = gpu_oracle
+    s = scenes.large_pile(nx=6, nz=6, ny=-(-n // 36), seed=n, spacing=1.0)
+    for f in ("shape_of", "pos", "quat", "linvel", "angvel", "mass", "friction", "restitution"):
+        setattr(s, f, getattr(s, f)[:n])
+    grads = []
+    for w in _plain_and_one_block(bgpu, s, False):
+        w.step(s.dt, 20)
+        t = bgpu.Tape(w, 6)
+        t.forward(s.dt, 15)
+        gx = np.random.default_rng(n).normal(size=(n, 3)).astype(np.float32)
+        grads.append(t.backward(gx))
+        assert w.stats()["num_contacts"] > n // 2
+    for k in ("v0", "w0", "friction", "restitution"):
+        scale = np.abs(grads[1][k]).max()
+        np.testing.assert_allclose(grads[0][k], grads[1][k], rtol=0.0, atol=1e-5 * max(scale, 1e-30), err_msg=k)
+    assert np.abs(grads[1]["v0"]).max() > 0.0 and np.abs(grads[1]["friction"]).max() > 0.0
 
 
 @pytest.fixture(scope="module")
