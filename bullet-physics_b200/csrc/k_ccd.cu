@@ -883,8 +883,9 @@ void launch_ccd_sweep(const BodyDev& b, const Shape* shapes, const float4* hull,
     const CcdItems items{scratch.items.p, scratch.count.p, m};
     k_ccd_sweep<<<m, CCD_THREADS, 0, s>>>(b, shapes, hull, ids, par, n, world_off, world_of, suppressed, nsuppressed,
                                           dt, clamp, status, tree_rec, tree_leaf, tree_m, unb, nunb, items);
-    k_ccd_cast<<<std::min<uint32_t>((m * CCD_RANKS * 32u + CCD_CAST_THREADS - 1) / CCD_CAST_THREADS, CCD_CAST_BLOCKS),
-                 CCD_CAST_THREADS, 0, s>>>(b, shapes, hull, ids, par, dt, clamp, status, items);
+    const uint64_t lanes = uint64_t(m) * CCD_RANKS * 32u;  // a warp for every cast there may be
+    const uint32_t blocks = uint32_t(std::min<uint64_t>((lanes + CCD_CAST_THREADS - 1) / CCD_CAST_THREADS, CCD_CAST_BLOCKS));
+    k_ccd_cast<<<blocks, CCD_CAST_THREADS, 0, s>>>(b, shapes, hull, ids, par, dt, clamp, status, items);
 }
 
 void launch_ccd_apply(const BodyDev& b, const uint32_t* ids, const float* clamp, uint32_t m, float dt, cudaStream_t s) {
