@@ -71,15 +71,16 @@ struct DevBuf {
 struct TileScan {
     unsigned long long* words;  // one per tile
     uint32_t* ticket;           // tiles are dealt in this order
-    uint32_t base, epoch;       // the ticket when the launch begins; the launch's mark in the words
+    uint32_t epoch;             // the launch's mark in the words
     uint32_t* status;
 };
 struct TileScanBuf {
     DevBuf<unsigned long long> words;
     DevBuf<uint32_t> ticket;
-    uint32_t tickets = 0, epoch = 0;
+    uint32_t epoch = 0;
     // The state of a launch of `tiles` blocks, each of which takes one ticket. No word needs
-    // clearing between launches: an earlier launch's words carry an earlier epoch.
+    // clearing between launches: an earlier launch's words carry an earlier epoch. The ticket is back at
+    // 0 after a launch, and a launch that fails leaves it there: the host counts nothing along.
     TileScan begin(uint32_t tiles, uint32_t* status, cudaStream_t s) {
         if (!ticket.p) {
             ticket.reserve(1);
@@ -90,9 +91,7 @@ struct TileScanBuf {
             check_cuda(cudaMemsetAsync(words.p, 0, words.cap * sizeof(unsigned long long), s), "memset");
             epoch = 0;
         }
-        const TileScan t{words.p, ticket.p, tickets, ++epoch, status};
-        tickets += tiles;
-        return t;
+        return TileScan{words.p, ticket.p, ++epoch, status};
     }
 };
 

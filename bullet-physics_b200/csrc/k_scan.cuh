@@ -14,10 +14,14 @@ __host__ __device__ __forceinline__ uint32_t tile_count(uint32_t n) {
     return (n + TILE_TB * ROUNDS - 1) / (TILE_TB * ROUNDS);
 }
 
-// The block's tile: tiles are dealt in order, so every tile before it has a running block.
+// The block's tile: tiles are dealt in order, so every tile before it has a running block. Every block of
+// the launch takes one; the last to do so puts the ticket back.
 __device__ __forceinline__ uint32_t tile_take(const TileScan& t) {
     __shared__ uint32_t s_tile;
-    if (threadIdx.x == 0) s_tile = atomicAdd(t.ticket, 1u) - t.base;
+    if (threadIdx.x == 0) {
+        s_tile = atomicAdd(t.ticket, 1u);
+        if (s_tile + 1u == gridDim.x) *t.ticket = 0u;
+    }
     __syncthreads();
     return s_tile;
 }
