@@ -357,6 +357,7 @@ __global__ void k_query(int m, uint32_t n, const uint32_t* __restrict__ is_unb, 
 // The partners j > h of each unbounded proxy h, tile by tile of proxies: their number (counts[h])
 // and, for the pass that writes them, how many lie before each tile (before[u tiles + tile]).
 constexpr uint32_t UNB_ROUNDS = 4;
+constexpr uint32_t UNB_TILES_MAX = 65536;  // tiles a launch: many unbounded proxies take several launches
 
 __device__ __forceinline__ uint32_t unb_ranks(uint32_t h, uint32_t base, uint32_t n, const float4* __restrict__ bmin,
                                               const float4* __restrict__ bmax, bool (&flag)[UNB_ROUNDS],
@@ -824,10 +825,13 @@ uint64_t Broadphase::run(const float4* aabb_min, const float4* aabb_max, uint32_
                                           nunb, counts.p, nullptr, nullptr, status_dev, overflow.p, scalars.p + 1,
                                           stash.p);
     const uint32_t utiles = tile_count<UNB_ROUNDS>(n), tiles = tile_count<4>(n);
-    if (nunb) {
-        unb_tiles.reserve(size_t(nunb) * utiles);
-        k_unb_tiles<<<nunb * utiles, TILE_TB, 0, s>>>(n, utiles, unbounded.p, aabb_min, aabb_max, unb_tiles.p, counts.p,
-                                                      scan.begin(nunb * utiles, status_dev, s));
+    const uint32_t upart = std::max(UNB_TILES_MAX / utiles, 1u);  // unbounded proxies a launch
+    unb_tiles.reserve(size_t(nunb) * utiles);
+    for (uint32_t u = 0; u < nunb; u += upart) {
+        const uint32_t blocks = std::min(upart, nunb - u) * utiles;
+        k_unb_tiles<<<blocks, TILE_TB, 0, s>>>(n, utiles, unbounded.p + u, aabb_min, aabb_max,
+                                               unb_tiles.p + size_t(u) * utiles, counts.p,
+                                               scan.begin(blocks, status_dev, s));
     }
     k_segments<<<tiles, TILE_TB, 0, s>>>(n, counts.p, offsets.p, scalars.p, host_scalars, scan.begin(tiles, status_dev, s));
     check_cuda(cudaStreamSynchronize(s), "broadphase sync");
@@ -835,10 +839,16 @@ uint64_t Broadphase::run(const float4* aabb_min, const float4* aabb_max, uint32_
     const uint32_t n_overflow = host_scalars[1];
     out.reserve(total + 1);
     if (total) {
-        const uint32_t sblocks = m > 0 ? (uint32_t(m) + TILE_TB - 1) / TILE_TB : 0u;
-        k_write_pairs<<<sblocks + nunb * utiles, TILE_TB, 0, s>>>(m, leaf_body.p, counts.p, offsets.p, stash.p, out.p,
-                                                                  sblocks, n, utiles, unbounded.p, aabb_min, aabb_max,
-                                                                  unb_tiles.p);
+        uint32_t sblocks = m > 0 ? (uint32_t(m) + TILE_TB - 1) / TILE_TB : 0u, u = 0;
+        do {
+            const uint32_t ublocks = std::min(upart, nunb - u) * utiles;
+            if (sblocks + ublocks)
+                k_write_pairs<<<sblocks + ublocks, TILE_TB, 0, s>>>(m, leaf_body.p, counts.p, offsets.p, stash.p, out.p,
+                                                                    sblocks, n, utiles, unbounded.p + u, aabb_min, aabb_max,
+                                                                    unb_tiles.p + size_t(u) * utiles);
+            sblocks = 0;
+            u += upart;
+        } while (u < nunb);
         if (n_overflow)
             k_query<Q_WRITE><<<(n_overflow + TB - 1) / TB, TB, 0, s>>>(
                 m, n, is_unb.p, aabb_min, aabb_max, node_rec.p, leaf_body.p, unbounded.p, nunb, counts.p, offsets.p,

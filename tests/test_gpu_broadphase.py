@@ -107,3 +107,37 @@ def test_tree_at_the_edges_of_a_refit_block(n):
     assert _entry(bgpu)(dev.data_ptr(), n, out.data_ptr(), len(want) + 8, ctypes.byref(got), None) == 0
     torch.cuda.synchronize()
     np.testing.assert_array_equal(out[: got.value].cpu().numpy().view(np.uint32), want)
+
+
+@pytest.mark.parametrize("meshes", [1, 4680, 4682, 9500])
+def test_many_proxies_outside_the_tree(meshes):
+    """Meshes are kept out of the tree, 14 tiles of 1,024 proxies each: 4,681 of them take a launch, more take
+    two and three. Small meshes among spheres, a few meshes under a crowd, against the oracle's
+    brute force."""
+    import bgpu
+    import oracle_api as orc
+
+    n = 14000
+    rng = np.random.default_rng(meshes)
+    side = (n * 0.3) ** (1.0 / 3.0) * 1.5
+    pos = rng.uniform(0.0, side, size=(n, 3))
+    kind = np.full(n, 1)
+    kind[rng.permutation(n)[:meshes]] = 0
+    big = np.flatnonzero(kind == 0)[::997]
+    worlds = []
+    for x in (bgpu.World(gravity=(0.0, 0.0, 0.0), num_iterations=1), orc.OracleWorld("f32")):
+        x.set_gravity((0.0, 0.0, 0.0))
+        tri = [[-0.3, 0.0, -0.3], [0.3, 0.1, -0.3], [0.0, 0.2, 0.3]]
+        assert [x.mesh(np.asarray(tri, np.float32), [[0, 2, 1]]), x.sphere(0.25),
+                x.mesh(20.0 * np.asarray(tri, np.float32), [[0, 2, 1]])] == [0, 1, 2]
+        k = kind.copy()
+        k[big] = 2
+        for i in range(n):
+            x.add_body(int(k[i]), tuple(pos[i]), mass=1.0 if k[i] == 1 else 0.0)
+        worlds.append(x)
+    w, o = worlds
+    o.set_brute_force(True)
+    w.step(1.0 / 240.0)
+    o.step(1.0 / 240.0)
+    np.testing.assert_array_equal(w.pairs(), o.pairs())
+    assert np.bincount(w.pairs()[:, 0]).max() > 32
