@@ -279,9 +279,10 @@ struct Broadphase {
     Broadphase();
     ~Broadphase();
     // Up to this many proxies every pair is tested (no tree): n^2 / 2 tests cost less than the tree's
-    // launches and climbs. Broad phase of settled piles, all pairs / tree: 1,024 bodies 57 / 118 us,
-    // 4,096 74 / 144, 8,000 97 / 197, 12,500 161 / 201, 16,250 218 / 208 (the all-pairs pass has become
-    // faster since: 5,700 bodies 56 -> 34 us).
+    // launches and climbs, and the masks take 19 MB at most. Broad phase of settled piles, all pairs / tree:
+    // 1,001 bodies 46 / 117 us, 4,097 62 / 138, 8,001 85 / 187, 12,168 122 / 194, 16,225 173 / 200, 18,001
+    // 194 / 208, 20,481 231 / 205. (The line was drawn where the two met before the all-pairs pass became faster;
+    // they meet near 18,500 now.)
     static constexpr uint32_t ALL_PAIRS_MAX = 12288;
     // Returns the pair count; pairs are written to `out` (grown as needed). all_pairs: test every
     // pair (n <= ALL_PAIRS_MAX). centres: the bounded proxies' centre bounds when a kernel before

@@ -882,10 +882,10 @@ namespace {
 
 constexpr size_t NOALLOC_SCRATCH_BYTES = size_t(24) << 20;
 // Bytes per proxy of the arrays taken below (AABBs 32, sort keys 16, flags / scans / counts /
-// offsets / tree links 36, parents 8, node boxes 64, node records 64, node index bounds 8),
+// offsets / tree links 36, parents 8, node boxes 64, node records 64),
 // plus 256 B of alignment per array and room for CUB's sort / scan scratch (a few hundred KB
 // at 65,536 keys; 4 MiB allowed). Each take() is also checked when the call runs.
-constexpr size_t NOALLOC_PER_PROXY_BYTES = 228;
+constexpr size_t NOALLOC_PER_PROXY_BYTES = 220;
 static_assert(NOALLOC_PER_PROXY_BYTES * BGPU_NOALLOC_MAX_PROXIES + 32 * 256 + (size_t(4) << 20) <= NOALLOC_SCRATCH_BYTES,
               "the allocation-free broad phase's scratch array is too small for its proxy limit");
 static __device__ __align__(256) unsigned char g_bp_scratch[NOALLOC_SCRATCH_BYTES];

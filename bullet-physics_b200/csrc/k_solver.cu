@@ -10,10 +10,11 @@
 // is touched twice, so the result is bit-identical to the reference's
 // sequential solve over the same rows taken in (colour, pair) order.
 //
-// Worlds without joints use the chunked PGS (k_solve_flow): the bodies are cut into
-// Morton-ordered chunks, one per block of a cooperative launch, and each warp solves its share of
-// the chunk's groups colour by colour, waiting only for the versions of its groups' own velocities
-// (a version rides in the fourth word of a velocity). A group's contacts are spread over lanes (one
+// Worlds without joints use the chunked PGS (k_solve_flow): the bodies are cut into chunks (in Morton
+// order where the broad phase has a tree, in index order where it has none), one per block of a
+// cooperative launch, and each warp solves its share of the chunk's groups colour by colour,
+// waiting only for the versions of its groups' own velocities (a version rides in the fourth word
+// of a velocity). A group's contacts are spread over lanes (one
 // contact per lane, the velocities handed from lane to lane in contact order), and the split
 // sweep s rides in the phases of velocity sweep s + 1. Worlds with joints use the team kernel
 // (k_solve): a persistent cooperative launch split into two teams of blocks with their own
@@ -489,8 +490,8 @@ __device__ __forceinline__ uint32_t claim_slot(uint32_t* cursor, uint32_t c) {
 
 // ---------------------------------------------------------------- chunks (chunked PGS)
 // The chunked PGS deals each colour batch to the blocks of the launch by chunk: a chunk is a
-// run of bodies in Morton order (the broad phase's tree leaves), and a group belongs to the
-// chunk of its first dynamic body. Block b solves chunk b's groups of every colour.
+// run of bodies in Morton order (the broad phase's tree leaves; without a tree in index order), and a
+// group belongs to the chunk of its first dynamic body. Block b solves chunk b's groups of every colour.
 //
 // Ordering: within a sweep a dynamic body is updated by its groups in colour order, so its
 // velocity goes through a chain of versions known before the solve starts: the group with rank r

@@ -945,7 +945,9 @@ struct World {
         reset.owned_n = cache[cur].count_dev;
         mark(0);
         // 1-3: velocities, predicted poses, AABBs (fused).
-        // Few bodies: every pair is tested, with no tree (which CCD sweeps over many bodies want).
+        // Few bodies: every pair is tested, with no tree. CCD sweeps walk the tree, or without one scan the
+        // world; a step of the rain of fast spheres, all pairs / tree: 945 bodies 1.49 / 1.53 ms, 2,257 1.66 /
+        // 1.69, 3,329 2.42 / 2.41, 8,465 (64 of them fast) 1.69 / 1.62, 8,901 (4,000 fast) 3.70 / 3.25.
         const bool all_pairs = !batch && n <= Broadphase::ALL_PAIRS_MAX && (nccd == 0 || n <= 1024);
         islands.reserve(n);
         const int now = begin_parity, next_begin = now ^ 1;

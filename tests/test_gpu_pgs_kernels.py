@@ -1,7 +1,7 @@
 """The two PGS kernels for worlds without joints give the same trajectory, bit for bit.
 
 A plain world of more than 1,024 bodies without joints is solved by the chunked kernel
-(Morton-ordered chunks, neighbour waits); BGPU_PGS=team in the environment selects the
+(bodies cut into chunks, versioned velocities); BGPU_PGS=team in the environment selects the
 team-barrier kernel instead (read once per process, so each runs in a child process). Both
 solve the groups in the same (colour, pair) order, so the states after every step must be
 identical, not merely close. The oracle lockstep tests pin the chunked kernel against the
