@@ -712,7 +712,6 @@ __global__ void __launch_bounds__(CCD_CAST_THREADS) k_ccd_cast(BodyDev b, const 
     const uint32_t mine = (g == 32u ? 0xffffffffu : (1u << g) - 1u) << (lane - sl);  // the segment's lanes
     // A walk takes at most 258 steps (the first support point, 64 iterations of at most four, the end), a
     // cast 41 rounds of them, and each vote is a step of every walk: the loop below ends before `left` does.
-    uint32_t left = (total / (nwarps * segs) + 1u) * (41u * 258u);
     // The segment's cast (the same values on all its lanes) and the lane's walk.
     enum { TERNARY, CLOSEST, BISECT, IDLE };
     int phase = IDLE;
@@ -725,7 +724,11 @@ __global__ void __launch_bounds__(CCD_CAST_THREADS) k_ccd_cast(BodyDev b, const 
     w.d2 = 0.0f;
     bool ready = true;   // the segment's round is over and its decisions are taken
     uint32_t seen = 0u;  // the last vote on the walks that are done
-    for (;; --left) {
+    // The loop ends by itself: a segment's lanes hold the same cast, each vote is a step of every walk that is
+    // not done, a walk has 258 steps at most (the first support point, 64 iterations of up to four, the end), a
+    // cast 41 rounds of walks, and every cast is taken once. (A count of the votes beside it is one register too
+    // many: it spills, and a launch takes 1.5 % longer; in shared memory 5 %.)
+    for (;;) {
         if (ready) {
             // The next round of probes: of this cast, or of the segment's next one.
             w.done = true;
@@ -796,10 +799,6 @@ __global__ void __launch_bounds__(CCD_CAST_THREADS) k_ccd_cast(BodyDev b, const 
             }
         }
         if (!__any_sync(0xffffffffu, phase != IDLE)) break;
-        if (left == 0u) {
-            if (lane == 0u) atomicOr(status, ST_BARRIER_TIMEOUT);
-            break;
-        }
         if (!w.done) w.step(t);
         // Follow the decisions as far as their probes are done: a round ends with the probes on the
         // taken path, whatever the walks beside it are still at.
